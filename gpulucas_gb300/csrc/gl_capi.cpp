@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "gl_internal.h"
@@ -19,6 +20,10 @@ using namespace gl;
 namespace {
 
 constexpr int kGraphBatch = 64;
+// An integer-form plan runs one iteration in this many in FP64: the same products, with
+// the round-off measured.
+constexpr int kFp64Every = 64;
+static_assert(kFp64Every == kGraphBatch, "a captured batch ends with its FP64 iteration");
 
 int cuda_status(cudaError_t e) { return e == cudaSuccess ? GL_OK : GL_ERR_CUDA; }
 
@@ -319,6 +324,63 @@ int stage_offsets(const LinePlan& lp, int* off) {
   return size;
 }
 
+int int_stage_offsets(LinePlan* lp) {
+  int size = 1, Ns = 1;
+  for (int s = 0; s < lp->nst; ++s) {
+    lp->off[s] = size;
+    if (Ns > 1) size += (lp->radix[s] - 1) * Ns;
+    Ns *= lp->radix[s];
+  }
+  return size;
+}
+
+// Geometry of the integer form on an H x W layout; false where GF(q^2) lacks the roots or
+// a CTA's lines do not fit its shared memory.
+bool choose_int_geom(int H, int W, IntGeom* g) {
+  if (!gf_supported(H * W)) return false;
+  if (!fill_line_plan(W, &g->pw) || !fill_line_plan(H, &g->ph)) return false;
+  int_stage_offsets(&g->pw);
+  int_stage_offsets(&g->ph);
+  auto threads = [](int butterflies) {
+    const int t = round_up32(butterflies);
+    return t < 64 ? 64 : (t > kMaxThreads ? kMaxThreads : t);
+  };
+  g->t_col = threads((H + 7) / 8);
+  g->t_row = row_threads(W, g->pw, threads((2 * W + 7) / 8));
+  g->sm_col = (size_t)2 * int_stride(H) * 16;
+  g->sm_row = (size_t)4 * int_stride(W) * 16;
+  return g->sm_col <= (size_t)kMaxIntSmem && g->sm_row <= (size_t)kMaxIntSmem;
+}
+
+// Column length of the first layout of the cost model that the integer form can run, or 0.
+int first_int_layout(int M, int sms) {
+  IntGeom g{};
+  for (const auto& c : ranked_layouts(M, sms))
+    if (choose_int_geom(c.second, M / c.second, &g)) return c.second;
+  return 0;
+}
+
+// Whether the products of (p, N) are determined by their residues mod q = 2^61 - 1 for
+// every state the iteration can reach: words are at most 2^LO plus a carry in magnitude,
+// an unweighted product sums N of their products times at most 2, and must stay below 2^60.
+// *vmax: the bound on a word used here (a loaded state is checked against it).
+bool int_range_ok(int p, int N, int* vmax) {
+  const int LO = p / N;
+  if (LO > 28) return false;
+  const double v = (double)(1 << LO) + 256.0;
+  *vmax = (1 << LO) + 256;
+  return 2.0 * N * v * v < 1152921504606846976.0;  // 2^60
+}
+
+// The integer form has no round-off to watch, so it is used where the FP64 form's stays
+// well below the default limit: up to 0.3 bits per word over gl_safe_signal_size's line
+// (measured round-off <= 0.125 on the line; it doubles every 0.5 bits, so <= 0.19 here) and
+// with a limit that is not tightened.  Elsewhere every iteration measures its round-off.
+constexpr double kIntBitsOverSafe = 0.3;
+bool int_roundoff_ok(int p, int N, double error_limit) {
+  return error_limit >= 0.4 && (double)p / N <= 19.2 + kIntBitsOverSafe - 0.26 * std::log2(N / 163840.0);
+}
+
 // Device time of one fused iteration with column length H, measured on zero-filled
 // buffers (the kernels' time does not depend on the values).  Returns ms, or -1.
 double time_layout(int M, int H, int rc, int rr, bool ip, bool pf, bool ws, int row, int n, int sms, int iters,
@@ -452,11 +514,97 @@ TunedLayout autotune_layout(int M, int n, int sms, cudaStream_t s, double* ms_ou
   return best;
 }
 
+// Device time of one integer-form iteration on the H x (M / H) layout, or -1.
+double time_int_layout(int M, int H, int n, int iters, cudaStream_t s) {
+  IntGeom g{};
+  const int W = M / H, N = 2 * M;
+  if (!choose_int_geom(H, W, &g)) return -1.0;
+  std::vector<RowPair> rows;
+  gf_row_pairs(W, H, rows);
+  LinePlan pw = g.pw, ph = g.ph;
+  const size_t szw = (size_t)int_stage_offsets(&pw) * 16, szh = (size_t)int_stage_offsets(&ph) * 16;
+  const size_t m16 = 16 * (size_t)M;
+  const size_t bytes[] = {8 * (size_t)N, (size_t)N, (size_t)N, (size_t)N, m16, m16, m16, m16, m16,
+                          szw, szw, szh, szh, rows.size() * sizeof(RowPair), sizeof(Status)};
+  constexpr int nb = sizeof(bytes) / sizeof(bytes[0]);
+  void* buf[nb] = {};
+  double ms = -1.0;
+  bool ok = true;
+  for (int i = 0; i < nb && ok; ++i)
+    ok = cudaMalloc(&buf[i], bytes[i]) == cudaSuccess && cudaMemsetAsync(buf[i], 0, bytes[i], s) == cudaSuccess;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  if (ok) ok = cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess;
+  if (ok) ok = set_int_smem_limits() == cudaSuccess;
+  if (ok)
+    ok = cudaMemcpyAsync(buf[13], rows.data(), rows.size() * sizeof(RowPair), cudaMemcpyHostToDevice, s) == cudaSuccess &&
+         cudaStreamSynchronize(s) == cudaSuccess;
+  if (ok) {
+    IterArgs a{};
+    a.N = N; a.M = M; a.W = W; a.H = H; a.G = 1; a.LO = 18; a.n = n;
+    a.ll = (long long*)buf[0]; a.flags = (const unsigned char*)buf[1]; a.span = (const unsigned char*)buf[2];
+    a.in.e = (const unsigned char*)buf[3]; a.Z = (DevCplx*)buf[4]; a.Z2 = (DevCplx*)buf[5];
+    a.in.k1 = (const int4*)buf[6]; a.in.pair = (const int4*)buf[7]; a.in.k2 = (const int4*)buf[8];
+    a.in.wf = (const int4*)buf[9]; a.in.wi = (const int4*)buf[10];
+    a.in.hf = (const int4*)buf[11]; a.in.hi = (const int4*)buf[12];
+    a.in.rows = (const int4*)buf[13]; a.status = (Status*)buf[14];
+    a.in.nrows = (int)rows.size();
+    a.in.qW = (int)(((1ull << 61) - 1) % (uint64_t)W);
+    a.in.ls_col = int_stride(H); a.in.ls_row = int_stride(W); a.in.pw = g.pw; a.in.ph = g.ph;
+    for (int i = 0; i < 2 && ok; ++i) ok = launch_int_iteration(a, g, s, false) == cudaSuccess;
+    ok = ok && cudaEventRecord(e0, s) == cudaSuccess;
+    for (int i = 0; i < iters && ok; ++i) ok = launch_int_iteration(a, g, s, false) == cudaSuccess;
+    ok = ok && cudaEventRecord(e1, s) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess;
+    float t = 0.f;
+    if (ok && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess) ms = t / iters;
+  }
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  cudaStreamSynchronize(s);
+  for (void* b : buf)
+    if (b) cudaFree(b);
+  return ms;
+}
+
+// Column length of the integer form for M complex points on this device: the candidates of
+// the layout model that it can run are timed and the fastest kept, once per (M, SM count)
+// per process.  0: no layout.
+std::map<std::pair<int, int>, std::pair<int, double>> g_int_tune_cache;
+constexpr int kIntLayoutsTimed = 8;
+
+int autotune_int_layout(int M, int n, int sms, cudaStream_t s, double* ms_out) {
+  {
+    std::lock_guard<std::mutex> lock(g_tune_mutex);
+    auto it = g_int_tune_cache.find({M, sms});
+    if (it != g_int_tune_cache.end()) {
+      if (ms_out) *ms_out = it->second.second;
+      return it->second.first;
+    }
+  }
+  int best = 0, timed = 0;
+  double best_ms = 1e300;
+  for (const auto& c : ranked_layouts(M, sms)) {
+    if (timed == kIntLayoutsTimed) break;
+    const double ms = time_int_layout(M, c.second, n, M >= (1 << 18) ? 10 : 40, s);
+    if (ms <= 0.0) continue;
+    ++timed;
+    if (ms < best_ms) {
+      best_ms = ms;
+      best = c.second;
+    }
+  }
+  if (!best) return 0;
+  std::lock_guard<std::mutex> lock(g_tune_mutex);
+  g_int_tune_cache[{M, sms}] = {best, best_ms};
+  if (ms_out) *ms_out = best_ms;
+  return best;
+}
+
 void free_plan(gl_plan* pl) {
   if (!pl) return;
   if (pl->device >= 0) cudaSetDevice(pl->device);
   if (pl->gexec) cudaGraphExecDestroy(pl->gexec);
-  if (pl->hw_exec) cudaGraphExecDestroy(pl->hw_exec);
+  for (cudaGraphExec_t g : pl->hw_exec)
+    if (g) cudaGraphExecDestroy(g);
   for (void* p : pl->allocs) cudaFree(p);
   if (pl->h_status) cudaFreeHost(pl->h_status);
   if (pl->h_res) cudaFreeHost(pl->h_res);
@@ -466,21 +614,35 @@ void free_plan(gl_plan* pl) {
   delete pl;
 }
 
+// One iteration on the plan's stream.  fp64: the FP64 form (its round-off is measured);
+// else the integer form, for plans that have it.  A state loaded by the caller
+// (from_state) may hold words the integer form has no bound for, and runs in FP64.
+int launch_iteration(gl_plan* pl, bool fp64) {
+  cudaError_t e;
+  if (pl->mode == GL_MODE_PLAIN) {
+    e = launch_plain_iteration(pl->args, pl->pg, pl->stream);
+  } else if (pl->int_form && !fp64 && !pl->from_state) {
+    e = launch_int_iteration(pl->args, pl->ig, pl->stream, false);
+  } else {
+    e = launch_fused_iteration(pl->args, pl->fg, pl->stream, pl->from_state);
+    pl->from_state = false;
+  }
+  return e == cudaSuccess ? GL_OK : GL_ERR_CUDA;
+}
+
+// k iterations; an integer-form plan runs one in kFp64Every in FP64
 int launch_iterations(gl_plan* pl, int64_t k) {
   for (int64_t i = 0; i < k; ++i) {
-    cudaError_t e;
-    if (pl->mode == GL_MODE_PLAIN) {
-      e = launch_plain_iteration(pl->args, pl->pg, pl->stream);
-    } else {
-      e = launch_fused_iteration(pl->args, pl->fg, pl->stream, pl->from_state);
-      pl->from_state = false;
-    }
-    if (e != cudaSuccess) return GL_ERR_CUDA;
+    const bool fp64 = pl->from_state || ++pl->since_fp64 >= kFp64Every;
+    const int rc = launch_iteration(pl, fp64);
+    if (rc != GL_OK) return rc;
+    if (fp64) pl->since_fp64 = 0;
   }
   return GL_OK;
 }
 
-// Enqueue k iterations, with batches of kGraphBatch replayed from one CUDA graph.
+// Enqueue k iterations, with batches of kGraphBatch replayed from one CUDA graph (in an
+// integer-form plan the last of the batch is the FP64 one).
 int enqueue(gl_plan* pl, int64_t k) {
   if (k <= 0) return GL_OK;
   int rc;
@@ -500,7 +662,8 @@ int enqueue(gl_plan* pl, int64_t k) {
     if (!pl->gexec) {
       cudaGraph_t graph = nullptr;
       GL_CUDA(cudaStreamBeginCapture(pl->stream, cudaStreamCaptureModeThreadLocal));
-      int lrc = launch_iterations(pl, kGraphBatch);
+      int lrc = GL_OK;
+      for (int i = 0; i < kGraphBatch && lrc == GL_OK; ++i) lrc = launch_iteration(pl, i == kGraphBatch - 1);
       cudaError_t ec = cudaStreamEndCapture(pl->stream, &graph);
       if (lrc != GL_OK || ec != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
@@ -517,6 +680,7 @@ int enqueue(gl_plan* pl, int64_t k) {
     while (k >= pl->gexec_iters) {
       GL_CUDA(cudaGraphLaunch(pl->gexec, pl->stream));
       k -= pl->gexec_iters;
+      pl->since_fp64 = 0;
     }
   }
   return launch_iterations(pl, k);
@@ -611,7 +775,72 @@ double gl_plan_unit_cost(const gl_plan* pl, bool row) {
   return pl->fg.H * (line_ops(pl->fg.ph) + 6.0);
 }
 
-int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, gl_plan** out) {
+// Options that choose among the FP64 form's layouts and kernels: such a plan runs them in
+// every iteration.
+static bool names_fp64_variant(const gl_plan_opts& o) {
+  return o.fft_h || o.cols_per_cta || o.max_radix_col || o.max_radix_row || o.resident > 0 || o.col_inplace ||
+         o.row_pass;
+}
+
+// Device bytes of the integer form's tables for an H x W layout.
+static size_t int_table_bytes(int H, int W, const IntGeom& g) {
+  LinePlan pw = g.pw, ph = g.ph;
+  const size_t M = (size_t)H * W;
+  std::vector<RowPair> rows;
+  gf_row_pairs(W, H, rows);
+  return 3 * M * 16 + 2 * M /* exponents */ + 2 * 16 * ((size_t)int_stage_offsets(&pw) + int_stage_offsets(&ph)) +
+         rows.size() * sizeof(RowPair);
+}
+
+static int build_int_tables(gl_plan* pl, int vmax) {
+  const int W = pl->fg.W, H = pl->fg.H, N = pl->N;
+  std::vector<HostTw> k1, pair, k2, wf, wi, hf, hi;
+  std::vector<RowPair> rows;
+  std::vector<uint8_t> e, e_c((size_t)N);
+  int off[8];
+  gf_pass_tables(W, H, k1, pair, k2);
+  gf_row_pairs(W, H, rows);
+  gf_weights(pl->p, N, e);
+  gf_stage_twiddles(W, pl->ig.pw.radix, pl->ig.pw.nst, false, wf, off);
+  gf_stage_twiddles(W, pl->ig.pw.radix, pl->ig.pw.nst, true, wi, off);
+  gf_stage_twiddles(H, pl->ig.ph.radix, pl->ig.ph.nst, false, hf, off);
+  gf_stage_twiddles(H, pl->ig.ph.radix, pl->ig.ph.nst, true, hi, off);
+  for (int m1 = 0, c = 0; m1 < W; ++m1)  // column-major, as the other per-word tables
+    for (int m2 = 0; m2 < H; ++m2, c += 2) {
+      e_c[c] = e[2 * (m1 + (size_t)W * m2)];
+      e_c[c + 1] = e[2 * (m1 + (size_t)W * m2) + 1];
+    }
+  IntArgs& in = pl->args.in;
+  auto up = [&](auto** dst, const void* src, size_t count) {
+    using T = std::remove_const_t<std::remove_pointer_t<std::remove_pointer_t<decltype(dst)>>>;
+    T* d = nullptr;
+    const int rc = dev_alloc(pl, &d, count);
+    if (rc != GL_OK) return rc;
+    *dst = d;
+    return cuda_status(cudaMemcpyAsync(d, src, count * sizeof(T), cudaMemcpyHostToDevice, pl->stream));
+  };
+  static_assert(sizeof(HostTw) == sizeof(int4) && sizeof(RowPair) == sizeof(int4), "table entries");
+  int rc;
+  if ((rc = up(&in.k1, k1.data(), k1.size())) || (rc = up(&in.pair, pair.data(), pair.size())) ||
+      (rc = up(&in.k2, k2.data(), k2.size())) || (rc = up(&in.wf, wf.data(), wf.size())) ||
+      (rc = up(&in.wi, wi.data(), wi.size())) || (rc = up(&in.hf, hf.data(), hf.size())) ||
+      (rc = up(&in.hi, hi.data(), hi.size())) || (rc = up(&in.rows, rows.data(), rows.size())) ||
+      (rc = up(&in.e, e_c.data(), e_c.size())))
+    return rc;
+  GL_CUDA(cudaStreamSynchronize(pl->stream));  // host tables go out of scope
+  in.nrows = (int)rows.size();
+  in.qW = (int)(((1ull << 61) - 1) % (uint64_t)W);
+  in.vmax = vmax;
+  in.ls_col = int_stride(H);
+  in.ls_row = int_stride(W);
+  in.pw = pl->ig.pw;
+  in.ph = pl->ig.ph;
+  GL_CUDA(set_int_smem_limits());
+  pl->int_form = true;
+  return GL_OK;
+}
+
+int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, gl_plan** out, bool fp64_only) {
   if (!out) return GL_ERR_ARG;
   *out = nullptr;
   gl_plan_opts o;
@@ -665,6 +894,16 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
     cudaGetLastError();
   }
   if (o.resident > 0 && !resident) return GL_ERR_SIZE;
+  // The integer form, unless an option names a variant of the FP64 kernels.
+  IntGeom ig{};
+  int vmax = 0;
+  bool int_form = o.mode == GL_MODE_FUSED && !resident && !fp64_only && !sms_override && !names_fp64_variant(o) &&
+                  int_range_ok(p, N, &vmax) && int_roundoff_ok(p, N, o.error_limit);
+  if (int_form) {
+    const int H = o.autotune && !sms_override ? autotune_int_layout(M, n, sms, 0, nullptr) : first_int_layout(M, sms);
+    if (H) force_h = H;
+    else int_form = false;
+  }
   bool col_ip = false, col_pf = false, col_ws = false;
   int row_var = 0;
   if (o.mode == GL_MODE_FUSED && !force_h && o.autotune && !sms_override) {
@@ -695,13 +934,14 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   if (rc == GL_ERR_SIZE && col_ip && o.col_inplace <= 0)  // the searched layout cannot: two buffers
     rc = choose_fused_geom(M, force_h, sms, &fg, cap_c, cap_r, false);
   if (rc != GL_OK) return rc;
+  int_form = int_form && choose_int_geom(fg.H, fg.W, &ig);
 
   gl_plan* pl = new (std::nothrow) gl_plan();
   if (!pl) return GL_ERR_NOMEM;
   pl->p = p; pl->N = N; pl->M = M; pl->LO = p / N; pl->n = n;
   pl->mode = o.mode; pl->device = o.device;
   pl->error_limit = o.error_limit; pl->check_every = o.check_every; pl->use_graphs = o.use_graphs;
-  pl->fg = fg; pl->pg = pg;
+  pl->fg = fg; pl->pg = pg; pl->ig = ig;
 
 #define GL_TRY(x)             \
   do {                        \
@@ -824,6 +1064,7 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   a.ll = ll; a.flags = fl; a.span = span; a.A = dA; a.Ainv = dAi; a.Z = Z; a.Z2 = Z2;
   a.twM = dtwM; a.twW = dtwW; a.twH = dtwH; a.twK1 = dK1; a.twPair = dPair; a.twK2 = dK2;
   a.digit = digit; a.hi = hi; a.status = status;
+  if (int_form) GL_TRY(build_int_tables(pl, vmax));
   *out = pl;
   int r = gl_reset(pl);
   if (r != GL_OK) {
@@ -857,7 +1098,11 @@ int gl_plan_describe(int p, int N, const gl_plan_opts* opts, gl_plan_info* info)
   if (o.batch_layout) sms = 1;
   int cap_c = kMaxRadix, cap_r = kMaxRadix;
   model_caps(tmp.M, o, o.batch_layout ? 1 : 0, &cap_c, &cap_r);
-  int rc = o.mode == GL_MODE_FUSED ? choose_fused_geom(tmp.M, o.fft_h, sms, &tmp.fg, cap_c, cap_r)
+  int vmax = 0;
+  const bool int_form = o.mode == GL_MODE_FUSED && !o.batch_layout && !names_fp64_variant(o) && int_range_ok(p, N, &vmax) &&
+                        int_roundoff_ok(p, N, o.error_limit);
+  const int int_h = int_form ? first_int_layout(tmp.M, sms) : 0;
+  int rc = o.mode == GL_MODE_FUSED ? choose_fused_geom(tmp.M, int_h ? int_h : o.fft_h, sms, &tmp.fg, cap_c, cap_r)
                                    : choose_plain_geom(tmp.M, &tmp.pg);
   if (rc != GL_OK) return rc;
   tmp.device = -1;
@@ -868,6 +1113,9 @@ int gl_plan_describe(int p, int N, const gl_plan_opts* opts, gl_plan_info* info)
     info->device_bytes = N8 /*ll*/ + 2 * (size_t)N /*flags, span*/ + 2 * N8 /*A, Ainv*/ +
                          5 * M * 16 /*Z, Z2, 3 twiddle tables*/ + stages * 16 + (size_t)N * 5 /*digit, hi*/ +
                          sizeof(Status) + residue_scratch_bytes(N);
+    IntGeom ig{};
+    if (int_h && choose_int_geom(tmp.fg.H, tmp.fg.W, &ig))
+      info->device_bytes += int_table_bytes(tmp.fg.H, tmp.fg.W, ig);
   }
   return r;
 }
@@ -909,6 +1157,7 @@ int gl_reset(gl_plan* pl) {
   GL_CUDA(cudaMemsetAsync(pl->args.status, 0, sizeof(Status), pl->stream));
   GL_CUDA(cudaStreamSynchronize(pl->stream));
   pl->iters_done = 0;
+  pl->since_fp64 = 0;
   pl->run_maxerr = 0.0;
   pl->from_state = false;
   pl->carry_valid = true;
@@ -1010,7 +1259,8 @@ int gl_profile_kernels(gl_plan* pl, int iters, double* ms_out, const char** name
   for (int it = 0; it < iters && rc == GL_OK; ++it) {
     for (int k = 0; k < 3; ++k) {
       if (cudaEventRecord(ev[k], pl->stream) != cudaSuccess) { rc = GL_ERR_CUDA; break; }
-      if (launch_fused_kernel(pl->args, pl->fg, pl->stream, k) != cudaSuccess) { rc = GL_ERR_CUDA; break; }
+      if ((pl->int_form ? launch_int_kernel(pl->args, pl->ig, pl->stream, k)
+                        : launch_fused_kernel(pl->args, pl->fg, pl->stream, k)) != cudaSuccess) { rc = GL_ERR_CUDA; break; }
     }
     if (rc != GL_OK) break;
     if (cudaEventRecord(ev[3], pl->stream) != cudaSuccess || cudaEventSynchronize(ev[3]) != cudaSuccess) {
@@ -1082,7 +1332,7 @@ struct HostStep {
 // the status into the mapped host buffers, so that transfer runs under the kernel instead
 // of as copies after it.  Enqueued on the plan's stream (captured into a graph by the
 // caller).
-static cudaError_t enqueue_host_step(gl_plan* pl, const HostStep& hs, Status* status_dev) {
+static cudaError_t enqueue_host_step(gl_plan* pl, const HostStep& hs, Status* status_dev, bool integer) {
   const size_t N = (size_t)pl->N;
   cudaError_t e;
   if ((e = cudaMemcpyAsync(pl->args.digit, hs.in[0], sizeof(int32_t) * N, cudaMemcpyHostToDevice, pl->stream)))
@@ -1091,7 +1341,11 @@ static cudaError_t enqueue_host_step(gl_plan* pl, const HostStep& hs, Status* st
   else e = cudaMemcpyAsync(pl->args.hi, hs.in[1], N, cudaMemcpyHostToDevice, pl->stream);
   if (e) return e;
   if ((e = cudaMemsetAsync(pl->args.status, 0, sizeof(Status), pl->stream))) return e;
-  if ((e = launch_fused_iteration(pl->args, pl->fg, pl->stream, true))) return e;
+  // the integer form's load checks the words against its bound, and the dicing below leaves
+  // the buffers alone if one is beyond it
+  e = integer ? launch_int_iteration(pl->args, pl->ig, pl->stream, true)
+              : launch_fused_iteration(pl->args, pl->fg, pl->stream, true);
+  if (e) return e;
   if (hs.kind == 1) return launch_dice_words(pl->args, true, pl->stream, (int32_t*)hs.out_dev[0], status_dev);
   return launch_dice_perm(pl->args, pl->stream, (int*)hs.out_dev[0], (signed char*)hs.out_dev[1], status_dev);
 }
@@ -1105,28 +1359,17 @@ static bool host_step_mapped(gl_plan* pl, int64_t iters, HostStep* hs, Status** 
   return (*status_dev = (Status*)mapped_host(pl->h_status)) != nullptr;
 }
 
-// Records the start event and launches the step as one graph (about ten calls fewer per
-// step), built on the first call for these buffers and kept by the plan.
-static int launch_host_step(gl_plan* pl, const HostStep& hs, Status* status_dev) {
-  bool same = pl->hw_exec && pl->hw_kind == hs.kind;
+// Launches the step between ev0 and ev1 as one graph (about ten calls fewer per
+// step), built on the first call for these buffers and kept by the plan: one graph in FP64,
+// one in the integer form.
+static int launch_host_step(gl_plan* pl, const HostStep& hs, Status* status_dev, bool integer) {
+  bool same = pl->hw_kind == hs.kind;
   for (int i = 0; i < 2; ++i)
     same = same && pl->hw_in[i] == hs.in[i] && pl->hw_out[i] == hs.out[i] && pl->hw_out_dev[i] == hs.out_dev[i];
   if (!same) {
-    if (pl->hw_exec) cudaGraphExecDestroy(pl->hw_exec);
-    pl->hw_exec = nullptr;
-    cudaGraph_t graph = nullptr;
-    GL_CUDA(cudaStreamBeginCapture(pl->stream, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t es = enqueue_host_step(pl, hs, status_dev);
-    const cudaError_t ec = cudaStreamEndCapture(pl->stream, &graph);
-    if (es != cudaSuccess || ec != cudaSuccess || !graph) {
-      if (graph) cudaGraphDestroy(graph);
-      return GL_ERR_CUDA;
-    }
-    const cudaError_t ei = cudaGraphInstantiate(&pl->hw_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ei != cudaSuccess) {
-      pl->hw_exec = nullptr;
-      return GL_ERR_CUDA;
+    for (cudaGraphExec_t& g : pl->hw_exec) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
     }
     pl->hw_kind = hs.kind;
     for (int i = 0; i < 2; ++i) {
@@ -1135,18 +1378,32 @@ static int launch_host_step(gl_plan* pl, const HostStep& hs, Status* status_dev)
       pl->hw_out_dev[i] = hs.out_dev[i];
     }
   }
+  cudaGraphExec_t& exec = pl->hw_exec[integer ? 1 : 0];
+  if (!exec) {
+    cudaGraph_t graph = nullptr;
+    GL_CUDA(cudaStreamBeginCapture(pl->stream, cudaStreamCaptureModeThreadLocal));
+    const cudaError_t es = enqueue_host_step(pl, hs, status_dev, integer);
+    const cudaError_t ec = cudaStreamEndCapture(pl->stream, &graph);
+    if (es != cudaSuccess || ec != cudaSuccess || !graph) {
+      if (graph) cudaGraphDestroy(graph);
+      return GL_ERR_CUDA;
+    }
+    const cudaError_t ei = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (ei != cudaSuccess) {
+      exec = nullptr;
+      return GL_ERR_CUDA;
+    }
+  }
   GL_CUDA(cudaEventRecord(pl->ev0, pl->stream));
-  GL_CUDA(cudaGraphLaunch(pl->hw_exec, pl->stream));
-  pl->from_state = false;
-  pl->iters_done += 1;
-  pl->carry_valid = true;  // the device (digit, hi) is the state the host received
+  GL_CUDA(cudaGraphLaunch(exec, pl->stream));
+  GL_CUDA(cudaEventRecord(pl->ev1, pl->stream));
   return GL_OK;
 }
 
-// The end of a host-state call whose work is enqueued after ev0: wait for it, read the
-// status it left in pl->h_status, report.
-static int finish_host_step(gl_plan* pl, int64_t iters, gl_iter_report* rep) {
-  GL_CUDA(cudaEventRecord(pl->ev1, pl->stream));
+// Report of a host-state call whose work lies between ev0 and ev1: wait for it, read the
+// status it left in pl->h_status.
+static int report_host_step(gl_plan* pl, int64_t iters, gl_iter_report* rep) {
   GL_CUDA(cudaEventSynchronize(pl->ev1));
   const double e = std::ldexp((double)pl->h_status->maxerr64, -64);
   if (e > pl->run_maxerr) pl->run_maxerr = e;
@@ -1166,6 +1423,28 @@ static int finish_host_step(gl_plan* pl, int64_t iters, gl_iter_report* rep) {
   return st;
 }
 
+static int finish_host_step(gl_plan* pl, int64_t iters, gl_iter_report* rep) {
+  GL_CUDA(cudaEventRecord(pl->ev1, pl->stream));
+  return report_host_step(pl, iters, rep);
+}
+
+// The captured step from launch to report.  A state with a word beyond the integer form's
+// bound has left the buffers as they were, and the step runs again in FP64.
+static int run_host_step(gl_plan* pl, const HostStep& hs, Status* status_dev, gl_iter_report* rep) {
+  bool integer = pl->int_form && ++pl->since_fp64 < kFp64Every;
+  int rc = launch_host_step(pl, hs, status_dev, integer);
+  if (rc == GL_OK && integer) {
+    GL_CUDA(cudaEventSynchronize(pl->ev1));
+    if (pl->h_status->flags & kStatusWide) rc = launch_host_step(pl, hs, status_dev, integer = false);
+  }
+  if (rc != GL_OK) return rc;
+  if (!integer) pl->since_fp64 = 0;
+  pl->from_state = false;
+  pl->iters_done += 1;
+  pl->carry_valid = true;  // the device (digit, hi) is the state the host received
+  return report_host_step(pl, 1, rep);
+}
+
 int gl_iterate_host(gl_plan* pl, const int32_t* digit_in, const int8_t* hi_in, int64_t iters, int32_t* digit_out,
                     int8_t* hi_out, gl_iter_report* rep) {
   if (!pl || !digit_in || !hi_in || !digit_out || !hi_out || iters < 0) return GL_ERR_ARG;
@@ -1173,11 +1452,7 @@ int gl_iterate_host(gl_plan* pl, const int32_t* digit_in, const int8_t* hi_in, i
   const size_t N = (size_t)pl->N;
   HostStep hs{2, {digit_in, hi_in}, {digit_out, hi_out}, {nullptr, nullptr}};
   Status* status_dev = nullptr;
-  if (host_step_mapped(pl, iters, &hs, &status_dev)) {
-    const int rc = launch_host_step(pl, hs, status_dev);
-    if (rc != GL_OK) return rc;
-    return finish_host_step(pl, iters, rep);
-  }
+  if (host_step_mapped(pl, iters, &hs, &status_dev)) return run_host_step(pl, hs, status_dev, rep);
   GL_CUDA(cudaEventRecord(pl->ev0, pl->stream));
   GL_CUDA(cudaMemcpyAsync(pl->args.digit, digit_in, sizeof(int32_t) * N, cudaMemcpyHostToDevice, pl->stream));
   GL_CUDA(cudaMemcpyAsync(pl->args.hi, hi_in, N, cudaMemcpyHostToDevice, pl->stream));
@@ -1205,11 +1480,7 @@ int gl_iterate_host_words(gl_plan* pl, const int32_t* words_in, int64_t iters, i
   const size_t N = (size_t)pl->N;
   HostStep hs{1, {words_in, nullptr}, {words_out, nullptr}, {nullptr, nullptr}};
   Status* status_dev = nullptr;
-  if (host_step_mapped(pl, iters, &hs, &status_dev)) {
-    const int rc = launch_host_step(pl, hs, status_dev);
-    if (rc != GL_OK) return rc;
-    return finish_host_step(pl, iters, rep);
-  }
+  if (host_step_mapped(pl, iters, &hs, &status_dev)) return run_host_step(pl, hs, status_dev, rep);
   GL_CUDA(cudaEventRecord(pl->ev0, pl->stream));
   GL_CUDA(cudaMemcpyAsync(pl->args.digit, words_in, sizeof(int32_t) * N, cudaMemcpyHostToDevice, pl->stream));
   GL_CUDA(cudaMemsetAsync(pl->args.hi, 0, N, pl->stream));
@@ -1333,7 +1604,8 @@ int gl_mersenne_test(gl_plan* pl, int64_t iters, gl_result* res) {
 
 int gl_error_test(int p, int N, const gl_plan_opts* opts, int iters, gl_iter_report* rep) {
   gl_plan* pl = nullptr;
-  int rc = gl_plan_create(p, N, opts, &pl);
+  // a round-off trial: FP64 in every iteration
+  int rc = gl_plan_create_ex(p, N, opts, opts && opts->batch_layout ? 1 : 0, &pl, true);
   if (rc != GL_OK) return rc;
   if (iters <= 0) {
     iters = p / 10000;
@@ -1372,7 +1644,7 @@ int gl_find_signal_size(int p, const gl_plan_opts* opts, int* N_out, double* ms_
   for (int N : cand) {
     if (first && N > first + first / 7) break;  // within ~15 % of the smallest accepted
     gl_plan* pl = nullptr;
-    int rc = gl_plan_create(p, N, &o, &pl);
+    int rc = gl_plan_create_ex(p, N, &o, o.batch_layout ? 1 : 0, &pl, true);  // measures the round-off
     if (rc == GL_ERR_NOMEM || rc == GL_ERR_NODEVICE || rc == GL_ERR_CUDA) return rc;
     if (rc != GL_OK) continue;
     gl_iter_report rep{};

@@ -1,0 +1,72 @@
+// gl_dice.cuh -- the load of one complex point in the forward column passes (FP64 and
+// integer form): dice the previous products into balanced digits and carries, add the
+// carry of the word below.
+#pragma once
+#include "gl_device.cuh"
+#include "gl_internal.h"
+
+namespace gl {
+
+// Words j0 = 2m, j0+1 of point m = m1 + W m2 as (v0, v1): from the carry-save state, or by
+// dicing the products with carry depth NC (llintToIrrBal<n>).  The digit sums of j0-1, j0,
+// j0+1 need the products of words j0-1-NC .. j0+1: P[k] = product of word j0+1-k,
+// k = 0 .. NC+2.  Words j0+1-2d and j0-2d are the two words of point m-d, column m1-d of
+// the same row (the previous row, from the last columns, when m1 < d), adjacent in the
+// column-major layout: one 16-byte load per point, and no division to find it.
+template <bool FROM_STATE, int NC>
+__device__ __forceinline__ void load_point(const IterArgs& a, const int m1, const int m2, int* v0, int* v1) {
+  const int H = a.H, W = a.W, N = a.N, LO = a.LO;
+  constexpr int D = (NC + 2) / 2;  // points m-1 .. m-D hold the words j0-1 .. j0+1-(NC+2)
+  const int s0 = 2 * (m1 * H + m2);
+  if (FROM_STATE) {
+    const int j0 = 2 * (m1 + W * m2);
+    *v0 = a.digit[j0] + (int)a.hi[j0 == 0 ? N - 1 : j0 - 1];
+    *v1 = a.digit[j0 + 1] + (int)a.hi[j0];
+  } else {
+    long long P[NC + 3];
+    const longlong2 own = __ldg(reinterpret_cast<const longlong2*>(a.ll + s0));
+    P[0] = own.y;
+    P[1] = own.x;
+    uint32_t fm = 0;  // flags of word j0-1 (the upper word of point m-1)
+#pragma unroll
+    for (int d = 1; d <= D; ++d) {
+      int c = m1 - d, r = m2;
+      if (c < 0) {  // one wrap suffices: layouts have W >= 4 >= D
+        c += W;
+        r = r == 0 ? H - 1 : r - 1;
+      }
+      const int sd = 2 * (c * H + r);
+      if (d == 1) fm = __ldg(a.flags + sd + 1);
+      if (2 * d + 1 < NC + 3) {
+        const longlong2 v = __ldg(reinterpret_cast<const longlong2*>(a.ll + sd));
+        P[2 * d] = v.y;
+        P[2 * d + 1] = v.x;
+      } else {  // only the upper word of the farthest point
+        P[2 * d] = __ldg(a.ll + sd + 1);
+      }
+    }
+    const uint32_t f0 = __ldg(a.flags + s0), f1 = __ldg(a.flags + s0 + 1);
+    auto dice_at = [&](uint32_t f, int off) {
+      const long long mask = (1ll << (LO + (int)(f & 1))) - 1;
+      const long long v = P[off];
+      long long sum = v < 0 ? -((-v) & mask) : (v & mask);
+      int shift = 0;
+#pragma unroll
+      for (int i = 1; i <= NC; ++i) {
+        shift += LO + (int)((f >> i) & 1);
+        const long long w = P[off + i];
+        sum += shift >= 63 ? 0 : (w < 0 ? -(((-w) >> shift) & mask) : ((w >> shift) & mask));
+      }
+      return sum;
+    };
+    const long long sw1 = dice_at(f1, 0), sw0 = dice_at(f0, 1), sm1 = dice_at(fm, 2);
+    int dm, hm, d0, h0, d1, h1;
+    balanced_split(sm1, LO + (int)(fm & 1), &dm, &hm);
+    balanced_split(sw0, LO + (int)(f0 & 1), &d0, &h0);
+    balanced_split(sw1, LO + (int)(f1 & 1), &d1, &h1);
+    *v0 = d0 + hm;
+    *v1 = d1 + h0;
+  }
+}
+
+}  // namespace gl

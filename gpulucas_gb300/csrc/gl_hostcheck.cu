@@ -1,6 +1,7 @@
 // gl_hostcheck.cu -- the device arithmetic helpers (small DFTs, integer-domain
 // rounding and conversion, dicing) compiled for the host, so the CPU test suite can
 // check them against numpy and the oracle without a GPU.  Not used by the product.
+#include <algorithm>
 #include <cstdint>
 
 #include "gl_device.cuh"
@@ -205,3 +206,125 @@ extern "C" int hc_line_fft(int L, const int* radices, int nst, int sign, double*
   }
   return 0;
 }
+
+// ---------------------------------------------------------------------------
+// The integer form's field arithmetic and tables (gl_gf61.cuh, gl_tables.cpp)
+// ---------------------------------------------------------------------------
+#include "gl_gf61.cuh"
+
+namespace {
+using gl::gf::g2;
+
+__host__ __device__ int4 tw4(const gl::HostTw& w) { return make_int4(w.c0, w.c1, w.d0, w.d1); }
+
+struct GfIn {
+  const g2* a;
+  int step;
+  __host__ __device__ g2 operator()(int q) const { return a[q * step]; }
+};
+struct GfSlot {
+  const gl::HostTw* tw;
+  int step;
+  __host__ __device__ int4 operator()(int q) const { return tw4(tw[q * step]); }
+};
+
+// One line of L points, stride st, transformed as the integer form's stages do; *peak: the
+// largest magnitude of a stage's output.
+template <int S>
+void gf_line(g2* x, int st, int L, const std::vector<int>& radices, int64_t* peak) {
+  std::vector<gl::HostTw> tw;
+  std::vector<int> off(radices.size() + 1);
+  gl::gf_stage_twiddles(L, radices.data(), (int)radices.size(), S > 0, tw, off.data());
+  std::vector<g2> a((size_t)L), b((size_t)L);
+  for (int i = 0; i < L; ++i) a[i] = x[(size_t)i * st];
+  int Ns = 1;
+  for (size_t s = 0; s < radices.size(); ++s) {
+    const int R = radices[s], LR = L / R;
+    for (int j = 0; j < LR; ++j) {
+      const int k = j % Ns;
+      g2 v[8];
+      const GfIn in{a.data() + j, LR};
+      const GfSlot slot{tw.data() + off[s] + k, Ns};
+      switch (R) {
+        case 2: gl::gf::butterfly<2, S>(v, Ns > 1, in, slot); break;
+        case 3: gl::gf::butterfly<3, S>(v, Ns > 1, in, slot); break;
+        case 4: gl::gf::butterfly<4, S>(v, Ns > 1, in, slot); break;
+        case 5: gl::gf::butterfly<5, S>(v, Ns > 1, in, slot); break;
+        case 7: gl::gf::butterfly<7, S>(v, Ns > 1, in, slot); break;
+        default: gl::gf::butterfly<8, S>(v, Ns > 1, in, slot); break;
+      }
+      for (int q = 0; q < R; ++q) {
+        b[(j - k) * R + k + q * Ns] = v[q];
+        for (int64_t m : {v[q].re, v[q].im}) *peak = std::max(*peak, m < 0 ? -m : m);
+      }
+    }
+    std::swap(a, b);
+    Ns *= R;
+  }
+  for (int i = 0; i < L; ++i) x[(size_t)i * st] = a[i];
+}
+}  // namespace
+
+extern "C" {
+
+// out = the unweighted products of the words v (N = 2 W H of them) by the integer form's
+// passes on an H x W layout; returns 0, or -1 where the field lacks the roots.  *peak: the
+// largest magnitude of a transform stage's output.
+int hc_gf_square(int p, int W, int H, const int* v, long long* out, long long* peak) {
+  const int M = W * H, N = 2 * M;
+  if (!gl::gf_supported(M)) return -1;
+  std::vector<uint8_t> e;
+  std::vector<gl::HostTw> k1, pair, k2;
+  std::vector<gl::RowPair> rows;
+  gl::gf_weights(p, N, e);
+  gl::gf_pass_tables(W, H, k1, pair, k2);
+  gl::gf_row_pairs(W, H, rows);
+  const std::vector<int> rw = gl::radix_plan(W, 8), rh = gl::radix_plan(H, 8);
+  int64_t pk = 0;
+  std::vector<g2> z((size_t)M);
+  for (int m = 0; m < M; ++m)
+    z[m] = g2{gl::gf::weighted(v[2 * m], e[2 * m]), gl::gf::weighted(v[2 * m + 1], e[2 * m + 1])};
+  for (int m1 = 0; m1 < W; ++m1) {
+    gf_line<-1>(&z[m1], W, H, rh, &pk);
+    for (int k = 0; k < H; ++k) z[k * W + m1] = gl::gf::cmul(z[k * W + m1], tw4(k1[m1 * H + k]));
+  }
+  const int qW = (int)(gl::gf::kQ % (uint64_t)W);
+  for (const gl::RowPair& r : rows) {
+    g2 *za = &z[(size_t)r.a * W], *zb = &z[(size_t)r.b * W];
+    gf_line<-1>(za, 1, W, rw, &pk);
+    if (za != zb) gf_line<-1>(zb, 1, W, rw, &pk);
+    for (int t = 0; t < W; ++t) {
+      const int u = (int)(((int64_t)qW * t + r.shift) % W);
+      if (za == zb && u < t) continue;
+      g2 vk, vkp;
+      gl::gf::pair_square(za[t], zb[u], tw4(pair[r.a * W + t]), &vk, &vkp);
+      za[t] = vk;
+      if (za != zb || t != u) zb[u] = vkp;
+    }
+    gf_line<+1>(za, 1, W, rw, &pk);
+    if (za != zb) gf_line<+1>(zb, 1, W, rw, &pk);
+    for (int t = 0; t < W; ++t) {
+      za[t] = gl::gf::cmul(za[t], tw4(k2[r.a * W + t]));
+      if (za != zb) zb[t] = gl::gf::cmul(zb[t], tw4(k2[r.b * W + t]));
+    }
+  }
+  for (int m1 = 0; m1 < W; ++m1) gf_line<+1>(&z[m1], W, H, rh, &pk);
+  for (int m = 0; m < M; ++m) {
+    out[2 * m] = gl::gf::unweighted(z[m].re, e[2 * m]);
+    out[2 * m + 1] = gl::gf::unweighted(z[m].im, e[2 * m + 1]);
+  }
+  *peak = pk;
+  return 0;
+}
+
+// (re, im) x (c + i d) as the kernels compute it (|re|, |im| < 2^62; c, d residues)
+void hc_gf_cmul(const long long* x, const unsigned long long* w, long long* out) {
+  const g2 r = gl::gf::cmul(g2{x[0], x[1]}, tw4(gl::gf_pack(w[0], w[1])));
+  out[0] = r.re;
+  out[1] = r.im;
+}
+long long hc_gf_red(long long x) { return gl::gf::red(x); }
+long long hc_gf_weighted(int v, int e) { return gl::gf::weighted(v, e); }
+long long hc_gf_unweighted(long long x, int e) { return gl::gf::unweighted(x, e); }
+
+}  // extern "C"

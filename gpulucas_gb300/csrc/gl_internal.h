@@ -39,6 +39,7 @@ struct Status {
 };
 constexpr unsigned kStatusBig = 1u;    // |product| >= 2^51: doubles cannot hold it exactly
 constexpr unsigned kStatusSlice = 2u;  // product bits beyond what n+1 slices place
+constexpr unsigned kStatusWide = 8u;   // a word of a loaded state is beyond the integer form's bound
 constexpr unsigned kStatusTimeout = 4u; // a bounded device-side wait ran out (kernel returned)
 
 // Geometry of the fused form: the N/2 complex points are an H x W array
@@ -73,6 +74,37 @@ struct PlainGeom {
   int threads;
 };
 
+// padded line stride of the integer form's shared-memory lines (16-byte slots): a slot of
+// padding every 8, since a radix-8 stage's first writes go to stride 8 and a warp's
+// 16-byte accesses are served eight lanes at a time
+constexpr int int_stride(int L) { return L + (L >> 3) + 1; }
+constexpr int kMaxIntSmem = 120 * 1024;
+
+// Geometry of the integer form (gl_int_kernels.cu) on the same H x W array.
+struct IntGeom {
+  int t_col, t_row;        // threads per CTA
+  size_t sm_col, sm_row;   // dynamic shared memory bytes
+  LinePlan pw, ph;         // line plans (offsets into the stage tables)
+};
+// Tables of the integer form: twiddles as four 31-bit limbs (gl_gf61.cuh), row pairs as
+// (row a, row b, shift, 0).
+struct IntArgs {
+  const int4* wf;             // stage values of the length-W line DFT, forward
+  const int4* wi;             // and inverse
+  const int4* hf;             // length H
+  const int4* hi;
+  const int4* k1;             // root(m1 k2, M) at m1*H + k2
+  const int4* pair;           // -(1 + root(k2 + H k1, M))/4 at k2*W + k1
+  const int4* k2;             // root(-m1 k2, M)/M at k2*W + m1
+  const int4* rows;           // row pairs
+  const unsigned char* e;     // weight exponents (column-major)
+  int nrows;                  // number of row pairs
+  int qW;                     // 2^61 - 1 mod W
+  int vmax;                   // bound on a loaded word's magnitude
+  int ls_col, ls_row;
+  LinePlan pw, ph;
+};
+
 // Arguments of one iteration (passed by value to every kernel).
 struct IterArgs {
   int N, M, W, H, G, LO, n;
@@ -95,6 +127,7 @@ struct IterArgs {
   signed char* hi;            // plain: i_hiBitArr, N
   Status* status;
   LinePlan pw, ph;
+  IntArgs in;                 // integer form (in.k1 null: this test has none)
 };
 
 // Resident form of a fused plan (short lengths): one thread-block cluster of C CTAs keeps
@@ -139,6 +172,12 @@ struct BatchLaunch {
 cudaError_t launch_fused_iteration(const IterArgs& a, const FusedGeom& g, cudaStream_t s, bool from_state);
 // one of the three fused kernels (0 = k_col_fwd, 1 = k_row_sq, 2 = k_col_inv)
 cudaError_t launch_fused_kernel(const IterArgs& a, const FusedGeom& g, cudaStream_t s, int which);
+// The same iteration in exact integer arithmetic over GF((2^61-1)^2): the products equal the
+// FP64 form's bit for bit; only the range flags of the status are written.  A loaded state
+// (from_state) with a word beyond a.in.vmax sets kStatusWide and its products are invalid.
+cudaError_t launch_int_iteration(const IterArgs& a, const IntGeom& g, cudaStream_t s, bool from_state);
+cudaError_t launch_int_kernel(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which);
+cudaError_t set_int_smem_limits();
 cudaError_t launch_plain_iteration(const IterArgs& a, const PlainGeom& g, cudaStream_t s);
 cudaError_t launch_set_initial(const IterArgs& a, int mode, cudaStream_t s);
 // carry-save state (digit, hi) = dice(ll) for the fused form; plain keeps it already

@@ -23,6 +23,7 @@
 #include <cooperative_groups.h>
 
 #include "gl_device.cuh"
+#include "gl_dice.cuh"
 #include "gl_internal.h"
 
 namespace gl {
@@ -258,74 +259,19 @@ __device__ __forceinline__ int colmajor(const IterArgs& a, int j) {
 // Fused kernels (one column / one row pair per CTA)
 // ---------------------------------------------------------------------------
 
-// Column pass, forward.  NC = carry depth n of llintToIrrBal<n>.  For words
-// j0 = 2m, j0+1 the digit sums of j0-1, j0, j0+1 need the products of words
-// j0-1-NC .. j0+1: P[k] = product of word j0+1-k, k = 0 .. NC+2.  Words j0+1-2d and
-// j0-2d are the two words of point m-d, column m1-d of the same row (the previous row,
-// from the last columns, when m1 < d), adjacent in the column-major layout: one 16-byte
-// load per point, and no division to find it.
+// Column pass, forward.  NC = carry depth n of llintToIrrBal<n>.
 // Loads column m1 into buf (threads tid, tid + nth, ...): dice the previous products into
 // balanced digits and carries, add the carry of the word below, weight.
 template <bool FROM_STATE, int NC>
 __device__ __forceinline__ void col_fwd_load(const IterArgs& a, const int m1, cplx* buf, int tid, int nth) {
-  const int H = a.H, W = a.W, N = a.N, LO = a.LO;
-  constexpr int D = (NC + 2) / 2;  // points m-1 .. m-D hold the words j0-1 .. j0+1-(NC+2)
+  const int H = a.H;
   // two points' loads in flight per thread (C3: 0.3038 -> 0.3016 ms per iteration); four,
   // or unrolling the passes' other per-point loops as well, spills registers
 #pragma unroll 2
   for (int m2 = tid; m2 < H; m2 += nth) {
-    const int s0 = 2 * (m1 * H + m2);
     int v0, v1;
-    if (FROM_STATE) {
-      const int j0 = 2 * (m1 + W * m2);
-      v0 = a.digit[j0] + (int)a.hi[j0 == 0 ? N - 1 : j0 - 1];
-      v1 = a.digit[j0 + 1] + (int)a.hi[j0];
-    } else {
-      long long P[NC + 3];
-      const longlong2 own = __ldg(reinterpret_cast<const longlong2*>(a.ll + s0));
-      P[0] = own.y;
-      P[1] = own.x;
-      uint32_t fm = 0;  // flags of word j0-1 (the upper word of point m-1)
-#pragma unroll
-      for (int d = 1; d <= D; ++d) {
-        int c = m1 - d, r = m2;
-        if (c < 0) {  // one wrap suffices: layouts have W >= 4 >= D
-          c += W;
-          r = r == 0 ? H - 1 : r - 1;
-        }
-        const int sd = 2 * (c * H + r);
-        if (d == 1) fm = __ldg(a.flags + sd + 1);
-        if (2 * d + 1 < NC + 3) {
-          const longlong2 v = __ldg(reinterpret_cast<const longlong2*>(a.ll + sd));
-          P[2 * d] = v.y;
-          P[2 * d + 1] = v.x;
-        } else {  // only the upper word of the farthest point
-          P[2 * d] = __ldg(a.ll + sd + 1);
-        }
-      }
-      const uint32_t f0 = __ldg(a.flags + s0), f1 = __ldg(a.flags + s0 + 1);
-      auto dice_at = [&](uint32_t f, int off) {
-        const long long mask = (1ll << (LO + (int)(f & 1))) - 1;
-        const long long v = P[off];
-        long long sum = v < 0 ? -((-v) & mask) : (v & mask);
-        int shift = 0;
-#pragma unroll
-        for (int i = 1; i <= NC; ++i) {
-          shift += LO + (int)((f >> i) & 1);
-          const long long w = P[off + i];
-          sum += shift >= 63 ? 0 : (w < 0 ? -(((-w) >> shift) & mask) : ((w >> shift) & mask));
-        }
-        return sum;
-      };
-      const long long sw1 = dice_at(f1, 0), sw0 = dice_at(f0, 1), sm1 = dice_at(fm, 2);
-      int dm, hm, d0, h0, d1, h1;
-      balanced_split(sm1, LO + (int)(fm & 1), &dm, &hm);
-      balanced_split(sw0, LO + (int)(f0 & 1), &d0, &h0);
-      balanced_split(sw1, LO + (int)(f1 & 1), &d1, &h1);
-      v0 = d0 + hm;
-      v1 = d1 + h0;
-    }
-    const double2 A = __ldg(reinterpret_cast<const double2*>(a.A + s0));
+    load_point<FROM_STATE, NC>(a, m1, m2, &v0, &v1);
+    const double2 A = __ldg(reinterpret_cast<const double2*>(a.A + 2 * (m1 * H + m2)));
     buf[pad(m2)] = mk(A.x * dbl_from_int(v0), A.y * dbl_from_int(v1));
   }
 }
@@ -874,7 +820,7 @@ cudaError_t launch_permute_words(const IterArgs& a, const long long* src, long l
 __global__ void k_dice_perm(IterArgs a, int* host_digit, signed char* host_hi, Status* host_status) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (host_status && j == 0) *host_status = *a.status;  // final: the passes before have ended
-  if (j >= a.N) return;
+  if (j >= a.N || (a.status->flags & kStatusWide)) return;  // products not valid: keep the state
   const int N = a.N;
   const uint32_t f = a.flags[colmajor(a, j)];
   const long long s = dice_sum(a.LO, a.n, f, [&](int i) {
@@ -910,7 +856,7 @@ __global__ void k_dice_words(IterArgs a, int32_t* host_words, Status* host_statu
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int N = a.N;
   if (host_status && j == 0) *host_status = *a.status;  // final: the passes before have ended
-  if (j >= N) return;
+  if (j >= N || (a.status->flags & kStatusWide)) return;  // products not valid: keep the state
   auto pos = [&](int k) {
     if (k < 0) k += N;
     return CM ? colmajor(a, k) : k;

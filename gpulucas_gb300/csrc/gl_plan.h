@@ -6,6 +6,7 @@
 #include "gl_internal.h"
 
 using gl::FusedGeom;
+using gl::IntGeom;
 using gl::IterArgs;
 using gl::PlainGeom;
 using gl::ResidentGeom;
@@ -20,6 +21,9 @@ struct gl_plan {
   cudaStream_t stream = nullptr;
   FusedGeom fg{};
   PlainGeom pg{};
+  IntGeom ig{};
+  bool int_form = false;       // most iterations run in exact integer arithmetic
+  int since_fp64 = 0;          // integer iterations since the last FP64 one
   IterArgs args{};
   std::vector<void*> allocs;
   Status* h_status = nullptr;  // pinned
@@ -32,7 +36,7 @@ struct gl_plan {
   // gl_iterate_host_words / gl_iterate_host, one iteration between pinned host buffers:
   // the whole step (copies in, from-state iteration, dicing stored straight into the
   // mapped output buffers and status) as one graph, kept for one set of buffers
-  cudaGraphExec_t hw_exec = nullptr;
+  cudaGraphExec_t hw_exec[2] = {nullptr, nullptr};  // FP64, integer form
   int hw_kind = 0;                  // 1: words step, 2: carry-save pair step
   const void* hw_in[2] = {nullptr, nullptr};
   void* hw_out[2] = {nullptr, nullptr};
@@ -48,7 +52,9 @@ struct gl_plan {
 
 // gl_plan_create with an explicit SM count for the layout cost model (1 = a member of
 // a batch: minimise total work, the batch spreads units over the device).
-int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, gl_plan** out);
+// fp64_only: no integer form (round-off trials).
+int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, gl_plan** out,
+                      bool fp64_only = false);
 // iterations done outside the plan's own launches (by a batch): bookkeeping only
 void gl_plan_note_external_iterations(gl_plan* pl, int64_t iters);
 // non-blocking stream; level 0: normal priority, 1: the device's highest, 2: between

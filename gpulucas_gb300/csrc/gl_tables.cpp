@@ -8,6 +8,8 @@
 // one octant by integer arithmetic on the angle's numerator.
 #include "gl_tables.h"
 
+#include "gl_gf61.cuh"
+
 #include <cmath>
 #include <cstring>
 #include <thread>
@@ -343,6 +345,181 @@ std::vector<int> radix_plan(int n, int max_radix) {
   int buf[64];
   const int count = radix_plan_into(n, max_radix, buf, 64);
   return count < 0 ? std::vector<int>() : std::vector<int>(buf, buf + count);
+}
+
+// ---------------------------------------------------------------------------
+// GF(q^2), q = 2^61 - 1: roots of unity and the tables of the integer form
+// ---------------------------------------------------------------------------
+namespace {
+struct Gf {
+  uint64_t re, im;
+};
+uint64_t addq(uint64_t a, uint64_t b) {
+  const uint64_t s = a + b;
+  return s >= gf::kQ ? s - gf::kQ : s;
+}
+uint64_t negq(uint64_t a) { return a ? gf::kQ - a : 0; }
+Gf gmul(Gf a, Gf b) {
+  return {addq(gf::mulq(a.re, b.re), negq(gf::mulq(a.im, b.im))), addq(gf::mulq(a.re, b.im), gf::mulq(a.im, b.re))};
+}
+Gf gpow(Gf a, uint64_t e) {
+  Gf r{1, 0};
+  for (; e; e >>= 1) {
+    if (e & 1) r = gmul(r, a);
+    a = gmul(a, a);
+  }
+  return r;
+}
+
+// A root of order 2^k for every k: 1, -1, -i, 2^30 (1 - i), then square roots inside the
+// norm-1 group: z = (x, y) of norm 1 has the root (z + 1)/sqrt(2 + 2x), since
+// (z + 1)^2 = z (z + 2 + 1/z) = z (2 + 2x); q = 3 mod 4 gives sqrt(a) = a^((q+1)/4).
+constexpr int kPow2Roots = 41;
+struct Pow2Roots {
+  Gf z[kPow2Roots];
+  Pow2Roots() {
+    z[0] = {1, 0};
+    z[1] = {gf::kQ - 1, 0};
+    z[2] = {0, gf::kQ - 1};
+    z[3] = {1ull << 30, gf::kQ - (1ull << 30)};
+    for (int k = 3; k + 1 < kPow2Roots; ++k) {
+      const uint64_t s = gf::powq(addq(2, addq(z[k].re, z[k].re)), (gf::kQ + 1) / 4);
+      const uint64_t inv = gf::powq(s, gf::kQ - 2);
+      z[k + 1] = {gf::mulq(addq(z[k].re, 1), inv), gf::mulq(z[k].im, inv)};
+    }
+  }
+};
+
+int64_t inv_mod(int64_t a, int64_t m) {
+  for (int64_t x = 1; x < m; ++x)
+    if (a % m * x % m == 1) return x;
+  return 0;  // m == 1
+}
+
+Gf groot(int64_t t, int64_t L) {
+  static const Pow2Roots pr;
+  t %= L;
+  if (t < 0) t += L;
+  int a = 0;
+  int64_t odd = L;
+  while (!(odd & 1)) {
+    odd >>= 1;
+    ++a;
+  }
+  const int64_t two = (int64_t)1 << a;
+  // t/L = u2/2^a + sum u_r/r mod 1 over the odd prime powers r of L
+  // odd^-1 mod 2^a by Newton
+  uint64_t x = 1;
+  for (int i = 0; i < 6; ++i) x *= 2 - (uint64_t)odd * x;
+  Gf w = gpow(pr.z[a], ((uint64_t)t * x) & (uint64_t)(two - 1));
+  uint64_t s = 1;
+  for (int64_t pr_ : {3, 5, 7}) {
+    int64_t r = 1;
+    while (odd % (r * pr_) == 0) r *= pr_;
+    if (r == 1) continue;
+    const int64_t rest = L / r;
+    const int64_t u = (t % r) * inv_mod(rest % r, r) % r;
+    s = gf::mulq(s, gf::powq(gf::root_odd((uint64_t)r), (uint64_t)u));
+  }
+  return {gf::mulq(w.re, s), gf::mulq(w.im, s)};
+}
+}  // namespace
+
+bool gf_supported(int M) {
+  if (M < 2) return false;
+  int odd = M;
+  while (!(odd & 1)) odd >>= 1;
+  return 1575 % odd == 0;  // 3^2 5^2 7
+}
+
+void gf_root(int64_t t, int64_t L, uint64_t* c, uint64_t* d) {
+  const Gf w = groot(t, L);
+  *c = w.re;
+  *d = w.im;
+}
+
+HostTw gf_pack(uint64_t c, uint64_t d) {
+  const gf::Limbs a = gf::limbs(c), b = gf::limbs(d);
+  return {a.c0, a.c1, b.c0, b.c1};
+}
+
+void gf_stage_twiddles(int L, const int* radices, int nst, bool inverse, std::vector<HostTw>& tw, int* off) {
+  tw.assign(1, HostTw{1, 0, 0, 0});
+  int Ns = 1;
+  for (int s = 0; s < nst; ++s) {
+    const int R = radices[s];
+    off[s] = (int)tw.size();
+    if (Ns > 1) {
+      const size_t start = tw.size();
+      tw.resize(start + (size_t)(R - 1) * Ns);
+      const Gf base = groot(inverse ? -1 : 1, (int64_t)Ns * R);
+      Gf w{1, 0};
+      for (int k = 0; k < Ns; ++k, w = gmul(w, base)) {
+        Gf v = w;
+        for (int q = 1; q < R; ++q, v = gmul(v, w)) tw[start + (size_t)(q - 1) * Ns + k] = gf_pack(v.re, v.im);
+      }
+    }
+    Ns *= R;
+  }
+  (void)L;
+}
+
+void gf_pass_tables(int W, int H, std::vector<HostTw>& k1, std::vector<HostTw>& pair, std::vector<HostTw>& k2t) {
+  const int64_t M = (int64_t)W * H;
+  k1.resize((size_t)M);
+  pair.resize((size_t)M);
+  k2t.resize((size_t)M);
+  const uint64_t minv = gf::powq((uint64_t)M, gf::kQ - 2);
+  const uint64_t quarter = gf::kQ - (1ull << 59);  // -1/4
+  parallel_for(M, [&](int64_t b, int64_t e) {
+    Gf base{1, 0}, cur{1, 0};
+    for (int64_t i = b; i < e; ++i) {
+      const int64_t m1 = i / H, j = i - m1 * H;
+      if (i == b || j == 0) {
+        base = groot(m1, M);
+        cur = groot(m1 * j, M);
+      }
+      k1[(size_t)i] = gf_pack(cur.re, cur.im);
+      cur = gmul(cur, base);
+    }
+    for (int64_t i = b; i < e; ++i) {
+      const int64_t r = i / W, j = i - r * W;
+      if (i == b || j == 0) {
+        base = groot(-r, M);
+        cur = groot(-r * j, M);
+        cur = {gf::mulq(cur.re, minv), gf::mulq(cur.im, minv)};
+      }
+      k2t[(size_t)i] = gf_pack(cur.re, cur.im);
+      cur = gmul(cur, base);
+    }
+    base = groot(1, W);
+    for (int64_t i = b; i < e; ++i) {
+      const int64_t r = i / W, j = i - r * W;
+      if (i == b || j == 0) cur = groot(r + (int64_t)H * j, M);
+      pair[(size_t)i] = gf_pack(gf::mulq(addq(cur.re, 1), quarter), gf::mulq(cur.im, quarter));
+      cur = gmul(cur, base);
+    }
+  });
+}
+
+void gf_row_pairs(int W, int H, std::vector<RowPair>& rows) {
+  const int64_t M = (int64_t)W * H;
+  const int64_t qM = (int64_t)(gf::kQ % (uint64_t)M);
+  rows.clear();
+  for (int64_t k2 = 0; k2 < H; ++k2) {
+    const int64_t b = qM * k2 % H;
+    if (b < k2) continue;
+    rows.push_back({(int32_t)k2, (int32_t)b, (int32_t)((qM * k2 - b) / H % W), 0});
+  }
+}
+
+void gf_weights(int p, int N, std::vector<uint8_t>& e) {
+  e.resize((size_t)N);
+  const int64_t ninv = inv_mod(N % 61, 61);
+  for (int j = 0; j < N; ++j) {
+    const int64_t r = ceil_div_pos((int64_t)p * j, N) * N - (int64_t)p * j;
+    e[(size_t)j] = (uint8_t)(r % 61 * ninv % 61);
+  }
 }
 
 }  // namespace gl

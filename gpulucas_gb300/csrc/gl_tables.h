@@ -60,6 +60,34 @@ int stage_values(int R);
 // real-signal square V_k = U_k^2 + c_k (U_k - conj(U_{M-k}))^2.
 HostCplx pair_coeff(int64_t k, int64_t M);
 
+// ---- tables of the integer form (gl_gf61.cuh): everything is exact in GF(q^2), q = 2^61 - 1
+
+// a table entry (c, d) for c + i d, each as two limbs c0 + c1 2^31
+struct HostTw {
+  int32_t c0, c1, d0, d1;
+};
+// whether GF(q^2) has the roots of unity that M complex points need (odd part of M
+// dividing 3^2 5^2 7; N = 2 M is then prime to 61, so the weights are powers of two)
+bool gf_supported(int M);
+// exp(-2 pi i t / L)'s counterpart: a multiplicative family of roots of unity (root(t, L)
+// root(u, L) = root(t + u, L), root(t k, L k) = root(t, L)), as c + i d with 0 <= c, d < q
+void gf_root(int64_t t, int64_t L, uint64_t* c, uint64_t* d);
+HostTw gf_pack(uint64_t c, uint64_t d);
+// Values of one Stockham line DFT of length L: for every stage after the first, span Ns
+// and radix R, w^q (q = 1..R-1) of w = root(+-k, Ns R) at off[s] + (q-1) Ns + k.
+void gf_stage_twiddles(int L, const int* radices, int nst, bool inverse, std::vector<HostTw>& tw, int* off);
+// k1[m1 H + k2] = root(m1 k2, M); k2t[k2 W + m1] = root(-m1 k2, M) / M;
+// pair[k2 W + k1] = -(1 + root(k2 + H k1, M)) / 4, M = W H
+void gf_pass_tables(int W, int H, std::vector<HostTw>& k1, std::vector<HostTw>& pair, std::vector<HostTw>& k2t);
+// The row pairs of the row pass.  Frequency k = k2 + H k1 pairs with q k mod M, so row k2
+// pairs with row q k2 mod H, and in it position k1 with q k1 + shift mod W.
+struct RowPair {
+  int32_t a, b, shift, pad;  // rows a <= b (a == b: a row paired with itself)
+};
+void gf_row_pairs(int W, int H, std::vector<RowPair>& rows);
+// weight exponent of word j: A[j] = 2^(r/N) = 2^e with r = ceil(jp/N) N - jp, e = r N^-1 mod 61
+void gf_weights(int p, int N, std::vector<uint8_t>& e);
+
 // factor n into the allowed radices (16, 8, 4, 2, 3, 5, 7; powers of two up to
 // max_radix), largest power of two first, then 3, 5, 7; empty if n has another prime
 // factor.

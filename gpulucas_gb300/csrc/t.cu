@@ -1,0 +1,360 @@
+// gl_int_kernels.cu -- one Lucas-Lehmer iteration in exact integer arithmetic.
+//
+// The same three passes as the fused FP64 form (gl_kernels.cu), over GF(q^2), q = 2^61 - 1
+// (gl_gf61.cuh), instead of the complex numbers: weights are rotations by e bits, twiddles
+// are field elements, and the inverse transform gives every product exactly (they are
+// below 2^60 in magnitude), so nothing is rounded.  The layout (H x W, column-major
+// per-word arrays), the dicing and the range checks are those of the FP64 form, and so are
+// the products, bit for bit.  GB300's FP64 units bound the FP64 form; this one is bound by
+// the integer pipes (a 32 x 32 -> 64-bit multiply-add holds one for 4 cycles per warp,
+// other integer instructions 1 to 2).
+//
+// Two differences from the complex numbers:
+//  * the row and position that a frequency pairs with (the real-signal split): conjugation
+//    sends frequency k to q k mod M, which is -k only in the power-of-two part, so the row
+//    pairs come from a table and the position in the partner row is q k1 + shift mod W;
+//  * roots of odd order are scalars of GF(q), not of norm 1, so the inverse transform has
+//    its own tables.
+#include "gl_dice.cuh"
+#include "gl_gf61.cuh"
+#include "gl_internal.h"
+
+namespace gl {
+namespace {
+
+using gf::g2;
+
+__device__ __forceinline__ int ipad(int i) { return i + (i >> 3); }
+
+__device__ __forceinline__ g2 ldz(const DevCplx* p) {
+  const longlong2 v = *reinterpret_cast<const longlong2*>(p);
+  return g2{v.x, v.y};
+}
+__device__ __forceinline__ void stz(DevCplx* p, g2 v) {
+  *reinterpret_cast<longlong2*>(p) = make_longlong2(v.re, v.im);
+}
+
+// Stockham DIT stage, out of place, as in the FP64 form: butterfly j of a line reads
+// x[j + q L/R], multiplies by w^q and writes x[(j - k) R + k + p Ns], k = j mod Ns.
+// The position k needs no division in the first stages (Ns a power of two) or the last
+// (Ns = L/R > j).
+template <int R, int S>
+__device__ __forceinline__ void int_stage(const g2* __restrict__ src, g2* __restrict__ dst, int nlines, int ls,
+                                          int L, int Ns, const int4* __restrict__ tw) {
+  const int LR = L / R;
+  const int nb = nlines * LR;
+  const bool last = Ns == LR, pow2 = (Ns & (Ns - 1)) == 0;
+#pragma unroll 1
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+    int l = 0;
+    if (nlines == 2) l = b >= LR;
+    else if (nlines > 2) l = b / LR;
+    const int j = b - l * LR;
+    const int k = last ? j : pow2 ? (j & (Ns - 1)) : j % Ns;
+    const g2* s = src + l * ls;
+    g2 v[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = s[ipad(j + q * LR)];
+    gf::butterfly<R, S>(v, Ns > 1, [&](int i) { return __ldg(tw + (k + i * Ns)); });
+    g2* d = dst + l * ls;
+    const int base = (j - k) * R + k;
+#pragma unroll
+    for (int q = 0; q < R; ++q) d[ipad(base + q * Ns)] = v[q];
+  }
+  __syncthreads();
+}
+
+// B57: the plan may have radices 5 and 7 (compiled apart: a kernel's registers are set by
+// its largest stage, and without them three CTAs of 256 threads fit an SM).
+template <int S, bool B57>
+__device__ __forceinline__ g2* int_line_fft(g2* a, g2* b, int nlines, int ls, const LinePlan& lp, const int4* tw) {
+  int Ns = 1;
+  for (int s = 0; s < lp.nst; ++s) {
+    const int4* st = tw + lp.off[s];
+    switch (lp.radix[s]) {
+      case 8: int_stage<8, S>(a, b, nlines, ls, lp.L, Ns, st); break;
+      case 4: int_stage<4, S>(a, b, nlines, ls, lp.L, Ns, st); break;
+      case 2: int_stage<2, S>(a, b, nlines, ls, lp.L, Ns, st); break;
+      case 3: int_stage<3, S>(a, b, nlines, ls, lp.L, Ns, st); break;
+      default:
+        if constexpr (B57) {
+          if (lp.radix[s] == 5) int_stage<5, S>(a, b, nlines, ls, lp.L, Ns, st);
+          else int_stage<7, S>(a, b, nlines, ls, lp.L, Ns, st);
+        }
+        break;
+    }
+    Ns *= lp.radix[s];
+    g2* t = a;
+    a = b;
+    b = t;
+  }
+  return a;
+}
+
+// Forward column pass: dice, add carries, weight, length-H DFT, twiddle, store to row k2 of Z.
+template <bool FROM_STATE, int NC, bool B57>
+__device__ __forceinline__ void int_col_fwd_body(const IterArgs& a, const int m1) {
+  extern __shared__ g2 ism[];
+  const int H = a.H, W = a.W, ls = a.in.ls_col;
+  bool wide = false;
+#pragma unroll 1
+  for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) {
+    int v0, v1;
+    load_point<FROM_STATE, NC>(a, m1, m2, &v0, &v1);
+    if (FROM_STATE) wide |= v0 > a.in.vmax || v0 < -a.in.vmax || v1 > a.in.vmax || v1 < -a.in.vmax;
+    const uchar2 e = __ldg(reinterpret_cast<const uchar2*>(a.in.e + 2 * (m1 * H + m2)));
+    ism[ipad(m2)] = g2{gf::weighted(v0, e.x), gf::weighted(v1, e.y)};
+  }
+  if (FROM_STATE && wide) atomicOr(&a.status->flags, kStatusWide);
+  __syncthreads();
+  const g2* res = int_line_fft<-1, B57>(ism, ism + ls, 1, ls, a.in.ph, a.in.hf);
+  const int4* tw = a.in.k1 + (size_t)m1 * H;
+#pragma unroll 2
+  for (int k2 = threadIdx.x; k2 < H; k2 += blockDim.x)
+    stz(a.Z + (size_t)k2 * W + m1, gf::cmul(res[ipad(k2)], __ldg(tw + k2)));
+}
+
+template <bool FROM_STATE, int NC, bool B57>
+__global__ void __launch_bounds__(kMaxThreads, B57 ? 2 : 3) ki_col_fwd(IterArgs a) {
+  int_col_fwd_body<FROM_STATE, NC, B57>(a, blockIdx.x);
+}
+
+// Row pass over the row pairs first .. first + k - 1: pair i's rows are the lines 2i and
+// 2i + 1 (a row paired with itself has one; with several pairs its second line is zero).
+template <bool ONE, bool B57>
+__device__ __forceinline__ void int_row_body(const IterArgs& a, const int first, const int k) {
+  extern __shared__ g2 ism[];
+  const int W = a.W, H = a.H, ls = a.in.ls_row;
+  const int4 r0 = __ldg(a.in.rows + first);
+  const int nl = ONE ? (r0.x == r0.y ? 1 : 2) : 2 * k;
+  g2* other = ism + (ONE ? 2 : 2 * k) * ls;
+#pragma unroll 2
+  for (int idx = threadIdx.x; idx < nl * W; idx += blockDim.x) {
+    const int l = ONE ? idx >= W : idx / W;
+    const int k1 = idx - l * W;
+    const int4 r = ONE ? r0 : __ldg(a.in.rows + first + (l >> 1));
+    const bool mirror = l & 1;
+    ism[l * ls + ipad(k1)] = !ONE && mirror && r.x == r.y ? g2{0, 0} : ldz(a.Z + (size_t)(mirror ? r.y : r.x) * W + k1);
+  }
+  __syncthreads();
+  g2* sp = int_line_fft<-1, B57>(ism, other, nl, ls, a.in.pw, a.in.wf);
+  g2* nx = sp == ism ? other : ism;
+  if (ONE) {
+    const bool self = r0.x == r0.y;
+    g2* lb = self ? sp : sp + ls;
+    const int4* tp = a.in.pair + (size_t)r0.x * W;
+    // partner position q t + shift mod W, stepped along with t
+    const unsigned qW = (unsigned)a.in.qW, uW = (unsigned)W;
+    int u = (int)((qW * threadIdx.x + (unsigned)r0.z) % uW);
+    const int du = (int)(qW * (blockDim.x % uW) % uW);
+#pragma unroll 1
+    for (int t = threadIdx.x; t < W; t += blockDim.x) {
+      if (!self || t <= u) {
+        g2 vk, vkp;
+        gf::pair_square(sp[ipad(t)], lb[ipad(u)], __ldg(tp + t), &vk, &vkp);
+        sp[ipad(t)] = vk;
+        if (!self || t != u) lb[ipad(u)] = vkp;
+      }
+      u += du;
+      u -= u >= W ? W : 0;
+    }
+  } else {
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < k * W; idx += blockDim.x) {
+      const int i = idx / W;
+      const int t = idx - i * W;
+      const int4 r = __ldg(a.in.rows + first + i);
+      const bool self = r.x == r.y;
+      g2* la = sp + 2 * i * ls;
+      g2* lb = self ? la : la + ls;
+      const int u = (int)(((unsigned)a.in.qW * (unsigned)t + (unsigned)r.z) % (unsigned)W);
+      if (self && u < t) continue;
+      g2 vk, vkp;
+      gf::pair_square(la[ipad(t)], lb[ipad(u)], __ldg(a.in.pair + (size_t)r.x * W + t), &vk, &vkp);
+      la[ipad(t)] = vk;
+      if (!self || t != u) lb[ipad(u)] = vkp;
+    }
+  }
+  __syncthreads();
+  const g2* res = int_line_fft<+1, B57>(sp, nx, nl, ls, a.in.pw, a.in.wi);
+#pragma unroll 2
+  for (int idx = threadIdx.x; idx < nl * W; idx += blockDim.x) {
+    const int l = ONE ? idx >= W : idx / W;
+    const int m1 = idx - l * W;
+    const int4 r = ONE ? r0 : __ldg(a.in.rows + first + (l >> 1));
+    const bool mirror = l & 1;
+    if (!ONE && mirror && r.x == r.y) continue;
+    const int row = mirror ? r.y : r.x;
+    stz(a.Z2 + (size_t)m1 * H + row, gf::cmul(res[l * ls + ipad(m1)], __ldg(a.in.k2 + (size_t)row * W + m1)));
+  }
+}
+
+template <bool B57>
+__global__ void __launch_bounds__(kRowThreads, B57 ? 2 : 3) ki_row_sq(IterArgs a) {
+  int_row_body<true, B57>(a, blockIdx.x, 1);
+}
+
+// the product's range checks, as round_word of the FP64 form
+__device__ __forceinline__ long long check_word(long long r, int span, unsigned* fl) {
+  const unsigned long long mag = (unsigned long long)(r < 0 ? -r : r);
+  if (mag >> 51) {
+    *fl |= kStatusBig;
+    return 0;
+  }
+  if (span < 63 && (mag >> span) != 0ull) *fl |= kStatusSlice;
+  return r;
+}
+
+// Inverse column pass: inverse length-H DFT, unweight, -2 at word 0, range checks, products.
+template <bool B57>
+__device__ __forceinline__ void int_col_inv_body(const IterArgs& a, const int m1) {
+  extern __shared__ g2 ism[];
+  const int H = a.H, ls = a.in.ls_col;
+#pragma unroll 2
+  for (int k2 = threadIdx.x; k2 < H; k2 += blockDim.x) ism[ipad(k2)] = ldz(a.Z2 + (size_t)m1 * H + k2);
+  __syncthreads();
+  const g2* res = int_line_fft<+1, B57>(ism, ism + ls, 1, ls, a.in.ph, a.in.hi);
+  unsigned fl = 0;
+#pragma unroll 1
+  for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) {
+    const int s0 = 2 * (m1 * H + m2);
+    const g2 v = res[ipad(m2)];
+    const uchar2 e = __ldg(reinterpret_cast<const uchar2*>(a.in.e + s0));
+    const uchar2 sp = __ldg(reinterpret_cast<const uchar2*>(a.span + s0));
+    long long r0 = check_word(gf::unweighted(v.re, e.x), sp.x, &fl);
+    const long long r1 = check_word(gf::unweighted(v.im, e.y), sp.y, &fl);
+    if (s0 == 0) r0 -= 2;  // word 0: the -2 of the LL step
+    *reinterpret_cast<longlong2*>(a.ll + s0) = make_longlong2(r0, r1);
+  }
+  fl = __reduce_or_sync(0xffffffffu, fl);
+  if ((threadIdx.x & 31) == 0 && fl) atomicOr(&a.status->flags, fl);
+}
+
+template <bool B57>
+__global__ void __launch_bounds__(kMaxThreads, B57 ? 2 : 3) ki_col_inv(IterArgs a) {
+  int_col_inv_body<B57>(a, blockIdx.x);
+}
+
+// ---------------------------------------------------------------------------
+// Batched: units[blockIdx.x] = (test, local unit), as in the FP64 form
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void load_desc(const IterArgs* __restrict__ tests, int t, IterArgs& sa) {
+  const int* src = reinterpret_cast<const int*>(tests + t);
+  int* dst = reinterpret_cast<int*>(&sa);
+  for (int i = threadIdx.x; i < (int)(sizeof(IterArgs) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kMaxThreads, 2) kbi_col_fwd(const IterArgs* __restrict__ tests,
+                                                              const int2* __restrict__ units) {
+  __shared__ IterArgs sa;
+  const int2 u = units[blockIdx.x];
+  load_desc(tests, u.x, sa);
+  switch (sa.n) {
+    case 2: int_col_fwd_body<false, 2, true>(sa, u.y); break;
+    case 3: int_col_fwd_body<false, 3, true>(sa, u.y); break;
+    case 4: int_col_fwd_body<false, 4, true>(sa, u.y); break;
+    case 5: int_col_fwd_body<false, 5, true>(sa, u.y); break;
+    default: int_col_fwd_body<false, 6, true>(sa, u.y); break;
+  }
+}
+
+__global__ void __launch_bounds__(kRowThreads, 2) kbi_row_sq(const IterArgs* __restrict__ tests,
+                                                             const int2* __restrict__ units) {
+  __shared__ IterArgs sa;
+  const int2 u = units[blockIdx.x];
+  load_desc(tests, u.x, sa);
+  const int first = u.y & ((1 << 20) - 1), k = u.y >> 20;
+  if (k == 1) int_row_body<true, true>(sa, first, 1);
+  else int_row_body<false, true>(sa, first, k);
+}
+
+__global__ void __launch_bounds__(kMaxThreads, 2) kbi_col_inv(const IterArgs* __restrict__ tests,
+                                                              const int2* __restrict__ units) {
+  __shared__ IterArgs sa;
+  const int2 u = units[blockIdx.x];
+  load_desc(tests, u.x, sa);
+  int_col_inv_body<true>(sa, u.y);
+}
+
+bool has57(const LinePlan& lp) {
+  for (int i = 0; i < lp.nst; ++i)
+    if (lp.radix[i] == 5 || lp.radix[i] == 7) return true;
+  return false;
+}
+
+template <bool FS, bool B57>
+void launch_col_fwd(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
+  switch (a.n) {
+    case 2: ki_col_fwd<FS, 2, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+    case 3: ki_col_fwd<FS, 3, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+    case 4: ki_col_fwd<FS, 4, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+    case 5: ki_col_fwd<FS, 5, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+    default: ki_col_fwd<FS, 6, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+  }
+}
+void launch_pass(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which, bool from_state) {
+  const bool c57 = has57(g.ph), r57 = has57(g.pw);
+  if (which == 0) {
+    if (from_state) c57 ? launch_col_fwd<true, true>(a, g, s) : launch_col_fwd<true, false>(a, g, s);
+    else c57 ? launch_col_fwd<false, true>(a, g, s) : launch_col_fwd<false, false>(a, g, s);
+  } else if (which == 1) {
+    if (r57) ki_row_sq<true><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
+    else ki_row_sq<false><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
+  } else {
+    if (c57) ki_col_inv<true><<<a.W, g.t_col, g.sm_col, s>>>(a);
+    else ki_col_inv<false><<<a.W, g.t_col, g.sm_col, s>>>(a);
+  }
+}
+
+template <typename K>
+cudaError_t raise(K* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxIntSmem);
+}
+
+template <bool FS, bool B57>
+cudaError_t raise_col_fwd() {
+  cudaError_t e;
+  if ((e = raise(ki_col_fwd<FS, 2, B57>))) return e;
+  if ((e = raise(ki_col_fwd<FS, 3, B57>))) return e;
+  if ((e = raise(ki_col_fwd<FS, 4, B57>))) return e;
+  if ((e = raise(ki_col_fwd<FS, 5, B57>))) return e;
+  return raise(ki_col_fwd<FS, 6, B57>);
+}
+
+}  // namespace
+
+// per kernel and process-wide, raised to the layout chooser's bound
+cudaError_t set_int_smem_limits() {
+  cudaError_t e;
+  if ((e = raise_col_fwd<false, false>())) return e;
+  if ((e = raise_col_fwd<false, true>())) return e;
+  if ((e = raise_col_fwd<true, false>())) return e;
+  if ((e = raise_col_fwd<true, true>())) return e;
+  if ((e = raise(ki_row_sq<false>))) return e;
+  if ((e = raise(ki_row_sq<true>))) return e;
+  if ((e = raise(ki_col_inv<false>))) return e;
+  if ((e = raise(ki_col_inv<true>))) return e;
+  if ((e = raise(kbi_col_fwd))) return e;
+  if ((e = raise(kbi_row_sq))) return e;
+  return raise(kbi_col_inv);
+}
+
+cudaError_t launch_int_kernel(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which) {
+  launch_pass(a, g, s, which, false);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_int_iteration(const IterArgs& a, const IntGeom& g, cudaStream_t s, bool from_state) {
+  for (int w = 0; w < 3; ++w) launch_pass(a, g, s, w, from_state);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_int_batch_iteration(const BatchLaunch& b, cudaStream_t s) {
+  kbi_col_fwd<<<b.ncol, b.t_col, b.sm_col, s>>>(b.tests, b.col_units);
+  kbi_row_sq<<<b.nrow, b.t_row, b.sm_row, s>>>(b.tests, b.row_units);
+  kbi_col_inv<<<b.ncol, b.t_col, b.sm_col, s>>>(b.tests, b.col_units);
+  return cudaGetLastError();
+}
+
+}  // namespace gl

@@ -1,0 +1,144 @@
+"""The integer form (GF(q^2), q = 2^61 - 1) against Python integers on the CPU and against the
+FP64 form and the oracle on the GPU.  Everything is exact, so every comparison is equality."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from gpulucas_gb300 import _build
+
+Q = (1 << 61) - 1
+R = (1 << 60) + (1 << 35)
+
+
+@pytest.fixture(scope="module")
+def hc():
+    L = ctypes.CDLL(_build.HOSTCHECK)
+    i64 = np.ctypeslib.ndpointer(np.int64, flags="C_CONTIGUOUS")
+    L.hc_gf_square.argtypes = [ctypes.c_int] * 3 + [np.ctypeslib.ndpointer(np.int32, flags="C_CONTIGUOUS"), i64,
+                                                    ctypes.POINTER(ctypes.c_longlong)]
+    L.hc_gf_cmul.argtypes = [i64, np.ctypeslib.ndpointer(np.uint64, flags="C_CONTIGUOUS"), i64]
+    for f, a in (("hc_gf_red", [ctypes.c_longlong]), ("hc_gf_weighted", [ctypes.c_int, ctypes.c_int]),
+                 ("hc_gf_unweighted", [ctypes.c_longlong, ctypes.c_int])):
+        getattr(L, f).argtypes = a
+        getattr(L, f).restype = ctypes.c_longlong
+    return L
+
+
+def test_field_operations_at_their_bounds(hc):
+    rng = np.random.default_rng(61)
+    edge = [(1 << 62) - 1, -(1 << 62), 0, 1, -1, Q, -Q, 1 << 61, -(1 << 61), (1 << 31) - 1, -(1 << 31)]
+    res = [0, 1, Q - 1, Q >> 1, (Q >> 1) + 1, 1 << 60, (1 << 60) - 1, (1 << 31) - 1, 1 << 30, Q - (1 << 30)]
+    for _ in range(20000):
+        x = [int(v) for v in rng.integers(-(1 << 62), 1 << 62, 2)]
+        w = [int(v) for v in rng.integers(0, Q, 2)]
+        for k in range(2):
+            if rng.random() < 0.3:
+                x[k] = edge[rng.integers(len(edge))]
+            if rng.random() < 0.3:
+                w[k] = res[rng.integers(len(res))]
+        out = np.zeros(2, np.int64)
+        hc.hc_gf_cmul(np.array(x, np.int64), np.array(w, np.uint64), out)
+        re, im = int(out[0]), int(out[1])
+        assert (re - (x[0] * w[0] - x[1] * w[1])) % Q == 0 and (im - (x[0] * w[1] + x[1] * w[0])) % Q == 0
+        assert abs(re) <= R and abs(im) <= R
+        y = int(rng.integers(-(1 << 63) + (1 << 60) + 1, (1 << 63) - (1 << 60) - 1))
+        r = hc.hc_gf_red(y)
+        assert (r - y) % Q == 0 and -(1 << 60) <= r <= (1 << 60) + 3
+        e = int(rng.integers(61))
+        v = int(rng.integers(-(1 << 28), 1 << 28))
+        g = hc.hc_gf_weighted(v, e)
+        assert (g - v * pow(2, e, Q)) % Q == 0 and abs(g) <= R
+        u = hc.hc_gf_unweighted(x[0] - x[0] // 4, e)  # within 3 R
+        assert (u * pow(2, e, Q) - (x[0] - x[0] // 4)) % Q == 0 and -(1 << 60) < u <= 1 << 60
+
+
+# layouts with every radix first and later, columns or rows with an odd part (rows that pair
+# with themselves in number), an odd number of points, and the smallest width
+@pytest.mark.parametrize("W,H", [(4, 4), (9, 8), (8, 64), (18, 16), (20, 10), (21, 8), (25, 6), (72, 5), (7, 32),
+                                 (36, 35), (15, 15), (63, 25), (128, 8), (5, 2)])
+def test_square_of_weighted_words(hc, W, H):
+    """out[k] = sum over i + j = k mod N of v_i v_j 2^(b_i + b_j - b_k (- p past the end)),
+    b_j = ceil(jp/N): the products an iteration rounds to, without rounding."""
+    N = 2 * W * H
+    p = 17 * N + 5
+    rng = np.random.default_rng(N)
+    for amp in (1 << 17, 1):
+        v = rng.integers(-amp, amp + 1, N).astype(np.int32)
+        if amp > 1:
+            v[:] = np.where(rng.random(N) < 0.5, amp, -amp)  # the largest words a state holds
+        b = [-((-p * j) // N) for j in range(N + 1)]
+        out = np.zeros(N, np.int64)
+        peak = ctypes.c_longlong()
+        assert hc.hc_gf_square(p, W, H, v, out, ctypes.byref(peak)) == 0
+        assert peak.value <= 3 * R
+        i = np.arange(N)
+        for k in range(0, N, max(1, N // 61)):
+            j = (k - i) % N
+            s = sum(int(v[x]) * int(v[y]) << (b[x] + b[y] - b[k] - (p if x + y >= N else 0)) for x, y in zip(i, j))
+            assert s == out[k]
+
+
+def test_lengths_the_field_has_no_roots_for(hc):
+    out, peak = np.zeros(54, np.int64), ctypes.c_longlong()
+    assert hc.hc_gf_square(1000, 27, 1, np.zeros(54, np.int32), out, ctypes.byref(peak)) == -1
+
+
+def _products(gl, p, N, k, **opts):
+    with gl.Plan(p, N, **opts) as pl:
+        rep = pl.iterate(k)
+        return pl.products(), rep, (pl.info.fft_h, pl.info.fft_w)
+
+
+# short and long lines, odd parts 1, 3, 5, 7, 9, 15, 25, 63 and carry depths 2..4; a limit
+# below the default keeps a plan in FP64
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,N", [(100003, 5120), (100003, 6272), (90007, 5600), (1000003, 53760), (859433, 49152),
+                                 (859433, 50400), (2976221, 163840), (2976221, 201600), (1398269, 86016)])
+def test_int_form_products_equal_fp64_form(gl, p, N):
+    for k in (1, 2, 70):
+        a, ra, _ = _products(gl, p, N, k)
+        b, rb, _ = _products(gl, p, N, k, error_limit=0.39)
+        assert ra.status == rb.status == 0
+        assert (a == b).all(), k
+    assert 0.0 < ra.max_roundoff <= rb.max_roundoff
+
+
+@pytest.mark.gpu
+def test_int_form_follows_the_oracle_and_a_loaded_state(gl, orc):
+    p, N = 100003, 5120
+    o = orc.IBDWT(p, N).iterate(37)
+    d, h = o.state()
+    with gl.Plan(p, N) as pl:
+        pl.set_carry_state(d, h, 37)
+        pl.iterate(100)
+        assert (pl.products() == o.iterate(100).ll()).all()
+        assert pl.res64() == orc.Exact(p).iterate(137).res64()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("big", [0, 3000000, -(1 << 24)])
+def test_captured_host_step_with_words_beyond_the_bound(gl, big):
+    """The captured one-iteration step runs in the integer form; a loaded word beyond that
+    form's bound sends the step through FP64, in place and into another buffer, with the
+    same words as the pageable path (FP64) gives."""
+    import torch
+    p, N = 1000003, 53760
+    rng = np.random.default_rng(3)
+    w = rng.integers(-5, 6, N).astype(np.int32) if big else rng.integers(-(1 << 17), 1 << 17, N).astype(np.int32)
+    if big:
+        w[17] = big
+    a = torch.from_numpy(w.copy()).pin_memory()
+    b = torch.empty(N, dtype=torch.int32).pin_memory()
+    ap, bp = ctypes.c_void_p(a.data_ptr()), ctypes.c_void_p(b.data_ptr())
+    rep = gl.IterReport()
+    with gl.Plan(p, N) as pl, gl.Plan(p, N) as ref:
+        want, _ = ref.iterate_host_words(w, 1)
+        assert gl.lib.gl_iterate_host_words(pl._h, ap, 1, bp, ctypes.byref(rep)) == 0
+        assert rep.total_iterations == 1 and (b.numpy() == want).all() and (a.numpy() == w).all()
+        assert gl.lib.gl_iterate_host_words(pl._h, ap, 1, ap, ctypes.byref(rep)) == 0
+        assert rep.total_iterations == 2 and (a.numpy() == want).all()
+        for _ in range(70):  # past the FP64 iteration of the schedule
+            want, _ = ref.iterate_host_words(want, 1)
+            assert gl.lib.gl_iterate_host_words(pl._h, ap, 1, ap, ctypes.byref(rep)) == 0
+        assert (a.numpy() == want).all() and (pl.products() == ref.products()).all()
