@@ -336,7 +336,7 @@ int int_stage_offsets(LinePlan* lp) {
 
 // Geometry of the integer form on an H x W layout; false where GF(q^2) lacks the roots or
 // a CTA's lines do not fit its shared memory.
-bool choose_int_geom(int H, int W, IntGeom* g) {
+bool choose_int_geom(int H, int W, IntGeom* g, bool col_p = false) {
   if (!gf_supported(H * W)) return false;
   if (!fill_line_plan(W, &g->pw) || !fill_line_plan(H, &g->ph)) return false;
   int_stage_offsets(&g->pw);
@@ -345,9 +345,15 @@ bool choose_int_geom(int H, int W, IntGeom* g) {
     const int t = round_up32(butterflies);
     return t < 64 ? 64 : (t > kMaxThreads ? kMaxThreads : t);
   };
+  g->col_p = col_p;
   g->t_col = threads((H + 7) / 8);
   g->t_row = row_threads(W, g->pw, threads((2 * W + 7) / 8));
-  g->sm_col = (size_t)2 * int_stride(H) * 16;
+  for (int s = 0; s < g->ph.nst && col_p; ++s) {
+    // radices 8, 4, 2, 3 only, and no more butterflies than the threads hold
+    const int R = g->ph.radix[s];
+    if (R == 5 || R == 7 || H / R > kIntHeld / R * g->t_col) return false;
+  }
+  g->sm_col = (size_t)(col_p ? 1 : 2) * int_stride(H) * 16;
   g->sm_row = (size_t)4 * int_stride(W) * 16;
   return g->sm_col <= (size_t)kMaxIntSmem && g->sm_row <= (size_t)kMaxIntSmem;
 }
@@ -515,10 +521,10 @@ TunedLayout autotune_layout(int M, int n, int sms, cudaStream_t s, double* ms_ou
 }
 
 // Device time of one integer-form iteration on the H x (M / H) layout, or -1.
-double time_int_layout(int M, int H, int n, int iters, cudaStream_t s) {
+double time_int_layout(int M, int H, bool col_p, int n, int iters, cudaStream_t s) {
   IntGeom g{};
   const int W = M / H, N = 2 * M;
-  if (!choose_int_geom(H, W, &g)) return -1.0;
+  if (!choose_int_geom(H, W, &g, col_p)) return -1.0;
   std::vector<RowPair> rows;
   gf_row_pairs(W, H, rows);
   LinePlan pw = g.pw, ph = g.ph;
@@ -565,37 +571,39 @@ double time_int_layout(int M, int H, int n, int iters, cudaStream_t s) {
   return ms;
 }
 
-// Column length of the integer form for M complex points on this device: the candidates of
-// the layout model that it can run are timed and the fastest kept, once per (M, SM count)
-// per process.  0: no layout.
-std::map<std::pair<int, int>, std::pair<int, double>> g_int_tune_cache;
+// Layout of the integer form for M complex points on this device: the candidates of the
+// layout model that it can run are timed, with two line buffers per column and in place,
+// and the fastest kept, once per (M, SM count) per process.  H = 0: no layout.
+struct IntTuned {
+  int H = 0;
+  bool col_p = false;
+  double ms = 1e300;
+};
+std::map<std::pair<int, int>, IntTuned> g_int_tune_cache;
 constexpr int kIntLayoutsTimed = 8;
 
-int autotune_int_layout(int M, int n, int sms, cudaStream_t s, double* ms_out) {
+IntTuned autotune_int_layout(int M, int n, int sms, cudaStream_t s) {
   {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     auto it = g_int_tune_cache.find({M, sms});
-    if (it != g_int_tune_cache.end()) {
-      if (ms_out) *ms_out = it->second.second;
-      return it->second.first;
-    }
+    if (it != g_int_tune_cache.end()) return it->second;
   }
-  int best = 0, timed = 0;
-  double best_ms = 1e300;
+  IntTuned best;
+  int timed = 0;
   for (const auto& c : ranked_layouts(M, sms)) {
     if (timed == kIntLayoutsTimed) break;
-    const double ms = time_int_layout(M, c.second, n, M >= (1 << 18) ? 10 : 40, s);
-    if (ms <= 0.0) continue;
-    ++timed;
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = c.second;
+    bool any = false;
+    for (bool p : {false, true}) {
+      const double ms = time_int_layout(M, c.second, p, n, M >= (1 << 18) ? 10 : 40, s);
+      if (ms <= 0.0) continue;
+      any = true;
+      if (ms < best.ms) best = IntTuned{c.second, p, ms};
     }
+    timed += any;
   }
-  if (!best) return 0;
+  if (!best.H) return best;
   std::lock_guard<std::mutex> lock(g_tune_mutex);
-  g_int_tune_cache[{M, sms}] = {best, best_ms};
-  if (ms_out) *ms_out = best_ms;
+  g_int_tune_cache[{M, sms}] = best;
   return best;
 }
 
@@ -897,12 +905,16 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   // The integer form, unless an option names a variant of the FP64 kernels.
   IntGeom ig{};
   int vmax = 0;
+  bool int_p = false;
   bool int_form = o.mode == GL_MODE_FUSED && !resident && !fp64_only && !sms_override && !names_fp64_variant(o) &&
                   int_range_ok(p, N, &vmax) && int_roundoff_ok(p, N, o.error_limit);
   if (int_form) {
-    const int H = o.autotune && !sms_override ? autotune_int_layout(M, n, sms, 0, nullptr) : first_int_layout(M, sms);
-    if (H) force_h = H;
-    else int_form = false;
+    IntTuned it;
+    if (o.autotune && !sms_override) it = autotune_int_layout(M, n, sms, 0);
+    else it.H = first_int_layout(M, sms);
+    force_h = it.H;
+    int_p = it.col_p;
+    int_form = it.H != 0;
   }
   bool col_ip = false, col_pf = false, col_ws = false;
   int row_var = 0;
@@ -934,7 +946,7 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   if (rc == GL_ERR_SIZE && col_ip && o.col_inplace <= 0)  // the searched layout cannot: two buffers
     rc = choose_fused_geom(M, force_h, sms, &fg, cap_c, cap_r, false);
   if (rc != GL_OK) return rc;
-  int_form = int_form && choose_int_geom(fg.H, fg.W, &ig);
+  int_form = int_form && choose_int_geom(fg.H, fg.W, &ig, int_p);
 
   gl_plan* pl = new (std::nothrow) gl_plan();
   if (!pl) return GL_ERR_NOMEM;

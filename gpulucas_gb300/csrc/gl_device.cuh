@@ -603,4 +603,15 @@ GL_HD void balanced_split(long long sum, int bits, int* digit, int* hi) {
   *hi = (int)h;
 }
 
+// The same for a digit sum of at most 30 bits: sign and magnitude, so that halves round as
+// there (a negative sum of exactly half a word keeps carry 0).
+GL_HD void balanced_split32(int sum, int bits, int* digit, int* hi) {
+  const int half = 1 << (bits - 1);
+  const int t = sum < 0 ? -sum : sum;
+  int h = (t + half) >> bits;
+  if (sum < 0) h = t == half ? 0 : -h;
+  *digit = sum - h * (1 << bits);
+  *hi = h;
+}
+
 }  // namespace gl

@@ -354,9 +354,15 @@ GL_HD g2 square(g2 u) {  // within 3R -> within 2R
 }
 GL_HD void pair_square(g2 u, g2 up, int4 c, g2* vk, g2* vkp) {
   const int64_t dr = red(u.re - up.re), di = red(u.im + up.im);
-  const g2 pc = cmul(g2{vmul(dr + di, red(dr - di)), vmul(2 * dr, di)}, c);
-  const g2 s = square(u), sp = square(up);
+  g2 pc = cmul(g2{vmul(dr + di, red(dr - di)), vmul(2 * dr, di)}, c);
+#ifdef __CUDA_ARCH__
+  // the squares after the product: computing them side by side takes more registers than
+  // four or five resident CTAs leave
+  asm("" : "+l"(u.re), "+l"(u.im), "+l"(up.re), "+l"(up.im), "+l"(pc.re), "+l"(pc.im));
+#endif
+  const g2 s = square(u);
   *vk = red(add(s, pc));
+  const g2 sp = square(up);
   *vkp = red(g2{sp.re + pc.re, sp.im - pc.im});
 }
 

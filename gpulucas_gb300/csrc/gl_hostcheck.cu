@@ -55,6 +55,7 @@ long long hc_dice_sum(int LO, int n, unsigned f, const long long* ll, int N, int
 }
 
 void hc_balanced_split(long long sum, int bits, int* digit, int* hi) { balanced_split(sum, bits, digit, hi); }
+void hc_balanced_split32(int sum, int bits, int* digit, int* hi) { balanced_split32(sum, bits, digit, hi); }
 
 }  // extern "C"
 

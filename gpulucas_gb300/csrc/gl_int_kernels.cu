@@ -62,6 +62,68 @@ __device__ __forceinline__ void int_stage(const g2* __restrict__ src, g2* __rest
   __syncthreads();
 }
 
+// In-place stage: every thread first reads the inputs of all its butterflies (at most P
+// points) into registers, then, after a barrier, transforms and writes them.  One line
+// buffer and 64 registers, so four CTAs of 256 threads are resident and the 576 columns of
+// N = 2359296 run as one wave: 137.8 -> 132.3 us per iteration there (the integer passes
+// alone) against two buffers and three CTAs.  Holding 16 points in 128 threads
+// (122 registers) took 154.  Short columns are faster with two buffers, one barrier per
+// stage (N = 49152: 20.4 against 21.1); the layout search times both.
+template <int R, int P>
+__host__ __device__ constexpr int ip_count() {
+  return P / R > 0 ? P / R : 1;
+}
+template <int R, int S, int P>
+__device__ __forceinline__ void int_stage_ip(g2* __restrict__ buf, int L, int Ns, const int4* __restrict__ tw) {
+  constexpr int B = ip_count<R, P>();
+  const int LR = L / R;
+  const bool last = Ns == LR, pow2 = (Ns & (Ns - 1)) == 0;
+  g2 held[B][R];
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    const int j = threadIdx.x + i * blockDim.x;
+    const int jj = j < LR ? j : 0;  // a thread without this butterfly reads a valid slot
+#pragma unroll
+    for (int q = 0; q < R; ++q) held[i][q] = buf[ipad(jj + q * LR)];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    const int j = threadIdx.x + i * blockDim.x;
+    if (j < LR) {
+      const int k = last ? j : pow2 ? (j & (Ns - 1)) : j % Ns;
+      g2 v[R];
+      gf::butterfly<R, S>(
+          v, Ns > 1, [&](int q) { return held[i][q]; }, [&](int s) { return __ldg(tw + (k + s * Ns)); });
+      const int base = (j - k) * R + k;
+#pragma unroll
+      for (int q = 0; q < R; ++q) buf[ipad(base + q * Ns)] = v[q];
+    }
+  }
+  __syncthreads();
+}
+
+template <int S, bool B57, int P>
+__device__ __forceinline__ void int_line_fft_ip(g2* a, const LinePlan& lp, const int4* tw) {
+  int Ns = 1;
+  for (int s = 0; s < lp.nst; ++s) {
+    const int4* st = tw + lp.off[s];
+    switch (lp.radix[s]) {
+      case 8: int_stage_ip<8, S, P>(a, lp.L, Ns, st); break;
+      case 4: int_stage_ip<4, S, P>(a, lp.L, Ns, st); break;
+      case 2: int_stage_ip<2, S, P>(a, lp.L, Ns, st); break;
+      case 3: int_stage_ip<3, S, P>(a, lp.L, Ns, st); break;
+      default:
+        if constexpr (B57) {
+          if (lp.radix[s] == 5) int_stage_ip<5, S, P>(a, lp.L, Ns, st);
+          else int_stage_ip<7, S, P>(a, lp.L, Ns, st);
+        }
+        break;
+    }
+    Ns *= lp.radix[s];
+  }
+}
+
 // B57: the plan may have radices 5 and 7 (compiled apart: a kernel's registers are set by
 // its largest stage, and without them three CTAs of 256 threads fit an SM).
 template <int S, bool B57>
@@ -90,11 +152,12 @@ __device__ __forceinline__ g2* int_line_fft(g2* a, g2* b, int nlines, int ls, co
 }
 
 // Forward column pass: dice, add carries, weight, length-H DFT, twiddle, store to row k2 of Z.
-template <bool FROM_STATE, int NC, bool B57>
+template <bool FROM_STATE, int NC, bool B57, int P>
 __device__ __forceinline__ void int_col_fwd_body(const IterArgs& a, const int m1) {
   extern __shared__ g2 ism[];
   const int H = a.H, W = a.W, ls = a.in.ls_col;
   bool wide = false;
+#pragma unroll 1
   for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) {
     int v0, v1;
     load_point<FROM_STATE, NC>(a, m1, m2, &v0, &v1);
@@ -104,15 +167,25 @@ __device__ __forceinline__ void int_col_fwd_body(const IterArgs& a, const int m1
   }
   if (FROM_STATE && wide) atomicOr(&a.status->flags, kStatusWide);
   __syncthreads();
-  const g2* res = int_line_fft<-1, B57>(ism, ism + ls, 1, ls, a.in.ph, a.in.hf);
-  const int4* tw = a.in.k1 + (size_t)m1 * H;
+  const g2* res = ism;
+  if constexpr (P > 0) int_line_fft_ip<-1, B57, P>(ism, a.in.ph, a.in.hf);
+  else res = int_line_fft<-1, B57>(ism, ism + ls, 1, ls, a.in.ph, a.in.hf);
+#pragma unroll 1
   for (int k2 = threadIdx.x; k2 < H; k2 += blockDim.x)
-    stz(a.Z + (size_t)k2 * W + m1, gf::cmul(res[ipad(k2)], __ldg(tw + k2)));
+    stz(a.Z + (k2 * W + m1), gf::cmul(res[ipad(k2)], __ldg(a.in.k1 + (m1 * H + k2))));
 }
 
-template <bool FROM_STATE, int NC, bool B57>
-__global__ void __launch_bounds__(kMaxThreads, B57 ? 2 : 3) ki_col_fwd(IterArgs a) {
-  int_col_fwd_body<FROM_STATE, NC, B57>(a, blockIdx.x);
+template <bool FROM_STATE, int NC, bool B57, int P>
+__global__ void __launch_bounds__(kMaxThreads, B57 ? 2 : P ? 4 : 3) ki_col_fwd(IterArgs a) {
+  int_col_fwd_body<FROM_STATE, NC, B57, P>(a, blockIdx.x);
+}
+
+// Row pair i of the table.  Loaded where it is used (volatile, so the compiler does not keep
+// it in registers through the transforms, which need them all).
+__device__ __forceinline__ int4 row_pair(const int4* rows, int i) {
+  int4 r;
+  asm volatile("ld.global.nc.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(rows + i));
+  return r;
 }
 
 // Row pass over one row pair (a row paired with itself: one line).
@@ -120,21 +193,24 @@ template <bool B57>
 __device__ __forceinline__ void int_row_body(const IterArgs& a, const int pair) {
   extern __shared__ g2 ism[];
   const int W = a.W, H = a.H, ls = a.in.ls_row;
-  const int4 r = __ldg(a.in.rows + pair);
-  const bool self = r.x == r.y;
-  const int nl = self ? 1 : 2;
   g2* other = ism + 2 * ls;
-  for (int idx = threadIdx.x; idx < nl * W; idx += blockDim.x) {
-    const int l = idx >= W;
-    const int k1 = idx - l * W;
-    ism[l * ls + ipad(k1)] = ldz(a.Z + (size_t)(l ? r.y : r.x) * W + k1);
+  int nl;
+  {
+    const int4 r = row_pair(a.in.rows, pair);
+    nl = r.x == r.y ? 1 : 2;
+    for (int idx = threadIdx.x; idx < nl * W; idx += blockDim.x) {
+      const int l = idx >= W;
+      const int k1 = idx - l * W;
+      ism[l * ls + ipad(k1)] = ldz(a.Z + ((l ? r.y : r.x) * W + k1));
+    }
   }
   __syncthreads();
   g2* sp = int_line_fft<-1, B57>(ism, other, nl, ls, a.in.pw, a.in.wf);
   g2* nx = sp == ism ? other : ism;
   {
+    const int4 r = row_pair(a.in.rows, pair);
+    const bool self = r.x == r.y;
     g2* lb = self ? sp : sp + ls;
-    const int4* tp = a.in.pair + (size_t)r.x * W;
     // partner position q t + shift mod W, stepped along with t
     const unsigned qW = (unsigned)a.in.qW, uW = (unsigned)W;
     int u = (int)((qW * threadIdx.x + (unsigned)r.z) % uW);
@@ -143,7 +219,7 @@ __device__ __forceinline__ void int_row_body(const IterArgs& a, const int pair) 
     for (int t = threadIdx.x; t < W; t += blockDim.x) {
       if (!self || t <= u) {
         g2 vk, vkp;
-        gf::pair_square(sp[ipad(t)], lb[ipad(u)], __ldg(tp + t), &vk, &vkp);
+        gf::pair_square(sp[ipad(t)], lb[ipad(u)], __ldg(a.in.pair + (r.x * W + t)), &vk, &vkp);
         sp[ipad(t)] = vk;
         if (!self || t != u) lb[ipad(u)] = vkp;
       }
@@ -153,16 +229,21 @@ __device__ __forceinline__ void int_row_body(const IterArgs& a, const int pair) 
   }
   __syncthreads();
   const g2* res = int_line_fft<+1, B57>(sp, nx, nl, ls, a.in.pw, a.in.wi);
+  const int4 r = row_pair(a.in.rows, pair);
   for (int idx = threadIdx.x; idx < nl * W; idx += blockDim.x) {
     const int l = idx >= W;
     const int m1 = idx - l * W;
     const int row = l ? r.y : r.x;
-    stz(a.Z2 + (size_t)m1 * H + row, gf::cmul(res[l * ls + ipad(m1)], __ldg(a.in.k2 + (size_t)row * W + m1)));
+    stz(a.Z2 + (m1 * H + row), gf::cmul(res[l * ls + ipad(m1)], __ldg(a.in.k2 + (row * W + m1))));
   }
 }
 
-template <bool B57>
-__global__ void __launch_bounds__(kRowThreads, B57 ? 2 : 3) ki_row_sq(IterArgs a) {
+// Two builds for radices 8, 4, 2, 3: five CTAs of 192 threads per SM (64 registers) where the
+// row pairs are enough to fill them, else 80 registers, which shorten the dependent chains
+// of a pass with few CTAs (N = 49152, 49 pairs: 14.1 us against 15.6).
+constexpr int kRowsFor5 = 3 * 152;
+template <bool B57, int T, int MB>
+__global__ void __launch_bounds__(T, MB) ki_row_sq(IterArgs a) {
   int_row_body<B57>(a, blockIdx.x);
 }
 
@@ -178,13 +259,15 @@ __device__ __forceinline__ long long check_word(long long r, int span, unsigned*
 }
 
 // Inverse column pass: inverse length-H DFT, unweight, -2 at word 0, range checks, products.
-template <bool B57>
+template <bool B57, int P>
 __device__ __forceinline__ void int_col_inv_body(const IterArgs& a, const int m1) {
   extern __shared__ g2 ism[];
   const int H = a.H, ls = a.in.ls_col;
   for (int k2 = threadIdx.x; k2 < H; k2 += blockDim.x) ism[ipad(k2)] = ldz(a.Z2 + (size_t)m1 * H + k2);
   __syncthreads();
-  const g2* res = int_line_fft<+1, B57>(ism, ism + ls, 1, ls, a.in.ph, a.in.hi);
+  const g2* res = ism;
+  if constexpr (P > 0) int_line_fft_ip<+1, B57, P>(ism, a.in.ph, a.in.hi);
+  else res = int_line_fft<+1, B57>(ism, ism + ls, 1, ls, a.in.ph, a.in.hi);
   unsigned fl = 0;
   for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) {
     const int s0 = 2 * (m1 * H + m2);
@@ -200,9 +283,9 @@ __device__ __forceinline__ void int_col_inv_body(const IterArgs& a, const int m1
   if ((threadIdx.x & 31) == 0 && fl) atomicOr(&a.status->flags, fl);
 }
 
-template <bool B57>
-__global__ void __launch_bounds__(kMaxThreads, B57 ? 2 : 3) ki_col_inv(IterArgs a) {
-  int_col_inv_body<B57>(a, blockIdx.x);
+template <bool B57, int P>
+__global__ void __launch_bounds__(kMaxThreads, B57 ? 2 : P ? 4 : 3) ki_col_inv(IterArgs a) {
+  int_col_inv_body<B57, P>(a, blockIdx.x);
 }
 
 bool has57(const LinePlan& lp) {
@@ -211,15 +294,25 @@ bool has57(const LinePlan& lp) {
   return false;
 }
 
+template <bool FS, bool B57, int P>
+void launch_col_fwd_p(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
+  switch (a.n) {
+    case 2: ki_col_fwd<FS, 2, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+    case 3: ki_col_fwd<FS, 3, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+    case 4: ki_col_fwd<FS, 4, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+    case 5: ki_col_fwd<FS, 5, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+    default: ki_col_fwd<FS, 6, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
+  }
+}
 template <bool FS, bool B57>
 void launch_col_fwd(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
-  switch (a.n) {
-    case 2: ki_col_fwd<FS, 2, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-    case 3: ki_col_fwd<FS, 3, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-    case 4: ki_col_fwd<FS, 4, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-    case 5: ki_col_fwd<FS, 5, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-    default: ki_col_fwd<FS, 6, B57><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-  }
+  if (!B57 && g.col_p) launch_col_fwd_p<FS, false, kIntHeld>(a, g, s);
+  else launch_col_fwd_p<FS, B57, 0>(a, g, s);
+}
+template <bool B57>
+void launch_col_inv(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
+  if (!B57 && g.col_p) ki_col_inv<false, kIntHeld><<<a.W, g.t_col, g.sm_col, s>>>(a);
+  else ki_col_inv<B57, 0><<<a.W, g.t_col, g.sm_col, s>>>(a);
 }
 void launch_pass(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which, bool from_state) {
   const bool c57 = has57(g.ph), r57 = has57(g.pw);
@@ -227,11 +320,12 @@ void launch_pass(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which,
     if (from_state) c57 ? launch_col_fwd<true, true>(a, g, s) : launch_col_fwd<true, false>(a, g, s);
     else c57 ? launch_col_fwd<false, true>(a, g, s) : launch_col_fwd<false, false>(a, g, s);
   } else if (which == 1) {
-    if (r57) ki_row_sq<true><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
-    else ki_row_sq<false><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
+    if (r57) ki_row_sq<true, 256, 2><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
+    else if (g.t_row <= 192 && a.in.nrows > kRowsFor5) ki_row_sq<false, 192, 5><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
+    else ki_row_sq<false, 256, 3><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
   } else {
-    if (c57) ki_col_inv<true><<<a.W, g.t_col, g.sm_col, s>>>(a);
-    else ki_col_inv<false><<<a.W, g.t_col, g.sm_col, s>>>(a);
+    if (c57) launch_col_inv<true>(a, g, s);
+    else launch_col_inv<false>(a, g, s);
   }
 }
 
@@ -240,14 +334,22 @@ cudaError_t raise(K* kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxIntSmem);
 }
 
-template <bool FS, bool B57>
+template <bool FS, bool B57, int P>
 cudaError_t raise_col_fwd() {
   cudaError_t e;
-  if ((e = raise(ki_col_fwd<FS, 2, B57>))) return e;
-  if ((e = raise(ki_col_fwd<FS, 3, B57>))) return e;
-  if ((e = raise(ki_col_fwd<FS, 4, B57>))) return e;
-  if ((e = raise(ki_col_fwd<FS, 5, B57>))) return e;
-  return raise(ki_col_fwd<FS, 6, B57>);
+  if ((e = raise(ki_col_fwd<FS, 2, B57, P>))) return e;
+  if ((e = raise(ki_col_fwd<FS, 3, B57, P>))) return e;
+  if ((e = raise(ki_col_fwd<FS, 4, B57, P>))) return e;
+  if ((e = raise(ki_col_fwd<FS, 5, B57, P>))) return e;
+  return raise(ki_col_fwd<FS, 6, B57, P>);
+}
+
+template <bool B57, int P>
+cudaError_t raise_col() {
+  cudaError_t e;
+  if ((e = raise_col_fwd<false, B57, P>())) return e;
+  if ((e = raise_col_fwd<true, B57, P>())) return e;
+  return raise(ki_col_inv<B57, P>);
 }
 
 }  // namespace
@@ -255,14 +357,13 @@ cudaError_t raise_col_fwd() {
 // per kernel and process-wide, raised to the layout chooser's bound
 cudaError_t set_int_smem_limits() {
   cudaError_t e;
-  if ((e = raise_col_fwd<false, false>())) return e;
-  if ((e = raise_col_fwd<false, true>())) return e;
-  if ((e = raise_col_fwd<true, false>())) return e;
-  if ((e = raise_col_fwd<true, true>())) return e;
-  if ((e = raise(ki_row_sq<false>))) return e;
-  if ((e = raise(ki_row_sq<true>))) return e;
-  if ((e = raise(ki_col_inv<false>))) return e;
-  return raise(ki_col_inv<true>);
+  if ((e = raise_col<false, 0>())) return e;
+  if ((e = raise_col<true, 0>())) return e;
+  if ((e = raise_col<false, kIntHeld>())) return e;
+  if ((e = raise(ki_row_sq<false, 192, 5>))) return e;
+  if ((e = raise(ki_row_sq<false, 256, 3>))) return e;
+  if ((e = raise(ki_row_sq<true, 256, 2>))) return e;
+  return cudaSuccess;
 }
 
 cudaError_t launch_int_kernel(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which) {

@@ -79,10 +79,12 @@ struct PlainGeom {
 // 16-byte accesses are served eight lanes at a time
 constexpr int int_stride(int L) { return L + (L >> 3) + 1; }
 constexpr int kMaxIntSmem = 120 * 1024;
+constexpr int kIntHeld = 8;
 
 // Geometry of the integer form (gl_int_kernels.cu) on the same H x W array.
 struct IntGeom {
   int t_col, t_row;        // threads per CTA
+  bool col_p;              // column passes transform in place (kIntHeld points per thread)
   size_t sm_col, sm_row;   // dynamic shared memory bytes
   LinePlan pw, ph;         // line plans (offsets into the stage tables)
 };

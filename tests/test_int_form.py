@@ -104,6 +104,16 @@ def test_int_form_products_equal_fp64_form(gl, p, N):
     assert 0.0 < ra.max_roundoff <= rb.max_roundoff
 
 
+# in-place columns (the layout search may pick either form): long power-of-two columns, and
+# rows of more than one butterfly per thread
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,N", [(9300017, 524288), (20996011, 1179648), (24000001, 1310720), (74207281, 4194304)])
+def test_int_form_long_lines_equal_fp64_form(gl, p, N):
+    a, ra, _ = _products(gl, p, N, 67)
+    b, rb, _ = _products(gl, p, N, 67, error_limit=0.39)
+    assert ra.status == rb.status == 0 and (a == b).all()
+
+
 @pytest.mark.gpu
 def test_int_form_follows_the_oracle_and_a_loaded_state(gl, orc):
     p, N = 100003, 5120
@@ -142,3 +152,20 @@ def test_captured_host_step_with_words_beyond_the_bound(gl, big):
             want, _ = ref.iterate_host_words(want, 1)
             assert gl.lib.gl_iterate_host_words(pl._h, ap, 1, ap, ctypes.byref(rep)) == 0
         assert (a.numpy() == want).all() and (pl.products() == ref.products()).all()
+
+
+def test_balanced_split_in_32_bits_equals_64(hc):
+    """The 32-bit split of the dicing against the general one, ties included."""
+    hc.hc_balanced_split.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.POINTER(ctypes.c_int),
+                                     ctypes.POINTER(ctypes.c_int)]
+    hc.hc_balanced_split32.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int),
+                                       ctypes.POINTER(ctypes.c_int)]
+    d, h, d2, h2 = (ctypes.c_int() for _ in range(4))
+    rng = np.random.default_rng(32)
+    for bits in range(14, 24):
+        half = 1 << (bits - 1)
+        sums = [k * half + o for k in range(-9, 10) for o in (-1, 0, 1)] + [int(v) for v in rng.integers(-8 * half, 8 * half, 300)]
+        for s in sums:
+            hc.hc_balanced_split(s, bits, d, h)
+            hc.hc_balanced_split32(s, bits, d2, h2)
+            assert (d.value, h.value) == (d2.value, h2.value), (s, bits)
