@@ -334,11 +334,19 @@ int int_stage_offsets(LinePlan* lp) {
   return size;
 }
 
-// Geometry of the integer form on an H x W layout; false where GF(q^2) lacks the roots or
-// a CTA's lines do not fit its shared memory.
+// Largest polynomial length (gf_excess) the integer form is used at.  Squaring takes about
+// t/2 products per coefficient, but a test alone waits on latencies more than it computes
+// (us per iteration, integer/FP64: N = 44100, t = 7, 25.2/35.5; 52500, 25, 29.4/35.8;
+// 54432, 27, 30.5/31.6; 78400, 49, 27.8/39.5).
+constexpr int kMaxIntPoly = 49;
+
+// Geometry of the integer form on an H x W layout; false where its polynomials do not fit
+// the rows or a CTA's lines its shared memory.
 bool choose_int_geom(int H, int W, IntGeom* g, bool col_p = false) {
-  if (!gf_supported(H * W)) return false;
-  if (!fill_line_plan(W, &g->pw) || !fill_line_plan(H, &g->ph)) return false;
+  g->t = gf_excess(H * W);
+  if (g->t > kMaxIntPoly || W % g->t) return false;
+  const int V = W / g->t;
+  if (!fill_line_plan(V, &g->pw) || !fill_line_plan(H, &g->ph)) return false;
   int_stage_offsets(&g->pw);
   int_stage_offsets(&g->ph);
   auto threads = [](int butterflies) {
@@ -347,14 +355,14 @@ bool choose_int_geom(int H, int W, IntGeom* g, bool col_p = false) {
   };
   g->col_p = col_p;
   g->t_col = threads((H + 7) / 8);
-  g->t_row = row_threads(W, g->pw, threads((2 * W + 7) / 8));
+  g->t_row = g->t > 1 ? threads(W) : row_threads(W, g->pw, threads((2 * W + 7) / 8));
   for (int s = 0; s < g->ph.nst && col_p; ++s) {
     // radices 8, 4, 2, 3 only, and no more butterflies than the threads hold
     const int R = g->ph.radix[s];
     if (R == 5 || R == 7 || H / R > kIntHeld / R * g->t_col) return false;
   }
   g->sm_col = (size_t)(col_p ? 1 : 2) * int_stride(H) * 16;
-  g->sm_row = (size_t)4 * int_stride(W) * 16;
+  g->sm_row = (size_t)int_row_slots(V, g->t) * 16;
   return g->sm_col <= (size_t)kMaxIntSmem && g->sm_row <= (size_t)kMaxIntSmem;
 }
 
@@ -526,7 +534,7 @@ double time_int_layout(int M, int H, bool col_p, int n, int iters, cudaStream_t 
   const int W = M / H, N = 2 * M;
   if (!choose_int_geom(H, W, &g, col_p)) return -1.0;
   std::vector<RowPair> rows;
-  gf_row_pairs(W, H, rows);
+  gf_row_pairs(W / g.t, H, rows);
   LinePlan pw = g.pw, ph = g.ph;
   const size_t szw = (size_t)int_stage_offsets(&pw) * 16, szh = (size_t)int_stage_offsets(&ph) * 16;
   const size_t m16 = 16 * (size_t)M;
@@ -554,8 +562,9 @@ double time_int_layout(int M, int H, bool col_p, int n, int iters, cudaStream_t 
     a.in.hf = (const int4*)buf[11]; a.in.hi = (const int4*)buf[12];
     a.in.rows = (const int4*)buf[13]; a.status = (Status*)buf[14];
     a.in.nrows = (int)rows.size();
-    a.in.qW = (int)(((1ull << 61) - 1) % (uint64_t)W);
-    a.in.ls_col = int_stride(H); a.in.ls_row = int_stride(W); a.in.pw = g.pw; a.in.ph = g.ph;
+    a.in.t = g.t; a.in.V = W / g.t;
+    a.in.qV = (int)(((1ull << 61) - 1) % (uint64_t)a.in.V);
+    a.in.ls_col = int_stride(H); a.in.ls_row = int_stride(a.in.V); a.in.pw = g.pw; a.in.ph = g.ph;
     for (int i = 0; i < 2 && ok; ++i) ok = launch_int_iteration(a, g, s, false) == cudaSuccess;
     ok = ok && cudaEventRecord(e0, s) == cudaSuccess;
     for (int i = 0; i < iters && ok; ++i) ok = launch_int_iteration(a, g, s, false) == cudaSuccess;
@@ -795,22 +804,22 @@ static size_t int_table_bytes(int H, int W, const IntGeom& g) {
   LinePlan pw = g.pw, ph = g.ph;
   const size_t M = (size_t)H * W;
   std::vector<RowPair> rows;
-  gf_row_pairs(W, H, rows);
-  return 3 * M * 16 + 2 * M /* exponents */ + 2 * 16 * ((size_t)int_stage_offsets(&pw) + int_stage_offsets(&ph)) +
+  gf_row_pairs(W / g.t, H, rows);
+  return (2 * M + M / g.t) * 16 + 2 * M /* exponents */ + 2 * 16 * ((size_t)int_stage_offsets(&pw) + int_stage_offsets(&ph)) +
          rows.size() * sizeof(RowPair);
 }
 
 static int build_int_tables(gl_plan* pl, int vmax) {
-  const int W = pl->fg.W, H = pl->fg.H, N = pl->N;
+  const int W = pl->fg.W, H = pl->fg.H, N = pl->N, t = pl->ig.t, V = W / t;
   std::vector<HostTw> k1, pair, k2, wf, wi, hf, hi;
   std::vector<RowPair> rows;
   std::vector<uint8_t> e, e_c((size_t)N);
   int off[8];
-  gf_pass_tables(W, H, k1, pair, k2);
-  gf_row_pairs(W, H, rows);
+  gf_pass_tables(W, H, t, k1, pair, k2);
+  gf_row_pairs(V, H, rows);
   gf_weights(pl->p, N, e);
-  gf_stage_twiddles(W, pl->ig.pw.radix, pl->ig.pw.nst, false, wf, off);
-  gf_stage_twiddles(W, pl->ig.pw.radix, pl->ig.pw.nst, true, wi, off);
+  gf_stage_twiddles(V, pl->ig.pw.radix, pl->ig.pw.nst, false, wf, off);
+  gf_stage_twiddles(V, pl->ig.pw.radix, pl->ig.pw.nst, true, wi, off);
   gf_stage_twiddles(H, pl->ig.ph.radix, pl->ig.ph.nst, false, hf, off);
   gf_stage_twiddles(H, pl->ig.ph.radix, pl->ig.ph.nst, true, hi, off);
   for (int m1 = 0, c = 0; m1 < W; ++m1)  // column-major, as the other per-word tables
@@ -837,10 +846,12 @@ static int build_int_tables(gl_plan* pl, int vmax) {
     return rc;
   GL_CUDA(cudaStreamSynchronize(pl->stream));  // host tables go out of scope
   in.nrows = (int)rows.size();
-  in.qW = (int)(((1ull << 61) - 1) % (uint64_t)W);
+  in.t = t;
+  in.V = V;
+  in.qV = (int)(((1ull << 61) - 1) % (uint64_t)V);
   in.vmax = vmax;
   in.ls_col = int_stride(H);
-  in.ls_row = int_stride(W);
+  in.ls_row = int_stride(V);
   in.pw = pl->ig.pw;
   in.ph = pl->ig.ph;
   GL_CUDA(set_int_smem_limits());

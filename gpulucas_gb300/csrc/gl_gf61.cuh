@@ -294,6 +294,10 @@ GL_HD void dft7_part(int64_t& x0, int64_t& x1, int64_t& x2, int64_t& x3, int64_t
 template <int S>
 GL_HD void dft7(g2* x) {
   dft7_part<S>(x[0].re, x[1].re, x[2].re, x[3].re, x[4].re, x[5].re, x[6].re);
+#ifdef __CUDA_ARCH__
+  // the imaginary parts after the real ones (no instruction; side by side they spill)
+  asm volatile("" : "+l"(x[0].re), "+l"(x[3].re), "+l"(x[1].im), "+l"(x[2].im), "+l"(x[3].im));
+#endif
   dft7_part<S>(x[0].im, x[1].im, x[2].im, x[3].im, x[4].im, x[5].im, x[6].im);
 }
 
@@ -365,6 +369,67 @@ GL_HD void pair_square(g2 u, g2 up, int4 c, g2* vk, g2* vkp) {
   const g2 sp = square(up);
   *vkp = red(g2{sp.re + pc.re, sp.im - pc.im});
 }
+
+// A value within R as two balanced limbs per part, the form of a twiddle: |c0| <= 2^30,
+// |c1| <= 2^29 + 16.
+GL_HD int4 as_limbs(g2 y) {
+  const uint32_t r = lo32((uint64_t)y.re), i = lo32((uint64_t)y.im);
+  return make_int4((int)(r << 1) >> 1, limb1(y.re) + (int)((r >> 30) & 1), (int)(i << 1) >> 1,
+                   limb1(y.im) + (int)((i >> 30) & 1));
+}
+GL_HD int4 conj(int4 w) { return make_int4(w.x, w.y, -w.z, -w.w); }
+
+// Biased accumulators of a sum of products of values in limbs.  A product adds at most
+// 3 2^60 to lo and 2^61 to mid, so two fit between folds (or one counted twice).
+struct Acc {
+  uint64_t rl, rm, il, im;
+};
+GL_HD Acc acc0() { return Acc{kAccLo, kAccMid, kAccLo, kAccMid}; }
+GL_HD void acc_mul(Acc& s, int4 x, int4 y) {
+  const int c2 = y.y * 2, d2 = y.w * 2, n0 = -y.z, n1 = -y.w, n2 = -d2;
+  s.rl = mad_s(x.w, n2, mad_s(x.z, n0, mad_s(x.y, c2, mad_s(x.x, y.x, s.rl))));
+  s.rm = mad_s(x.w, n0, mad_s(x.z, n1, mad_s(x.y, y.x, mad_s(x.x, y.y, s.rm))));
+  s.il = mad_s(x.w, c2, mad_s(x.z, y.x, mad_s(x.y, d2, mad_s(x.x, y.z, s.il))));
+  s.im = mad_s(x.w, y.x, mad_s(x.z, y.y, mad_s(x.y, y.z, mad_s(x.x, y.w, s.im))));
+}
+GL_HD g2 acc_fold(const Acc& s) { return g2{fold(s.rl, s.rm), fold(s.il, s.im)}; }
+
+// Coefficient b of u(y)^2 mod y^t - z; get(i) is coefficient i of u in limbs.  Within R.
+// The products u_i u_j of each half (i + j = b, and i + j = b + t times z) are summed over
+// i < j, folded two at a time, and doubled.
+template <typename Get>
+GL_HD g2 poly_square(const Get& get, int t, int b, int4 z) {
+  g2 out = {0, 0};
+#pragma unroll 1
+  for (int h = b < t - 1 ? 1 : 0; h >= 0; --h) {
+    const int s = b + h * t;  // i + j
+    int i = h ? b + 1 : 0, j = s - i;
+    g2 sum = {0, 0};
+#pragma unroll 1
+    for (; i + 1 < j - 1; i += 2, j -= 2) {
+      Acc a = acc0();
+      acc_mul(a, get(i), get(j));
+      acc_mul(a, get(i + 1), get(j - 1));
+      sum = red(add(sum, acc_fold(a)));
+    }
+    if (i < j) {
+      Acc a = acc0();
+      acc_mul(a, get(i), get(j));
+      sum = red(add(sum, acc_fold(a)));
+      ++i, --j;
+    }
+    sum = add(sum, sum);
+    if (i == j) {
+      Acc a = acc0();
+      const int4 x = get(i);
+      acc_mul(a, x, x);
+      sum = add(sum, acc_fold(a));
+    }
+    out = h ? cmul(red(sum), z) : red(add(out, red(sum)));
+  }
+  return out;
+}
+constexpr Limbs kMinusQuarter = limbs(kQ - (1ull << 59));
 
 // v 2^e within R, 0 <= e <= 60, |v| < 2^31
 GL_HD int64_t weighted(int v, int e) {

@@ -273,12 +273,12 @@ extern "C" {
 // largest magnitude of a transform stage's output.
 int hc_gf_square(int p, int W, int H, const int* v, long long* out, long long* peak) {
   const int M = W * H, N = 2 * M;
-  if (!gl::gf_supported(M)) return -1;
+  if (gl::gf_excess(M) != 1) return -1;
   std::vector<uint8_t> e;
   std::vector<gl::HostTw> k1, pair, k2;
   std::vector<gl::RowPair> rows;
   gl::gf_weights(p, N, e);
-  gl::gf_pass_tables(W, H, k1, pair, k2);
+  gl::gf_pass_tables(W, H, 1, k1, pair, k2);
   gl::gf_row_pairs(W, H, rows);
   const std::vector<int> rw = gl::radix_plan(W, 8), rh = gl::radix_plan(H, 8);
   int64_t pk = 0;

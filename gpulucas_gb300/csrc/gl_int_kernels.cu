@@ -212,7 +212,7 @@ __device__ __forceinline__ void int_row_body(const IterArgs& a, const int pair) 
     const bool self = r.x == r.y;
     g2* lb = self ? sp : sp + ls;
     // partner position q t + shift mod W, stepped along with t
-    const unsigned qW = (unsigned)a.in.qW, uW = (unsigned)W;
+    const unsigned qW = (unsigned)a.in.qV, uW = (unsigned)W;
     int u = (int)((qW * threadIdx.x + (unsigned)r.z) % uW);
     const int du = (int)(qW * (blockDim.x % uW) % uW);
 #pragma unroll 1
@@ -238,6 +238,76 @@ __device__ __forceinline__ void int_row_body(const IterArgs& a, const int pair) 
   }
 }
 
+// Row pass of a transform over polynomials (t > 1): a row is t interleaved lines of V
+// points, line b holding coefficient b, and a frequency's t coefficients are squared mod
+// y^t - z (poly_square).  With D = U - conj(U') as in pair_square,
+// V = U^2 - (1 + y) D^2 / 4 and V' = U'^2 + conj(the same), coefficient by coefficient.
+// U, U' and D are brought into limbs first (each is read t times), then one thread takes
+// one coefficient of one frequency; D^2 goes through shared memory, since its product with
+// y takes a coefficient from the neighbour.
+__device__ __forceinline__ void int_row_poly_body(const IterArgs& a, const int pair) {
+  extern __shared__ g2 ism[];
+  const int W = a.W, H = a.H, ls = a.in.ls_row, t = a.in.t, V = a.in.V;
+  const int4 r = __ldg(a.in.rows + pair);
+  const bool self = r.x == r.y;
+  const int rows = self ? 1 : 2, nl = rows * t;  // line mirror t + b
+  g2* other = ism + 2 * t * ls;
+  int4* dif = reinterpret_cast<int4*>(ism + 4 * t * ls);  // line b: D in limbs
+  g2* dsq = ism + 5 * t * ls;                             // line b: D^2
+  for (int idx = threadIdx.x; idx < rows * W; idx += blockDim.x) {
+    const int l = idx >= W;
+    const int m1 = idx - l * W;
+    const int v = m1 / t;
+    ism[(l * t + m1 - v * t) * ls + ipad(v)] = ldz(a.Z + ((l ? r.y : r.x) * W + m1));
+  }
+  __syncthreads();
+  g2* sp = int_line_fft<-1, true>(ism, other, nl, ls, a.in.pw, a.in.wf);
+  g2* nx = sp == ism ? other : ism;
+  int4* sl = reinterpret_cast<int4*>(sp);
+#pragma unroll 1
+  for (int step = 0; step < 3; ++step) {
+#pragma unroll 1
+    for (int x = threadIdx.x; x < W; x += blockDim.x) {
+      const int b = x / V;
+      const int v = x - b * V;  // frequency position
+      const int u = (int)(((unsigned)a.in.qV * (unsigned)v + (unsigned)r.z) % (unsigned)V);
+      if (self && u < v) continue;
+      const int la = ipad(v), lb = (self ? 0 : t * ls) + ipad(u);
+      const int4 z = __ldg(a.in.pair + (r.x * V + v));
+      if (step == 0) {
+        const g2 p = sp[la + b * ls], q = sp[lb + b * ls];
+        dif[la + b * ls] = gf::as_limbs(gf::red(g2{p.re - q.re, p.im + q.im}));
+        sl[la + b * ls] = gf::as_limbs(gf::red(p));
+        if (la != lb) sl[lb + b * ls] = gf::as_limbs(gf::red(q));
+      } else if (step == 1) {
+        nx[la + b * ls] = gf::poly_square([&](int c) { return sl[la + c * ls]; }, t, b, z);
+        if (la != lb) nx[lb + b * ls] = gf::poly_square([&](int c) { return sl[lb + c * ls]; }, t, b, gf::conj(z));
+        dsq[la + b * ls] = gf::poly_square([&](int c) { return dif[la + c * ls]; }, t, b, z);
+      } else {
+        const g2 e = gf::add(dsq[la + b * ls], b ? dsq[la + (b - 1) * ls] : gf::cmul(dsq[la + (t - 1) * ls], z));
+        const g2 pc = g2{gf::rmul(e.re, gf::kMinusQuarter), gf::rmul(e.im, gf::kMinusQuarter)};
+        nx[la + b * ls] = gf::red(gf::add(nx[la + b * ls], pc));
+        if (la != lb) {
+          const g2 s = nx[lb + b * ls];
+          nx[lb + b * ls] = gf::red(g2{s.re + pc.re, s.im - pc.im});
+        }
+      }
+    }
+    __syncthreads();
+  }
+  const g2* res = int_line_fft<+1, true>(nx, sp, nl, ls, a.in.pw, a.in.wi);
+  for (int idx = threadIdx.x; idx < rows * W; idx += blockDim.x) {
+    const int l = idx >= W;
+    const int m1 = idx - l * W;
+    const int v = m1 / t;
+    const int row = l ? r.y : r.x;
+    stz(a.Z2 + (m1 * H + row),
+        gf::cmul(res[(l * t + m1 - v * t) * ls + ipad(v)], __ldg(a.in.k2 + (row * W + m1))));
+  }
+}
+
+__global__ void __launch_bounds__(kRowThreads, 2) ki_row_poly(IterArgs a) { int_row_poly_body(a, blockIdx.x); }
+
 // Two builds for radices 8, 4, 2, 3: five CTAs of 192 threads per SM (64 registers) where the
 // row pairs are enough to fill them, else 80 registers, which shorten the dependent chains
 // of a pass with few CTAs (N = 49152, 49 pairs: 14.1 us against 15.6).
@@ -258,6 +328,16 @@ __device__ __forceinline__ long long check_word(long long r, int span, unsigned*
   return r;
 }
 
+// The two products of one point: unweight, check, -2 at word 0 (the LL step), store.
+__device__ __forceinline__ void int_store_products(const IterArgs& a, g2 v, int s0, unsigned* fl) {
+  const uchar2 e = __ldg(reinterpret_cast<const uchar2*>(a.in.e + s0));
+  const uchar2 sp = __ldg(reinterpret_cast<const uchar2*>(a.span + s0));
+  long long r0 = check_word(gf::unweighted(v.re, e.x), sp.x, fl);
+  const long long r1 = check_word(gf::unweighted(v.im, e.y), sp.y, fl);
+  if (s0 == 0) r0 -= 2;
+  *reinterpret_cast<longlong2*>(a.ll + s0) = make_longlong2(r0, r1);
+}
+
 // Inverse column pass: inverse length-H DFT, unweight, -2 at word 0, range checks, products.
 template <bool B57, int P>
 __device__ __forceinline__ void int_col_inv_body(const IterArgs& a, const int m1) {
@@ -269,16 +349,7 @@ __device__ __forceinline__ void int_col_inv_body(const IterArgs& a, const int m1
   if constexpr (P > 0) int_line_fft_ip<+1, B57, P>(ism, a.in.ph, a.in.hi);
   else res = int_line_fft<+1, B57>(ism, ism + ls, 1, ls, a.in.ph, a.in.hi);
   unsigned fl = 0;
-  for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) {
-    const int s0 = 2 * (m1 * H + m2);
-    const g2 v = res[ipad(m2)];
-    const uchar2 e = __ldg(reinterpret_cast<const uchar2*>(a.in.e + s0));
-    const uchar2 sp = __ldg(reinterpret_cast<const uchar2*>(a.span + s0));
-    long long r0 = check_word(gf::unweighted(v.re, e.x), sp.x, &fl);
-    const long long r1 = check_word(gf::unweighted(v.im, e.y), sp.y, &fl);
-    if (s0 == 0) r0 -= 2;  // word 0: the -2 of the LL step
-    *reinterpret_cast<longlong2*>(a.ll + s0) = make_longlong2(r0, r1);
-  }
+  for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) int_store_products(a, res[ipad(m2)], 2 * (m1 * H + m2), &fl);
   fl = __reduce_or_sync(0xffffffffu, fl);
   if ((threadIdx.x & 31) == 0 && fl) atomicOr(&a.status->flags, fl);
 }
@@ -320,7 +391,8 @@ void launch_pass(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which,
     if (from_state) c57 ? launch_col_fwd<true, true>(a, g, s) : launch_col_fwd<true, false>(a, g, s);
     else c57 ? launch_col_fwd<false, true>(a, g, s) : launch_col_fwd<false, false>(a, g, s);
   } else if (which == 1) {
-    if (r57) ki_row_sq<true, 256, 2><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
+    if (g.t > 1) ki_row_poly<<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
+    else if (r57) ki_row_sq<true, 256, 2><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
     else if (g.t_row <= 192 && a.in.nrows > kRowsFor5) ki_row_sq<false, 192, 5><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
     else ki_row_sq<false, 256, 3><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
   } else {
@@ -360,6 +432,7 @@ cudaError_t set_int_smem_limits() {
   if ((e = raise_col<false, 0>())) return e;
   if ((e = raise_col<true, 0>())) return e;
   if ((e = raise_col<false, kIntHeld>())) return e;
+  if ((e = raise(ki_row_poly))) return e;
   if ((e = raise(ki_row_sq<false, 192, 5>))) return e;
   if ((e = raise(ki_row_sq<false, 256, 3>))) return e;
   if ((e = raise(ki_row_sq<true, 256, 2>))) return e;

@@ -86,22 +86,27 @@ struct IntGeom {
   int t_col, t_row;        // threads per CTA
   bool col_p;              // column passes transform in place (kIntHeld points per thread)
   size_t sm_col, sm_row;   // dynamic shared memory bytes
-  LinePlan pw, ph;         // line plans (offsets into the stage tables)
+  LinePlan pw, ph;         // line plans of V and H points (offsets into the stage tables)
+  int t;                   // polynomial length (gf_excess), W = t V
 };
+// 16-byte slots of one row pair in the row pass: its 2 t lines of V points, ping-pong, and
+// for t > 1 the difference polynomials and their squares
+constexpr int int_row_slots(int V, int t) { return (t > 1 ? 6 : 4) * t * int_stride(V); }
 // Tables of the integer form: twiddles as four 31-bit limbs (gl_gf61.cuh), row pairs as
 // (row a, row b, shift, 0).
 struct IntArgs {
-  const int4* wf;             // stage values of the length-W line DFT, forward
+  const int4* wf;             // stage values of the length-V line DFT, forward
   const int4* wi;             // and inverse
   const int4* hf;             // length H
   const int4* hi;
-  const int4* k1;             // root(m1 k2, M) at m1*H + k2
-  const int4* pair;           // -(1 + root(k2 + H k1, M))/4 at k2*W + k1
-  const int4* k2;             // root(-m1 k2, M)/M at k2*W + m1
+  const int4* k1;             // root((m1/t) k2, L) at m1*H + k2
+  const int4* pair;           // -(1 + root(k2 + H k1, L))/4 at k2*V + k1 (t > 1: the root)
+  const int4* k2;             // root(-(m1/t) k2, L)/L at k2*W + m1
   const int4* rows;           // row pairs
   const unsigned char* e;     // weight exponents (column-major)
   int nrows;                  // number of row pairs
-  int qW;                     // 2^61 - 1 mod W
+  int t, V;                   // W = t V; the transform has length L = V H (gf_excess)
+  int qV;                     // 2^61 - 1 mod V
   int vmax;                   // bound on a loaded word's magnitude
   int ls_col, ls_row;
   LinePlan pw, ph;
@@ -129,7 +134,8 @@ struct IterArgs {
   signed char* hi;            // plain: i_hiBitArr, N
   Status* status;
   LinePlan pw, ph;
-  IntArgs in;                 // integer form (in.k1 null: this test has none)
+  IntArgs in;                 // integer form (in.k1 null: this test has none); last, so that
+                              // the batch kernels copy only what precedes it
 };
 
 // Resident form of a fused plan (short lengths): one thread-block cluster of C CTAs keeps

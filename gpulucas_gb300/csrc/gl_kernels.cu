@@ -560,7 +560,8 @@ __device__ __forceinline__ void load_desc(const IterArgs* __restrict__ tests, in
   // IterArgs is a plain struct of ints and pointers: copy it word by word
   const int* src = reinterpret_cast<const int*>(tests + t);
   int* dst = reinterpret_cast<int*>(&sa);
-  for (int i = threadIdx.x; i < (int)(sizeof(IterArgs) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
+  constexpr int words = (int)(offsetof(IterArgs, in) / sizeof(int));
+  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
   __syncthreads();
 }
 

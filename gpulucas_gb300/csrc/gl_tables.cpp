@@ -425,11 +425,16 @@ Gf groot(int64_t t, int64_t L) {
 }
 }  // namespace
 
-bool gf_supported(int M) {
-  if (M < 2) return false;
+int gf_excess(int M) {
   int odd = M;
   while (!(odd & 1)) odd >>= 1;
-  return 1575 % odd == 0;  // 3^2 5^2 7
+  int t = 1;
+  for (int pr : {3, 5, 7}) {
+    int e = 0;
+    for (; odd % pr == 0; ++e) odd /= pr;
+    for (int keep = pr == 7 ? 1 : 2; e > keep; --e) t *= pr;
+  }
+  return t;
 }
 
 void gf_root(int64_t t, int64_t L, uint64_t* c, uint64_t* d) {
@@ -464,20 +469,22 @@ void gf_stage_twiddles(int L, const int* radices, int nst, bool inverse, std::ve
   (void)L;
 }
 
-void gf_pass_tables(int W, int H, std::vector<HostTw>& k1, std::vector<HostTw>& pair, std::vector<HostTw>& k2t) {
-  const int64_t M = (int64_t)W * H;
+void gf_pass_tables(int W, int H, int t, std::vector<HostTw>& k1, std::vector<HostTw>& pair,
+                    std::vector<HostTw>& k2t) {
+  const int V = W / t;
+  const int64_t M = (int64_t)W * H, L = (int64_t)V * H;
   k1.resize((size_t)M);
-  pair.resize((size_t)M);
+  pair.resize((size_t)L);
   k2t.resize((size_t)M);
-  const uint64_t minv = gf::powq((uint64_t)M, gf::kQ - 2);
+  const uint64_t linv = gf::powq((uint64_t)L, gf::kQ - 2);
   const uint64_t quarter = gf::kQ - (1ull << 59);  // -1/4
   parallel_for(M, [&](int64_t b, int64_t e) {
     Gf base{1, 0}, cur{1, 0};
     for (int64_t i = b; i < e; ++i) {
-      const int64_t m1 = i / H, j = i - m1 * H;
+      const int64_t a = i / H / t, j = i % H;
       if (i == b || j == 0) {
-        base = groot(m1, M);
-        cur = groot(m1 * j, M);
+        base = groot(a, L);
+        cur = groot(a * j, L);
       }
       k1[(size_t)i] = gf_pack(cur.re, cur.im);
       cur = gmul(cur, base);
@@ -485,31 +492,34 @@ void gf_pass_tables(int W, int H, std::vector<HostTw>& k1, std::vector<HostTw>& 
     for (int64_t i = b; i < e; ++i) {
       const int64_t r = i / W, j = i - r * W;
       if (i == b || j == 0) {
-        base = groot(-r, M);
-        cur = groot(-r * j, M);
-        cur = {gf::mulq(cur.re, minv), gf::mulq(cur.im, minv)};
+        base = groot(-r, L);
+        cur = groot(-r * (j / t), L);
+        cur = {gf::mulq(cur.re, linv), gf::mulq(cur.im, linv)};
       }
       k2t[(size_t)i] = gf_pack(cur.re, cur.im);
-      cur = gmul(cur, base);
+      if ((j + 1) % t == 0) cur = gmul(cur, base);
     }
-    base = groot(1, W);
+  });
+  parallel_for(L, [&](int64_t b, int64_t e) {
+    Gf base = groot(1, V), cur{1, 0};
     for (int64_t i = b; i < e; ++i) {
-      const int64_t r = i / W, j = i - r * W;
-      if (i == b || j == 0) cur = groot(r + (int64_t)H * j, M);
-      pair[(size_t)i] = gf_pack(gf::mulq(addq(cur.re, 1), quarter), gf::mulq(cur.im, quarter));
+      const int64_t r = i / V, j = i - r * V;
+      if (i == b || j == 0) cur = groot(r + (int64_t)H * j, L);
+      pair[(size_t)i] = t > 1 ? gf_pack(cur.re, cur.im)
+                              : gf_pack(gf::mulq(addq(cur.re, 1), quarter), gf::mulq(cur.im, quarter));
       cur = gmul(cur, base);
     }
   });
 }
 
-void gf_row_pairs(int W, int H, std::vector<RowPair>& rows) {
-  const int64_t M = (int64_t)W * H;
-  const int64_t qM = (int64_t)(gf::kQ % (uint64_t)M);
+void gf_row_pairs(int V, int H, std::vector<RowPair>& rows) {
+  const int64_t L = (int64_t)V * H;
+  const int64_t qL = (int64_t)(gf::kQ % (uint64_t)L);
   rows.clear();
   for (int64_t k2 = 0; k2 < H; ++k2) {
-    const int64_t b = qM * k2 % H;
+    const int64_t b = qL * k2 % H;
     if (b < k2) continue;
-    rows.push_back({(int32_t)k2, (int32_t)b, (int32_t)((qM * k2 - b) / H % W), 0});
+    rows.push_back({(int32_t)k2, (int32_t)b, (int32_t)((qL * k2 - b) / H % V), 0});
   }
 }
 

@@ -66,9 +66,12 @@ HostCplx pair_coeff(int64_t k, int64_t M);
 struct HostTw {
   int32_t c0, c1, d0, d1;
 };
-// whether GF(q^2) has the roots of unity that M complex points need (odd part of M
-// dividing 3^2 5^2 7; N = 2 M is then prime to 61, so the weights are powers of two)
-bool gf_supported(int M);
+// GF(q^2) has roots of unity of order M for odd parts of M that divide 3^2 5^2 7.  For
+// other M the transform is of length M/t, t the excess odd part, over polynomials of degree
+// below t: u[b + t a] is coefficient b of element a, and frequency k holds a polynomial mod
+// y^t - root(k, M/t).  Returns t (1: a plain transform).  N = 2 M is prime to 61, so the
+// weights are powers of two.
+int gf_excess(int M);
 // exp(-2 pi i t / L)'s counterpart: a multiplicative family of roots of unity (root(t, L)
 // root(u, L) = root(t + u, L), root(t k, L k) = root(t, L)), as c + i d with 0 <= c, d < q
 void gf_root(int64_t t, int64_t L, uint64_t* c, uint64_t* d);
@@ -76,15 +79,16 @@ HostTw gf_pack(uint64_t c, uint64_t d);
 // Values of one Stockham line DFT of length L: for every stage after the first, span Ns
 // and radix R, w^q (q = 1..R-1) of w = root(+-k, Ns R) at off[s] + (q-1) Ns + k.
 void gf_stage_twiddles(int L, const int* radices, int nst, bool inverse, std::vector<HostTw>& tw, int* off);
-// k1[m1 H + k2] = root(m1 k2, M); k2t[k2 W + m1] = root(-m1 k2, M) / M;
-// pair[k2 W + k1] = -(1 + root(k2 + H k1, M)) / 4, M = W H
-void gf_pass_tables(int W, int H, std::vector<HostTw>& k1, std::vector<HostTw>& pair, std::vector<HostTw>& k2t);
-// The row pairs of the row pass.  Frequency k = k2 + H k1 pairs with q k mod M, so row k2
-// pairs with row q k2 mod H, and in it position k1 with q k1 + shift mod W.
+// For t = gf_excess(W H), W = t V, L = V H (t = 1: V = W, L = M):
+// k1[m1 H + k2] = root((m1/t) k2, L); k2t[k2 W + m1] = root(-(m1/t) k2, L) / L;
+// pair[k2 V + k1] = -(1 + root(k2 + H k1, L)) / 4 for t = 1, root(k2 + H k1, L) for t > 1
+void gf_pass_tables(int W, int H, int t, std::vector<HostTw>& k1, std::vector<HostTw>& pair, std::vector<HostTw>& k2t);
+// The row pairs of the row pass.  Frequency k = k2 + H k1 pairs with q k mod L, so row k2
+// pairs with row q k2 mod H, and in it position k1 with q k1 + shift mod V.
 struct RowPair {
   int32_t a, b, shift, pad;  // rows a <= b (a == b: a row paired with itself)
 };
-void gf_row_pairs(int W, int H, std::vector<RowPair>& rows);
+void gf_row_pairs(int V, int H, std::vector<RowPair>& rows);
 // weight exponent of word j: A[j] = 2^(r/N) = 2^e with r = ceil(jp/N) N - jp, e = r N^-1 mod 61
 void gf_weights(int p, int N, std::vector<uint8_t>& e);
 

@@ -169,3 +169,15 @@ def test_balanced_split_in_32_bits_equals_64(hc):
             hc.hc_balanced_split(s, bits, d, h)
             hc.hc_balanced_split32(s, bits, d2, h2)
             assert (d.value, h.value) == (d2.value, h2.value), (s, bits)
+
+
+# lengths whose odd part the field's roots do not cover: transforms over polynomials mod
+# y^t - z, t = 3, 5, 7, 9, 25, 27, 49, with and without radices 5 and 7 in the rows
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,N", [(100003, 5184), (500009, 27648), (300007, 16000), (748003, 44100), (300007, 16200),
+                                 (1000003, 52500), (1000003, 54432), (1500007, 78400)])
+def test_polynomial_transforms_equal_fp64_form(gl, p, N):
+    for k in (1, 66):
+        a, ra, _ = _products(gl, p, N, k)
+        b, rb, _ = _products(gl, p, N, k, error_limit=0.39)
+        assert ra.status == rb.status == 0 and (a == b).all(), k
