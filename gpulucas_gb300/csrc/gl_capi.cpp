@@ -342,28 +342,45 @@ constexpr int kMaxIntPoly = 49;
 
 // Geometry of the integer form on an H x W layout; false where its polynomials do not fit
 // the rows or a CTA's lines its shared memory.
-bool choose_int_geom(int H, int W, IntGeom* g, bool col_p = false) {
+// in_place, wide, rc, rr: the variants autotune_int_layout times.
+struct IntVariant {
+  bool in_place = false;  // column passes in place
+  bool wide = false;      // a thread per two points instead of one per butterfly
+  int rc = kMaxRadix, rr = kMaxRadix;  // largest radix of the columns and rows
+};
+bool choose_int_geom(int H, int W, IntGeom* g, const IntVariant& var = IntVariant()) {
   g->t = gf_excess(H * W);
   if (g->t > kMaxIntPoly || W % g->t) return false;
   const int V = W / g->t;
-  if (!fill_line_plan(V, &g->pw) || !fill_line_plan(H, &g->ph)) return false;
+  if (!fill_line_plan(V, &g->pw, var.rr) || !fill_line_plan(H, &g->ph, var.rc)) return false;
   int_stage_offsets(&g->pw);
   int_stage_offsets(&g->ph);
-  auto threads = [](int butterflies) {
-    const int t = round_up32(butterflies);
+  auto threads = [](int n) {
+    const int t = round_up32(n);
     return t < 64 ? 64 : (t > kMaxThreads ? kMaxThreads : t);
   };
-  g->col_p = col_p;
-  g->t_col = threads((H + 7) / 8);
-  g->t_row = g->t > 1 ? threads(W) : row_threads(W, g->pw, threads((2 * W + 7) / 8));
-  for (int s = 0; s < g->ph.nst && col_p; ++s) {
+  g->col_p = var.in_place;
+  g->t_col = threads(var.wide ? H / 2 : (H + var.rc - 1) / var.rc);
+  g->t_row = var.wide || g->t > 1 ? threads(W) : row_threads(W, g->pw, threads((2 * W + var.rr - 1) / var.rr));
+  for (int s = 0; s < g->ph.nst && var.in_place; ++s) {
     // radices 8, 4, 2, 3 only, and no more butterflies than the threads hold
     const int R = g->ph.radix[s];
     if (R == 5 || R == 7 || H / R > kIntHeld / R * g->t_col) return false;
   }
-  g->sm_col = (size_t)(col_p ? 1 : 2) * int_stride(H) * 16;
+  g->sm_col = (size_t)(var.in_place ? 1 : 2) * int_stride(H) * 16;
   g->sm_row = (size_t)int_row_slots(V, g->t) * 16;
   return g->sm_col <= (size_t)kMaxIntSmem && g->sm_row <= (size_t)kMaxIntSmem;
+}
+
+// The variant for a layout chosen without timing: below 2^17 points the one the search
+// usually picks there.
+IntVariant small_variant(int M) {
+  IntVariant v;
+  if (M < (1 << 17)) {
+    v.rc = v.rr = 4;
+    v.wide = true;
+  }
+  return v;
 }
 
 // Column length of the first layout of the cost model that the integer form can run, or 0.
@@ -373,6 +390,10 @@ int first_int_layout(int M, int sms) {
     if (choose_int_geom(c.second, M / c.second, &g)) return c.second;
   return 0;
 }
+
+// Whether the passes touch the tables they will read at their start (IntArgs::touch): where
+// at most one CTA runs per SM, its L1 is empty and has room for all of them.
+int int_touch(int H, int W) { return W <= 152 * 2 && H / 2 < 152 * 2; }
 
 // Whether the products of (p, N) are determined by their residues mod q = 2^61 - 1 for
 // every state the iteration can reach: words are at most 2^LO plus a carry in magnitude,
@@ -529,10 +550,10 @@ TunedLayout autotune_layout(int M, int n, int sms, cudaStream_t s, double* ms_ou
 }
 
 // Device time of one integer-form iteration on the H x (M / H) layout, or -1.
-double time_int_layout(int M, int H, bool col_p, int n, int iters, cudaStream_t s) {
+double time_int_layout(int M, int H, const IntVariant& var, int n, int iters, cudaStream_t s) {
   IntGeom g{};
   const int W = M / H, N = 2 * M;
-  if (!choose_int_geom(H, W, &g, col_p)) return -1.0;
+  if (!choose_int_geom(H, W, &g, var)) return -1.0;
   std::vector<RowPair> rows;
   gf_row_pairs(W / g.t, H, rows);
   LinePlan pw = g.pw, ph = g.ph;
@@ -561,10 +582,7 @@ double time_int_layout(int M, int H, bool col_p, int n, int iters, cudaStream_t 
     a.in.wf = (const int4*)buf[9]; a.in.wi = (const int4*)buf[10];
     a.in.hf = (const int4*)buf[11]; a.in.hi = (const int4*)buf[12];
     a.in.rows = (const int4*)buf[13]; a.status = (Status*)buf[14];
-    a.in.nrows = (int)rows.size();
-    a.in.t = g.t; a.in.V = W / g.t;
-    a.in.qV = (int)(((1ull << 61) - 1) % (uint64_t)a.in.V);
-    a.in.ls_col = int_stride(H); a.in.ls_row = int_stride(a.in.V); a.in.pw = g.pw; a.in.ph = g.ph;
+    gl_int_args(H, W, g, (int)rows.size(), &a.in);
     for (int i = 0; i < 2 && ok; ++i) ok = launch_int_iteration(a, g, s, false) == cudaSuccess;
     ok = ok && cudaEventRecord(e0, s) == cudaSuccess;
     for (int i = 0; i < iters && ok; ++i) ok = launch_int_iteration(a, g, s, false) == cudaSuccess;
@@ -582,10 +600,13 @@ double time_int_layout(int M, int H, bool col_p, int n, int iters, cudaStream_t 
 
 // Layout of the integer form for M complex points on this device: the candidates of the
 // layout model that it can run are timed, with two line buffers per column and in place,
-// and the fastest kept, once per (M, SM count) per process.  H = 0: no layout.
+// and the fastest kept, once per (M, SM count) per process.  Below 2^17 points lines are
+// too few to fill the device and a pass is its chain of latencies: there the three fastest
+// are also timed with radix-4 stages (more threads, shorter butterflies) and with a thread
+// per two points (the loads, dicing and twiddles of a line side by side).  H = 0: no layout.
 struct IntTuned {
   int H = 0;
-  bool col_p = false;
+  IntVariant var;
   double ms = 1e300;
 };
 std::map<std::pair<int, int>, IntTuned> g_int_tune_cache;
@@ -598,18 +619,35 @@ IntTuned autotune_int_layout(int M, int n, int sms, cudaStream_t s) {
     if (it != g_int_tune_cache.end()) return it->second;
   }
   IntTuned best;
-  int timed = 0;
+  std::vector<std::pair<double, int>> timed;  // column lengths by their best time
+  auto consider = [&](int H, const IntVariant& var) {
+    const double ms = time_int_layout(M, H, var, n, M >= (1 << 18) ? 10 : 40, s);
+    if (ms > 0.0 && ms < best.ms) best = IntTuned{H, var, ms};
+    return ms;
+  };
   for (const auto& c : ranked_layouts(M, sms)) {
-    if (timed == kIntLayoutsTimed) break;
-    bool any = false;
+    if (timed.size() == (size_t)kIntLayoutsTimed) break;
+    double ms = -1.0;
     for (bool p : {false, true}) {
-      const double ms = time_int_layout(M, c.second, p, n, M >= (1 << 18) ? 10 : 40, s);
-      if (ms <= 0.0) continue;
-      any = true;
-      if (ms < best.ms) best = IntTuned{c.second, p, ms};
+      IntVariant v;
+      v.in_place = p;
+      const double t = consider(c.second, v);
+      if (t > 0.0 && (ms <= 0.0 || t < ms)) ms = t;
     }
-    timed += any;
+    if (ms > 0.0) timed.emplace_back(ms, c.second);
   }
+  std::sort(timed.begin(), timed.end());
+  for (size_t i = 0; i < timed.size() && i < 3 && M < (1 << 17); ++i)
+    for (int rc : {8, 4})
+      for (int rr : {8, 4})
+        for (bool wide : {false, true}) {
+          if (rc == 8 && rr == 8 && !wide) continue;
+          IntVariant v;
+          v.rc = rc;
+          v.rr = rr;
+          v.wide = wide;
+          consider(timed[i].second, v);
+        }
   if (!best.H) return best;
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   g_int_tune_cache[{M, sms}] = best;
@@ -776,6 +814,26 @@ cudaError_t gl_make_stream(cudaStream_t* s, int level) {
   return cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, prio);
 }
 
+void gl_int_args(int H, int W, const IntGeom& g, int nrows, IntArgs* in) {
+  in->nrows = nrows;
+  in->touch = int_touch(H, W);
+  in->t = g.t;
+  in->V = W / g.t;
+  in->qV = (int)(((1ull << 61) - 1) % (uint64_t)in->V);
+  in->ls_col = int_stride(H);
+  in->ls_row = int_stride(in->V);
+  in->pw = g.pw;
+  in->ph = g.ph;
+}
+
+bool gl_int_layout(int p, int N, int* H, IntGeom* g) {
+  int vmax = 0;
+  if (!int_range_ok(p, N, &vmax) || !int_roundoff_ok(p, N, 0.4)) return false;
+  const int M = N / 2;
+  if (!(*H = first_int_layout(M, 152))) return false;
+  return choose_int_geom(*H, M / *H, g, small_variant(M));
+}
+
 void gl_plan_note_external_iterations(gl_plan* pl, int64_t iters) {
   pl->iters_done += iters;
   pl->from_state = false;
@@ -845,15 +903,8 @@ static int build_int_tables(gl_plan* pl, int vmax) {
       (rc = up(&in.e, e_c.data(), e_c.size())))
     return rc;
   GL_CUDA(cudaStreamSynchronize(pl->stream));  // host tables go out of scope
-  in.nrows = (int)rows.size();
-  in.t = t;
-  in.V = V;
-  in.qV = (int)(((1ull << 61) - 1) % (uint64_t)V);
+  gl_int_args(H, W, pl->ig, (int)rows.size(), &in);
   in.vmax = vmax;
-  in.ls_col = int_stride(H);
-  in.ls_row = int_stride(V);
-  in.pw = pl->ig.pw;
-  in.ph = pl->ig.ph;
   GL_CUDA(set_int_smem_limits());
   pl->int_form = true;
   return GL_OK;
@@ -916,15 +967,18 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   // The integer form, unless an option names a variant of the FP64 kernels.
   IntGeom ig{};
   int vmax = 0;
-  bool int_p = false;
+  IntVariant int_var;
   bool int_form = o.mode == GL_MODE_FUSED && !resident && !fp64_only && !sms_override && !names_fp64_variant(o) &&
                   int_range_ok(p, N, &vmax) && int_roundoff_ok(p, N, o.error_limit);
   if (int_form) {
     IntTuned it;
     if (o.autotune && !sms_override) it = autotune_int_layout(M, n, sms, 0);
-    else it.H = first_int_layout(M, sms);
+    else {
+      it.H = first_int_layout(M, sms);
+      it.var = small_variant(M);
+    }
     force_h = it.H;
-    int_p = it.col_p;
+    int_var = it.var;
     int_form = it.H != 0;
   }
   bool col_ip = false, col_pf = false, col_ws = false;
@@ -957,7 +1011,7 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   if (rc == GL_ERR_SIZE && col_ip && o.col_inplace <= 0)  // the searched layout cannot: two buffers
     rc = choose_fused_geom(M, force_h, sms, &fg, cap_c, cap_r, false);
   if (rc != GL_OK) return rc;
-  int_form = int_form && choose_int_geom(fg.H, fg.W, &ig, int_p);
+  int_form = int_form && choose_int_geom(fg.H, fg.W, &ig, int_var);
 
   gl_plan* pl = new (std::nothrow) gl_plan();
   if (!pl) return GL_ERR_NOMEM;

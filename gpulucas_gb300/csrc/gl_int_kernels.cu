@@ -34,6 +34,19 @@ __device__ __forceinline__ void stz(DevCplx* p, g2 v) {
   *reinterpret_cast<longlong2*>(p) = make_longlong2(v.re, v.im);
 }
 
+// Starts the load of n table entries into L1: one word of every 128-byte line, into a
+// register nobody reads, so the pass does not wait for them here.  Where few CTAs run, a
+// pass is a chain of latencies and every stage would wait on L2 for its twiddles.
+__device__ __forceinline__ void touch(const int4* p, int n) {
+  for (int i = threadIdx.x * 8; i < n; i += blockDim.x * 8) {
+    asm volatile("{\n .reg .s32 d;\n ld.global.nc.s32 d, [%0];\n}" ::"l"(p + i));
+  }
+}
+__device__ __forceinline__ int plan_slots(const LinePlan& lp) {  // entries of its stage table
+  const int s = lp.nst - 1, R = lp.radix[s];
+  return lp.off[s] + (s ? (R - 1) * (lp.L / R) : 0);
+}
+
 // Stockham DIT stage, out of place, as in the FP64 form: butterfly j of a line reads
 // x[j + q L/R], multiplies by w^q and writes x[(j - k) R + k + p Ns], k = j mod Ns.
 // The position k needs no division in the first stages (Ns a power of two) or the last
@@ -156,8 +169,12 @@ template <bool FROM_STATE, int NC, bool B57, int P>
 __device__ __forceinline__ void int_col_fwd_body(const IterArgs& a, const int m1) {
   extern __shared__ g2 ism[];
   const int H = a.H, W = a.W, ls = a.in.ls_col;
+  if (P == 0 && a.in.touch) {
+    touch(a.in.hf, plan_slots(a.in.ph));
+    touch(a.in.k1 + m1 * H, H);
+  }
   bool wide = false;
-#pragma unroll 1
+#pragma unroll (P == 0 ? 2 : 1)
   for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) {
     int v0, v1;
     load_point<FROM_STATE, NC>(a, m1, m2, &v0, &v1);
@@ -198,6 +215,13 @@ __device__ __forceinline__ void int_row_body(const IterArgs& a, const int pair) 
   {
     const int4 r = row_pair(a.in.rows, pair);
     nl = r.x == r.y ? 1 : 2;
+    if (a.in.touch) {
+      touch(a.in.wf, plan_slots(a.in.pw));
+      touch(a.in.pair + r.x * W, W);
+      touch(a.in.wi, plan_slots(a.in.pw));
+      touch(a.in.k2 + r.x * W, W);
+      touch(a.in.k2 + r.y * W, W);
+    }
     for (int idx = threadIdx.x; idx < nl * W; idx += blockDim.x) {
       const int l = idx >= W;
       const int k1 = idx - l * W;
@@ -251,6 +275,13 @@ __device__ __forceinline__ void int_row_poly_body(const IterArgs& a, const int p
   const int4 r = __ldg(a.in.rows + pair);
   const bool self = r.x == r.y;
   const int rows = self ? 1 : 2, nl = rows * t;  // line mirror t + b
+  if (a.in.touch) {
+    touch(a.in.wf, plan_slots(a.in.pw));
+    touch(a.in.pair + r.x * V, V);
+    touch(a.in.wi, plan_slots(a.in.pw));
+    touch(a.in.k2 + r.x * W, W);
+    touch(a.in.k2 + r.y * W, W);
+  }
   g2* other = ism + 2 * t * ls;
   int4* dif = reinterpret_cast<int4*>(ism + 4 * t * ls);  // line b: D in limbs
   g2* dsq = ism + 5 * t * ls;                             // line b: D^2
@@ -343,6 +374,7 @@ template <bool B57, int P>
 __device__ __forceinline__ void int_col_inv_body(const IterArgs& a, const int m1) {
   extern __shared__ g2 ism[];
   const int H = a.H, ls = a.in.ls_col;
+  if (P == 0 && a.in.touch) touch(a.in.hi, plan_slots(a.in.ph));
   for (int k2 = threadIdx.x; k2 < H; k2 += blockDim.x) ism[ipad(k2)] = ldz(a.Z2 + (size_t)m1 * H + k2);
   __syncthreads();
   const g2* res = ism;

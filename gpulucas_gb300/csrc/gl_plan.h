@@ -64,3 +64,8 @@ cudaError_t gl_make_stream(cudaStream_t* s, int level);
 double gl_model_iteration_cost(int M, int sms);
 // cost of one column-pass unit and one row-pass unit of a fused plan (FP64 model)
 double gl_plan_unit_cost(const gl_plan* pl, bool row);
+// Layout of the integer form for (p, N), chosen without timing; false where a plan with the
+// default limit would not use it.
+bool gl_int_layout(int p, int N, int* H, IntGeom* g);
+// the fields of IntArgs that follow from the layout (the tables' pointers are the caller's)
+void gl_int_args(int H, int W, const IntGeom& g, int nrows, gl::IntArgs* in);
