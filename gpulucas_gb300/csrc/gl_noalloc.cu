@@ -9,16 +9,21 @@
 // and everything else the iterations need -- the two FFT work arrays, the weight,
 // flag and twiddle tables of the test, the carry-save digits and the round-off
 // status word -- lives in one file-scope __device__ array below.  It is sized for
-// N <= kNoAllocMaxN (65536 words, about 3.3 MiB) and stays resident on every GPU that
+// N <= kNoAllocMaxN (65536 words, about 5.9 MiB) and stays resident on every GPU that
 // loads this library until the process exits.
 //
-// The iterations are the plain form (one kernel per reference step), launched
-// through the same launchers as a plan of GL_MODE_PLAIN, so the products equal those
-// of gl_iterate bit for bit.
+// The iterations are the integer form (gl_int_kernels.cu) where a plan of (p, N) would use
+// it, one in 64 and the last of a call in FP64; elsewhere all are FP64.  FP64 iterations
+// are the plain form (one kernel per reference step), launched through the same launchers
+// as a plan of GL_MODE_PLAIN.  The products equal those of gl_iterate bit for bit.
+// N = 65536: 110.7 us per iteration in the plain form, whose twenty launches each read and
+// write the whole signal, against 22 in the integer form's three.
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "gl_internal.h"
+#include "gl_plan.h"
 #include "gl_tables.h"
 
 namespace gl {
@@ -40,7 +45,18 @@ constexpr size_t kOffDigit = kOffAinv + align256(sizeof(double) * kNoAllocMaxN);
 constexpr size_t kOffHi = kOffDigit + align256(sizeof(int) * kNoAllocMaxN);
 constexpr size_t kOffFlags = kOffHi + align256(kNoAllocMaxN);
 constexpr size_t kOffStatus = kOffFlags + align256(kNoAllocMaxN);
-constexpr size_t kScratchBytes = kOffStatus + align256(sizeof(Status));
+// the integer form's state and tables
+constexpr int kNoAllocMaxLine = 4096;  // points of a line, and rows
+constexpr size_t kOffLl = kOffStatus + align256(sizeof(Status));
+constexpr size_t kOffFlagsC = kOffLl + align256(sizeof(long long) * kNoAllocMaxN);
+constexpr size_t kOffSpan = kOffFlagsC + align256(kNoAllocMaxN);
+constexpr size_t kOffExp = kOffSpan + align256(kNoAllocMaxN);
+constexpr size_t kOffK1 = kOffExp + align256(kNoAllocMaxN);
+constexpr size_t kOffK2 = kOffK1 + align256(sizeof(HostTw) * kNoAllocMaxM);
+constexpr size_t kOffIntPair = kOffK2 + align256(sizeof(HostTw) * kNoAllocMaxM);
+constexpr size_t kOffStages = kOffIntPair + align256(sizeof(HostTw) * kNoAllocMaxM);  // wf, wi, hf, hi
+constexpr size_t kOffRows = kOffStages + 4 * align256(sizeof(HostTw) * kNoAllocMaxLine);
+constexpr size_t kScratchBytes = kOffRows + align256(sizeof(RowPair) * kNoAllocMaxLine);
 
 // The scratch.  In host code this name is only a host-side stand-in for the symbol,
 // never a device address: the address comes from cudaGetSymbolAddress below.
@@ -54,9 +70,21 @@ static double h_Ainv[kNoAllocMaxN];
 static unsigned char h_flags[kNoAllocMaxN];
 static Status h_status;
 
+// The integer form of the test whose tables are staged (H = 0: it has none).
+static struct {
+  int H = 0;
+  IntGeom g{};
+  std::vector<HostTw> k1, pair, k2, stages[4];
+  std::vector<RowPair> rows;
+  std::vector<uint8_t> flags, span, e;
+} h_int;
+
 struct DeviceSlot {
   unsigned char* base = nullptr;  // device address of g_noalloc_scratch on this device
   int p = 0, N = 0;               // test whose tables the scratch holds
+  int H = 0;                      // integer form: column length, geometry (H = 0: none)
+  IntGeom g{};
+  int nrows = 0;
 };
 static DeviceSlot g_slots[kMaxDevices];
 static std::mutex g_mutex;  // host-side state: staging buffers and the slots
@@ -74,6 +102,46 @@ void build_tables(int p, int N) {
   for (int j = 0; j < N; ++j) weight_entry(p, N, j, (double)M, &h_A[j], &h_Ainv[j]);
   for (int j = 0; j < N; ++j) h_flags[j] = word_flags(p, N, j);
 }
+
+// The same for the integer form, from the helpers a plan's tables are built from.
+void build_int_tables(int p, int N, int n) {
+  h_int.H = 0;
+  int H = 0;
+  if (!gl_int_layout(p, N, &H, &h_int.g)) return;
+  const int M = N / 2, W = M / H, t = h_int.g.t, V = W / t;
+  gf_pass_tables(W, H, t, h_int.k1, h_int.pair, h_int.k2);
+  gf_row_pairs(V, H, h_int.rows);
+  std::vector<uint8_t> e;
+  gf_weights(p, N, e);
+  int off[8];
+  const LinePlan &pw = h_int.g.pw, &ph = h_int.g.ph;
+  gf_stage_twiddles(V, pw.radix, pw.nst, false, h_int.stages[0], off);
+  gf_stage_twiddles(V, pw.radix, pw.nst, true, h_int.stages[1], off);
+  gf_stage_twiddles(H, ph.radix, ph.nst, false, h_int.stages[2], off);
+  gf_stage_twiddles(H, ph.radix, ph.nst, true, h_int.stages[3], off);
+  for (const auto& s : h_int.stages)
+    if (s.size() > (size_t)kNoAllocMaxLine) return;
+  if (h_int.rows.size() > (size_t)kNoAllocMaxLine) return;
+  h_int.flags.resize((size_t)N);
+  h_int.span.resize((size_t)N);
+  h_int.e.resize((size_t)N);
+  for (int j = 0; j < N; ++j) {  // column-major
+    const int m = j >> 1, m2 = m / W, m1 = m - m2 * W;
+    const int c = 2 * (m1 * H + m2) + (j & 1);
+    int tot = 0;
+    for (int i = 0; i <= n; ++i) tot += word_bits(p, N, (j + i) % N);
+    h_int.flags[(size_t)c] = h_flags[j];
+    h_int.span[(size_t)c] = (uint8_t)(tot > 255 ? 255 : tot);
+    h_int.e[(size_t)c] = e[(size_t)j];
+  }
+  h_int.H = H;
+}
+
+constexpr size_t stage_offset(int i) { return kOffStages + (size_t)i * align256(sizeof(HostTw) * kNoAllocMaxLine); }
+
+// One FP64 iteration in this many, and the last of a call: the round-off a call reports
+// is theirs.
+constexpr int kNoAllocFp64Every = 64;
 
 }  // namespace
 }  // namespace gl
@@ -136,6 +204,22 @@ extern "C" int gl_iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* l
       slot.p = slot.N = 0;
       return GL_ERR_CUDA;
     }
+    build_int_tables(p, N, n);
+    if (h_int.H) {
+      auto up = [&](size_t off, const auto& v) {
+        return cudaMemcpyAsync(base + off, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, s) != cudaSuccess;
+      };
+      bool bad = up(kOffFlagsC, h_int.flags) || up(kOffSpan, h_int.span) || up(kOffExp, h_int.e) ||
+                 up(kOffK1, h_int.k1) || up(kOffK2, h_int.k2) || up(kOffIntPair, h_int.pair) || up(kOffRows, h_int.rows);
+      for (int i = 0; i < 4; ++i) bad = bad || up(stage_offset(i), h_int.stages[i]);
+      if (bad || set_int_smem_limits() != cudaSuccess) {
+        slot.p = slot.N = 0;
+        return GL_ERR_CUDA;
+      }
+    }
+    slot.H = h_int.H;
+    slot.g = h_int.g;
+    slot.nrows = (int)h_int.rows.size();
     slot.p = p;
     slot.N = N;
   }
@@ -159,9 +243,36 @@ extern "C" int gl_iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* l
   if (ll_out != ll_in &&
       cudaMemcpyAsync(ll_out, ll_in, sizeof(int64_t) * N, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return GL_ERR_CUDA;
-  if (launch_dice(a, s) != cudaSuccess) return GL_ERR_CUDA;
-  for (int64_t i = 0; i < iters; ++i)
-    if (launch_plain_iteration(a, pg, s) != cudaSuccess) return GL_ERR_CUDA;
+  if (!slot.H || iters < 2) {
+    if (launch_dice(a, s) != cudaSuccess) return GL_ERR_CUDA;
+    for (int64_t i = 0; i < iters; ++i)
+      if (launch_plain_iteration(a, pg, s) != cudaSuccess) return GL_ERR_CUDA;
+  } else {
+    const int H = slot.H, W = M / H;
+    IterArgs b = a;
+    b.W = W; b.H = H; b.G = 1;
+    b.ll = reinterpret_cast<long long*>(base + kOffLl);
+    b.flags = base + kOffFlagsC;
+    b.span = base + kOffSpan;
+    auto tw = [&](size_t off) { return reinterpret_cast<const int4*>(base + off); };
+    b.in.wf = tw(stage_offset(0)); b.in.wi = tw(stage_offset(1));
+    b.in.hf = tw(stage_offset(2)); b.in.hi = tw(stage_offset(3));
+    b.in.k1 = tw(kOffK1); b.in.pair = tw(kOffIntPair); b.in.k2 = tw(kOffK2); b.in.rows = tw(kOffRows);
+    b.in.e = base + kOffExp;
+    gl_int_args(H, W, slot.g, slot.nrows, &b.in);
+    int64_t left = iters;
+    while (left > 0) {
+      const int64_t k = (left < kNoAllocFp64Every ? left : kNoAllocFp64Every) - 1;
+      if (k > 0) {
+        if (launch_permute_words(b, a.ll, b.ll, true, s) != cudaSuccess) return GL_ERR_CUDA;
+        for (int64_t i = 0; i < k; ++i)
+          if (launch_int_iteration(b, slot.g, s, false) != cudaSuccess) return GL_ERR_CUDA;
+        if (launch_permute_words(b, b.ll, a.ll, false, s) != cudaSuccess) return GL_ERR_CUDA;
+      }
+      if (launch_dice(a, s) != cudaSuccess || launch_plain_iteration(a, pg, s) != cudaSuccess) return GL_ERR_CUDA;
+      left -= k + 1;
+    }
+  }
   if (cudaMemcpyAsync(&h_status, a.status, sizeof(Status), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return GL_ERR_CUDA;

@@ -380,13 +380,14 @@ int gl_server_destroy(gl_server* server);
 
 /* No counterpart in the reference.  For callers that may not call cudaMalloc (a
  * framework memory pool owns the device, or allocation would stall shared work):
- * runs `iters` LL iterations (the plain form, bit-identical products to a
- * GL_MODE_PLAIN plan) on the current device and `stream` (NULL = default stream),
+ * runs `iters` LL iterations (products bit-identical to a GL_MODE_PLAIN plan's) on the
+ * current device and `stream` (NULL = default stream),
  * from the products ll_in to the products ll_out (N int64 each, device memory owned
  * by the caller, natural word order; they may be the same buffer, but buffers that
- * overlap only in part return GL_ERR_ARG), and stores the maximum round-off in
+ * overlap only in part return GL_ERR_ARG), and stores the maximum round-off of its
+ * floating-point iterations (all, or one in 64 and the call's last; see gl_iterate) in
  * *max_roundoff.  It allocates nothing: its work arrays, tables and status word live in
- * a static device array sized for N <= 65536 (about 3.3 MiB, held on every GPU that
+ * a static device array sized for N <= 65536 (about 5.9 MiB, held on every GPU that
  * loads the library until exit); larger N returns GL_ERR_TOO_LARGE.  A call with new
  * (p, N) uploads that test's tables into the array first.  The call is synchronous: it
  * returns after `stream` has finished the iterations, so it cannot be captured into a

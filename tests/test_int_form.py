@@ -181,3 +181,20 @@ def test_polynomial_transforms_equal_fp64_form(gl, p, N):
         a, ra, _ = _products(gl, p, N, k)
         b, rb, _ = _products(gl, p, N, k, error_limit=0.39)
         assert ra.status == rb.status == 0 and (a == b).all(), k
+
+
+# layouts chosen without timing (radix-4 stages, a thread per two points) and the
+# no-allocation entry on the same lengths: one block of integer iterations, several, none
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,N", [(100003, 5120), (300007, 16200), (859433, 49152), (1000003, 54432), (1257787, 65536)])
+def test_untimed_layouts_and_noalloc_equal_fp64_form(gl, p, N):
+    import torch
+    start = np.zeros(N, np.int64)
+    start[0] = 4
+    for k in (1, 2, 66, 130):
+        want, _, _ = _products(gl, p, N, k, error_limit=0.39)
+        got, _, _ = _products(gl, p, N, k, autotune=0)
+        assert (got == want).all(), k
+        d = torch.from_numpy(start).cuda()
+        err = gl.iterate_noalloc(p, N, d.data_ptr(), d.data_ptr(), k, torch.cuda.current_stream().cuda_stream)
+        assert (d.cpu().numpy() == want).all() and 0.0 <= err < 0.4, k
