@@ -408,12 +408,15 @@ bool int_range_ok(int p, int N, int* vmax) {
 }
 
 // The integer form has no round-off to watch, so it is used where the FP64 form's stays
-// well below the default limit: up to 0.3 bits per word over gl_safe_signal_size's line
-// (measured round-off <= 0.125 on the line; it doubles every 0.5 bits, so <= 0.19 here) and
-// with a limit that is not tightened.  Elsewhere every iteration measures its round-off.
-constexpr double kIntBitsOverSafe = 0.3;
+// below the default limit and with a limit that is not tightened; elsewhere every iteration
+// measures its round-off.  The line is gl_safe_signal_size's (round-off <= 0.125) plus 0.3
+// bits per word: the round-off doubles every 0.45 bits or so, so <= 0.2 there.  At the
+// resident lengths the line is known better, from 60000 iterations each: plus 0.9 up to
+// N = 2048 (0.34 at 2048 and 21.73 bits, 0.31 at 1024 and 21.98), plus 0.75 up to 4096
+// (0.28 at 4096 and 21.29 bits, plus 0.72; 0.22 at 3072 and 21.30, plus 0.61).
 bool int_roundoff_ok(int p, int N, double error_limit) {
-  return error_limit >= 0.4 && (double)p / N <= 19.2 + kIntBitsOverSafe - 0.26 * std::log2(N / 163840.0);
+  const double over = N <= 2048 ? 0.9 : N <= kResidentAutoN ? 0.75 : 0.3;
+  return error_limit >= 0.4 && (double)p / N <= 19.2 + over - 0.26 * std::log2(N / 163840.0);
 }
 
 // Device time of one fused iteration with column length H, measured on zero-filled
@@ -705,10 +708,19 @@ int enqueue(gl_plan* pl, int64_t k) {
     if ((rc = launch_iterations(pl, 1)) != GL_OK) return rc;
     --k;
   }
-  if (pl->resident) {  // one cluster launch runs them all
+  if (pl->resident) {  // one cluster launch runs them all, or all up to the next FP64 one
     while (k > 0) {
-      const int chunk = (int)std::min<int64_t>(k, 1 << 30);
+      const int left = kFp64Every - 1 - pl->since_fp64;
+      if (pl->int_form && left > 0) {
+        const int chunk = (int)std::min<int64_t>(k, left);
+        GL_CUDA(launch_int_resident(pl->args, pl->irg, chunk, pl->stream));
+        pl->since_fp64 += chunk;
+        k -= chunk;
+        continue;
+      }
+      const int chunk = pl->int_form ? 1 : (int)std::min<int64_t>(k, 1 << 30);
       GL_CUDA(launch_resident(pl->args, pl->rg, chunk, pl->stream));
+      pl->since_fp64 = 0;
       k -= chunk;
     }
     return GL_OK;
@@ -943,18 +955,45 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   // a layout with W divisible by the cluster size fits; it replaces the layout search.
   bool resident = false;
   ResidentGeom rg{};
+  int vmax = 0;
+  // The integer form, unless an option names a variant of the FP64 kernels.
+  bool int_form = o.mode == GL_MODE_FUSED && !fp64_only && !sms_override && !names_fp64_variant(o) &&
+                  int_range_ok(p, N, &vmax) && int_roundoff_ok(p, N, o.error_limit);
+  IntGeom ig{};
+  IntVariant int_var;
+  IntResidentGeom irg{};
   if (o.mode == GL_MODE_FUSED && !sms_override && !force_h &&
       (o.resident > 0 ? N <= kResidentMaxN : (o.resident == 0 && N <= kResidentAutoN))) {
     // radix 4: each CTA's lines are short, and more, shorter butterflies keep more warps
     // issuing FP64 work (measured: 13.8 us at N = 2048 against 16.6 us with radix 8)
     const int rcap = o.max_radix_col ? o.max_radix_col : 4, wcap = o.max_radix_row ? o.max_radix_row : 4;
-    for (const auto& c : ranked_layouts(M, sms)) {
+    IntVariant var;
+    var.rc = var.rr = 8;
+    // a layout both forms can run; failing that, any for FP64 alone
+    bool int_resident = int_form;
+    auto ranked = ranked_layouts(M, sms);
+    if (int_form) {
+      const auto all = ranked;
+      ranked.insert(ranked.end(), all.begin(), all.end());
+    }
+    size_t tried = 0;
+    const size_t first_round = int_form ? ranked.size() / 2 : 0;
+    for (const auto& c : ranked) {
+      int_resident = int_form && tried++ < first_round;
       FusedGeom t{};
       if (choose_fused_geom(M, c.second, sms, &t, rcap, wcap) != GL_OK) continue;
+      if (int_resident) {
+        if (!choose_int_geom(t.H, t.W, &ig, var)) continue;
+        LinePlan pw = ig.pw, ph = ig.ph;
+        const int hn = int_stage_offsets(&ph), wn = int_stage_offsets(&pw);
+        if (int_resident_geom(t.H, t.W, ig, hn, wn, n, &irg) != cudaSuccess) continue;
+      }
       int offh[8], offw[8];
       const int nh = stage_offsets(t.ph, offh), nw = stage_offsets(t.pw, offw);
       if (resident_geom(t, nh, nw, n, &rg) == cudaSuccess) {
         resident = true;
+        int_form = int_resident;
+        int_var = var;
         force_h = c.second;
         cap_c = rcap;
         cap_r = wcap;
@@ -964,13 +1003,7 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
     cudaGetLastError();
   }
   if (o.resident > 0 && !resident) return GL_ERR_SIZE;
-  // The integer form, unless an option names a variant of the FP64 kernels.
-  IntGeom ig{};
-  int vmax = 0;
-  IntVariant int_var;
-  bool int_form = o.mode == GL_MODE_FUSED && !resident && !fp64_only && !sms_override && !names_fp64_variant(o) &&
-                  int_range_ok(p, N, &vmax) && int_roundoff_ok(p, N, o.error_limit);
-  if (int_form) {
+  if (int_form && !resident) {
     IntTuned it;
     if (o.autotune && !sms_override) it = autotune_int_layout(M, n, sms, 0);
     else {
@@ -1018,7 +1051,7 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   pl->p = p; pl->N = N; pl->M = M; pl->LO = p / N; pl->n = n;
   pl->mode = o.mode; pl->device = o.device;
   pl->error_limit = o.error_limit; pl->check_every = o.check_every; pl->use_graphs = o.use_graphs;
-  pl->fg = fg; pl->pg = pg; pl->ig = ig;
+  pl->fg = fg; pl->pg = pg; pl->ig = ig; pl->irg = irg;
 
 #define GL_TRY(x)             \
   do {                        \

@@ -7,6 +7,62 @@
 
 namespace gl {
 
+// The words j0, j0+1 from the products P[k] of the words j0+1-k, k = 0 .. NC+2, and the
+// flags of the words j0-1, j0, j0+1: their digits plus the carry of the word below.
+template <int NC>
+__device__ __forceinline__ void dice_pair(const long long* P, int LO, uint32_t fm, uint32_t f0, uint32_t f1, int* v0,
+                                          int* v1) {
+  int dm, hm, d0, h0, d1, h1;
+  if (NC <= 3) {
+    // words of 16 bits or more: in 32-bit arithmetic, from sign and magnitude of each
+    // product taken once
+    uint32_t lo[NC + 3], hi[NC + 3], sg[NC + 3];
+#pragma unroll
+    for (int k = 0; k < NC + 3; ++k) {
+      const unsigned long long g = (unsigned long long)(P[k] >> 63);
+      const unsigned long long m = ((unsigned long long)P[k] ^ g) - g;
+      lo[k] = (uint32_t)m;
+      hi[k] = (uint32_t)(m >> 32);
+      sg[k] = (uint32_t)g;
+    }
+    auto dice_at = [&](uint32_t f, int off) {
+      const uint32_t mask = (1u << (LO + (int)(f & 1))) - 1;
+      uint32_t sum = ((lo[off] & mask) ^ sg[off]) - sg[off];
+      int shift = 0;
+#pragma unroll
+      for (int i = 1; i <= NC; ++i) {
+        shift += LO + (int)((f >> i) & 1);
+        const int k = off + i;  // shift < 32 for i = 1, >= 32 beyond
+        const uint32_t w = (i == 1 ? __funnelshift_r(lo[k], hi[k], shift) : hi[k] >> (shift - 32)) & mask;
+        sum += (w ^ sg[k]) - sg[k];
+      }
+      return (int)sum;
+    };
+    balanced_split32(dice_at(fm, 2), LO + (int)(fm & 1), &dm, &hm);
+    balanced_split32(dice_at(f0, 1), LO + (int)(f0 & 1), &d0, &h0);
+    balanced_split32(dice_at(f1, 0), LO + (int)(f1 & 1), &d1, &h1);
+  } else {
+    auto dice_at = [&](uint32_t f, int off) {
+      const long long mask = (1ll << (LO + (int)(f & 1))) - 1;
+      const long long v = P[off];
+      long long sum = v < 0 ? -((-v) & mask) : (v & mask);
+      int shift = 0;
+#pragma unroll
+      for (int i = 1; i <= NC; ++i) {
+        shift += LO + (int)((f >> i) & 1);
+        const long long w = P[off + i];
+        sum += shift >= 63 ? 0 : (w < 0 ? -(((-w) >> shift) & mask) : ((w >> shift) & mask));
+      }
+      return sum;
+    };
+    balanced_split(dice_at(fm, 2), LO + (int)(fm & 1), &dm, &hm);
+    balanced_split(dice_at(f0, 1), LO + (int)(f0 & 1), &d0, &h0);
+    balanced_split(dice_at(f1, 0), LO + (int)(f1 & 1), &d1, &h1);
+  }
+  *v0 = d0 + hm;
+  *v1 = d1 + h0;
+}
+
 // Words j0 = 2m, j0+1 of point m = m1 + W m2 as (v0, v1): from the carry-save state, or by
 // dicing the products with carry depth NC (llintToIrrBal<n>).  The digit sums of j0-1, j0,
 // j0+1 need the products of words j0-1-NC .. j0+1: P[k] = product of word j0+1-k,
@@ -47,55 +103,7 @@ __device__ __forceinline__ void load_point(const IterArgs& a, const int m1, cons
     }
     const uchar2 ff = __ldg(reinterpret_cast<const uchar2*>(a.flags + s0));
     const uint32_t f0 = ff.x, f1 = ff.y;
-    int dm, hm, d0, h0, d1, h1;
-    if (NC <= 3) {
-      // words of 16 bits or more: in 32-bit arithmetic, from sign and magnitude of each
-      // product taken once
-      uint32_t lo[NC + 3], hi[NC + 3], sg[NC + 3];
-#pragma unroll
-      for (int k = 0; k < NC + 3; ++k) {
-        const unsigned long long g = (unsigned long long)(P[k] >> 63);
-        const unsigned long long m = ((unsigned long long)P[k] ^ g) - g;
-        lo[k] = (uint32_t)m;
-        hi[k] = (uint32_t)(m >> 32);
-        sg[k] = (uint32_t)g;
-      }
-      auto dice_at = [&](uint32_t f, int off) {
-        const uint32_t mask = (1u << (LO + (int)(f & 1))) - 1;
-        uint32_t sum = ((lo[off] & mask) ^ sg[off]) - sg[off];
-        int shift = 0;
-#pragma unroll
-        for (int i = 1; i <= NC; ++i) {
-          shift += LO + (int)((f >> i) & 1);
-          const int k = off + i;  // shift < 32 for i = 1, >= 32 beyond
-          const uint32_t w = (i == 1 ? __funnelshift_r(lo[k], hi[k], shift) : hi[k] >> (shift - 32)) & mask;
-          sum += (w ^ sg[k]) - sg[k];
-        }
-        return (int)sum;
-      };
-      balanced_split32(dice_at(fm, 2), LO + (int)(fm & 1), &dm, &hm);
-      balanced_split32(dice_at(f0, 1), LO + (int)(f0 & 1), &d0, &h0);
-      balanced_split32(dice_at(f1, 0), LO + (int)(f1 & 1), &d1, &h1);
-    } else {
-      auto dice_at = [&](uint32_t f, int off) {
-        const long long mask = (1ll << (LO + (int)(f & 1))) - 1;
-        const long long v = P[off];
-        long long sum = v < 0 ? -((-v) & mask) : (v & mask);
-        int shift = 0;
-#pragma unroll
-        for (int i = 1; i <= NC; ++i) {
-          shift += LO + (int)((f >> i) & 1);
-          const long long w = P[off + i];
-          sum += shift >= 63 ? 0 : (w < 0 ? -(((-w) >> shift) & mask) : ((w >> shift) & mask));
-        }
-        return sum;
-      };
-      balanced_split(dice_at(fm, 2), LO + (int)(fm & 1), &dm, &hm);
-      balanced_split(dice_at(f0, 1), LO + (int)(f0 & 1), &d0, &h0);
-      balanced_split(dice_at(f1, 0), LO + (int)(f1 & 1), &d1, &h1);
-    }
-    *v0 = d0 + hm;
-    *v1 = d1 + h0;
+    dice_pair<NC>(P, LO, fm, f0, f1, v0, v1);
   }
 }
 

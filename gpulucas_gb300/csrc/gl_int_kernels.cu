@@ -16,15 +16,11 @@
 //  * roots of odd order are scalars of GF(q), not of norm 1, so the inverse transform has
 //    its own tables.
 #include "gl_dice.cuh"
-#include "gl_gf61.cuh"
+#include "gl_int_stage.cuh"
 #include "gl_internal.h"
 
 namespace gl {
 namespace {
-
-using gf::g2;
-
-__device__ __forceinline__ int ipad(int i) { return i + (i >> 3); }
 
 __device__ __forceinline__ g2 ldz(const DevCplx* p) {
   const longlong2 v = *reinterpret_cast<const longlong2*>(p);
@@ -45,34 +41,6 @@ __device__ __forceinline__ void touch(const int4* p, int n) {
 __device__ __forceinline__ int plan_slots(const LinePlan& lp) {  // entries of its stage table
   const int s = lp.nst - 1, R = lp.radix[s];
   return lp.off[s] + (s ? (R - 1) * (lp.L / R) : 0);
-}
-
-// Stockham DIT stage, out of place, as in the FP64 form: butterfly j of a line reads
-// x[j + q L/R], multiplies by w^q and writes x[(j - k) R + k + p Ns], k = j mod Ns.
-// The position k needs no division in the first stages (Ns a power of two) or the last
-// (Ns = L/R > j).
-template <int R, int S>
-__device__ __forceinline__ void int_stage(const g2* __restrict__ src, g2* __restrict__ dst, int nlines, int ls,
-                                          int L, int Ns, const int4* __restrict__ tw) {
-  const int LR = L / R;
-  const int nb = nlines * LR;
-  const bool last = Ns == LR, pow2 = (Ns & (Ns - 1)) == 0;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    int l = 0;
-    if (nlines == 2) l = b >= LR;
-    else if (nlines > 2) l = b / LR;
-    const int j = b - l * LR;
-    const int k = last ? j : pow2 ? (j & (Ns - 1)) : j % Ns;
-    const g2* s = src + l * ls;
-    g2 v[R];
-    gf::butterfly<R, S>(
-        v, Ns > 1, [&](int q) { return s[ipad(j + q * LR)]; }, [&](int i) { return __ldg(tw + (k + i * Ns)); });
-    g2* d = dst + l * ls;
-    const int base = (j - k) * R + k;
-#pragma unroll
-    for (int q = 0; q < R; ++q) d[ipad(base + q * Ns)] = v[q];
-  }
-  __syncthreads();
 }
 
 // In-place stage: every thread first reads the inputs of all its butterflies (at most P
@@ -135,33 +103,6 @@ __device__ __forceinline__ void int_line_fft_ip(g2* a, const LinePlan& lp, const
     }
     Ns *= lp.radix[s];
   }
-}
-
-// B57: the plan may have radices 5 and 7 (compiled apart: a kernel's registers are set by
-// its largest stage, and without them three CTAs of 256 threads fit an SM).
-template <int S, bool B57>
-__device__ __forceinline__ g2* int_line_fft(g2* a, g2* b, int nlines, int ls, const LinePlan& lp, const int4* tw) {
-  int Ns = 1;
-  for (int s = 0; s < lp.nst; ++s) {
-    const int4* st = tw + lp.off[s];
-    switch (lp.radix[s]) {
-      case 8: int_stage<8, S>(a, b, nlines, ls, lp.L, Ns, st); break;
-      case 4: int_stage<4, S>(a, b, nlines, ls, lp.L, Ns, st); break;
-      case 2: int_stage<2, S>(a, b, nlines, ls, lp.L, Ns, st); break;
-      case 3: int_stage<3, S>(a, b, nlines, ls, lp.L, Ns, st); break;
-      default:
-        if constexpr (B57) {
-          if (lp.radix[s] == 5) int_stage<5, S>(a, b, nlines, ls, lp.L, Ns, st);
-          else int_stage<7, S>(a, b, nlines, ls, lp.L, Ns, st);
-        }
-        break;
-    }
-    Ns *= lp.radix[s];
-    g2* t = a;
-    a = b;
-    b = t;
-  }
-  return a;
 }
 
 // Forward column pass: dice, add carries, weight, length-H DFT, twiddle, store to row k2 of Z.
@@ -348,17 +289,6 @@ __global__ void __launch_bounds__(T, MB) ki_row_sq(IterArgs a) {
   int_row_body<B57>(a, blockIdx.x);
 }
 
-// the product's range checks, as round_word of the FP64 form
-__device__ __forceinline__ long long check_word(long long r, int span, unsigned* fl) {
-  const unsigned long long mag = (unsigned long long)(r < 0 ? -r : r);
-  if (mag >> 51) {
-    *fl |= kStatusBig;
-    return 0;
-  }
-  if (span < 63 && (mag >> span) != 0ull) *fl |= kStatusSlice;
-  return r;
-}
-
 // The two products of one point: unweight, check, -2 at word 0 (the LL step), store.
 __device__ __forceinline__ void int_store_products(const IterArgs& a, g2 v, int s0, unsigned* fl) {
   const uchar2 e = __ldg(reinterpret_cast<const uchar2*>(a.in.e + s0));
@@ -389,12 +319,6 @@ __device__ __forceinline__ void int_col_inv_body(const IterArgs& a, const int m1
 template <bool B57, int P>
 __global__ void __launch_bounds__(kMaxThreads, B57 ? 2 : P ? 4 : 3) ki_col_inv(IterArgs a) {
   int_col_inv_body<B57, P>(a, blockIdx.x);
-}
-
-bool has57(const LinePlan& lp) {
-  for (int i = 0; i < lp.nst; ++i)
-    if (lp.radix[i] == 5 || lp.radix[i] == 7) return true;
-  return false;
 }
 
 template <bool FS, bool B57, int P>

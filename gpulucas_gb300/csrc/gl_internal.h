@@ -159,6 +159,17 @@ constexpr int kResidentMaxN = 32768;   // largest N the resident form is tried a
 constexpr int kResidentAutoN = 4096;   // used by default up to here: measured faster than the
                                        // three-launch form (13.8 vs 18.3 us at N = 2048, 16.1 vs
                                        // 19.6 us at 4096; slower from 8192 on)
+// The resident form in integer arithmetic (gl_int_resident.cu), on the same layout; regions as
+// in ResidentGeom, with weight exponents (ex) for the weights and stage tables of both
+// directions (hn and wn entries each).
+struct IntResidentGeom {
+  int C, cw, hn, wn, smem;
+  int o_zc, o_zc2, o_zr, o_zr2, o_ll, o_ex, o_fl, o_sp, o_K1, o_pr, o_K2, o_hf, o_hi, o_wf, o_wi;
+};
+constexpr int kIntResidentThreads = 256;
+constexpr int kIntResidentSmem = 160 * 1024;
+cudaError_t int_resident_geom(int H, int W, const IntGeom& g, int hn, int wn, int n, IntResidentGeom* r);
+cudaError_t launch_int_resident(const IterArgs& a, const IntResidentGeom& r, int iters, cudaStream_t s);
 // smallest cluster first; fills r and returns cudaSuccess if the layout fits one cluster
 cudaError_t resident_geom(const FusedGeom& g, int twH_n, int twW_n, int n, ResidentGeom* r);
 cudaError_t launch_resident(const IterArgs& a, const ResidentGeom& r, int iters, cudaStream_t s);

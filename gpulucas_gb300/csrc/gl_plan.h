@@ -45,6 +45,7 @@ struct gl_plan {
   size_t device_bytes = 0;
   bool resident = false;        // short length: whole check intervals in one cluster
   ResidentGeom rg{};
+  gl::IntResidentGeom irg{};    // with int_form: the resident form in integer arithmetic
   uint8_t* rscratch = nullptr;  // device scratch of the residue kernels
   int32_t* h_res = nullptr;     // pinned: 64 canonical head digits, scalars, flags
 };

@@ -198,3 +198,22 @@ def test_untimed_layouts_and_noalloc_equal_fp64_form(gl, p, N):
         d = torch.from_numpy(start).cuda()
         err = gl.iterate_noalloc(p, N, d.data_ptr(), d.data_ptr(), k, torch.cuda.current_stream().cuda_stream)
         assert (d.cpu().numpy() == want).all() and 0.0 <= err < 0.4, k
+
+
+# the resident integer form: one and several launches between FP64 iterations, odd parts in
+# the rows, the largest word size it runs at, and lengths whose layout leaves it to FP64
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,N", [(9689, 512), (21701, 1024), (33013, 1536), (44497, 2048), (60013, 3072), (86243, 4096),
+                                 (21023, 1120), (12379, 640), (76003, 3840)])
+def test_resident_integer_form_follows_the_oracle(gl, orc, p, N):
+    o = orc.IBDWT(p, N)
+    with gl.Plan(p, N) as pl:
+        assert pl.info.resident_ctas in (8, 16)
+        for k in (1, 2, 60, 3, 130):
+            rep = pl.iterate(k)
+            o.iterate(k)
+            assert rep.status == 0 and (pl.products() == o.ll()).all(), k
+        d, h = pl.carry_state()
+        pl.set_carry_state(d, h, 0)
+        pl.iterate(5)
+        assert (pl.products() == o.iterate(5).ll()).all()
