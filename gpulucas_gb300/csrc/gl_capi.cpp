@@ -917,6 +917,7 @@ static int build_int_tables(gl_plan* pl, int vmax) {
   GL_CUDA(cudaStreamSynchronize(pl->stream));  // host tables go out of scope
   gl_int_args(H, W, pl->ig, (int)rows.size(), &in);
   in.vmax = vmax;
+  in.check_span = (pl->n + 1) * pl->LO < 51;
   GL_CUDA(set_int_smem_limits());
   pl->int_form = true;
   return GL_OK;

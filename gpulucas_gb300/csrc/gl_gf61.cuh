@@ -69,7 +69,7 @@ GL_HD uint64_t pack(uint32_t l, uint32_t h) { return ((uint64_t)h << 32) | l; }
 GL_HD uint32_t funnel(uint32_t l, uint32_t h, int s) { return (uint32_t)((((uint64_t)h << 32) | l) >> s); }
 #endif
 
-// x reduced to [-2^60, 2^60 + 3], |x| < 2^63 - 2^60
+// x reduced to [-2^60 - 4, 2^60 + 3], |x| < 2^63 - 2^60
 GL_HD int64_t red(int64_t x) {
   const int hi = (int)hi32((uint64_t)x);
   const int h = (hi + (1 << 28)) >> 29;  // x = h 2^61 + a balanced remainder
@@ -431,21 +431,17 @@ GL_HD g2 poly_square(const Get& get, int t, int b, int4 z) {
 }
 constexpr Limbs kMinusQuarter = limbs(kQ - (1ull << 59));
 
-// v 2^e within R, 0 <= e <= 60, |v| < 2^31
+// v 2^e within R, 0 <= e <= 60: v 2^e = (v >> (61 - e)) 2^61 + the low 61 bits
 GL_HD int64_t weighted(int v, int e) {
-  const uint64_t x = (uint64_t)(int64_t)v << e;
-  const int hi = (int)(hi32(x) << 3) >> 3;  // bits 0..60, sign-extended
-  const int64_t k = ((int64_t)v + ((int64_t)1 << (60 - e))) >> (61 - e);
-  return (int64_t)pack(lo32(x), (uint32_t)hi) + k;
+  const uint64_t x = ((uint64_t)(int64_t)v << e) & kQ;
+  const int s = 61 - e;
+  return red((int64_t)mad_s(v >> (s < 31 ? s : 31), 1, x));
 }
 
-// the integer congruent to x 2^-e in (-2^60, 2^60], x within 3R, 0 <= e <= 60
+// The integer congruent to x 2^-e in [-2^60 - 4, 2^60 + 3], x within 3R, 0 <= e <= 60.  A
+// product below 2^59 in magnitude is that integer itself.
 GL_HD int64_t unweighted(int64_t x, int e) {
-  const uint64_t y = (uint64_t)x + kAccLo;
-  const uint64_t u1 = (y & kQ) + (y >> 61);
-  const uint64_t u = (u1 & kQ) + (u1 >> 61);
-  const uint64_t r = ((u >> e) | (u << (61 - e))) & kQ;
-  return (int64_t)r - (r > (1ull << 60) ? (int64_t)kQ : 0);
+  return red((int64_t)(((uint64_t)x << (61 - e)) & kQ) + (x >> e));
 }
 
 }  // namespace gf

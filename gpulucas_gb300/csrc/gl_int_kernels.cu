@@ -38,6 +38,11 @@ __device__ __forceinline__ void touch(const int4* p, int n) {
     asm volatile("{\n .reg .s32 d;\n ld.global.nc.s32 d, [%0];\n}" ::"l"(p + i));
   }
 }
+// Starts bringing n table entries into L2 (one thread): with many CTAs the tables of the end
+// of a pass come from DRAM, and every CTA of a wave asks for them at the same time.
+__device__ __forceinline__ void prefetch_l2(const int4* p, int n) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(n * 16));
+}
 __device__ __forceinline__ int plan_slots(const LinePlan& lp) {  // entries of its stage table
   const int s = lp.nst - 1, R = lp.radix[s];
   return lp.off[s] + (s ? (R - 1) * (lp.L / R) : 0);
@@ -114,6 +119,7 @@ __device__ __forceinline__ void int_col_fwd_body(const IterArgs& a, const int m1
     touch(a.in.hf, plan_slots(a.in.ph));
     touch(a.in.k1 + m1 * H, H);
   }
+  if (P && threadIdx.x == 0) prefetch_l2(a.in.k1 + m1 * H, H);
   bool wide = false;
 #pragma unroll (P == 0 ? 2 : 1)
   for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) {
@@ -128,7 +134,7 @@ __device__ __forceinline__ void int_col_fwd_body(const IterArgs& a, const int m1
   const g2* res = ism;
   if constexpr (P > 0) int_line_fft_ip<-1, B57, P>(ism, a.in.ph, a.in.hf);
   else res = int_line_fft<-1, B57>(ism, ism + ls, 1, ls, a.in.ph, a.in.hf);
-#pragma unroll 1
+#pragma unroll 2
   for (int k2 = threadIdx.x; k2 < H; k2 += blockDim.x)
     stz(a.Z + (k2 * W + m1), gf::cmul(res[ipad(k2)], __ldg(a.in.k1 + (m1 * H + k2))));
 }
@@ -162,6 +168,8 @@ __device__ __forceinline__ void int_row_body(const IterArgs& a, const int pair) 
       touch(a.in.wi, plan_slots(a.in.pw));
       touch(a.in.k2 + r.x * W, W);
       touch(a.in.k2 + r.y * W, W);
+    } else if (threadIdx.x < 3) {
+      prefetch_l2(threadIdx.x == 0 ? a.in.pair + r.x * W : a.in.k2 + (threadIdx.x == 1 ? r.x : r.y) * W, W);
     }
     for (int idx = threadIdx.x; idx < nl * W; idx += blockDim.x) {
       const int l = idx >= W;
@@ -292,9 +300,13 @@ __global__ void __launch_bounds__(T, MB) ki_row_sq(IterArgs a) {
 // The two products of one point: unweight, check, -2 at word 0 (the LL step), store.
 __device__ __forceinline__ void int_store_products(const IterArgs& a, g2 v, int s0, unsigned* fl) {
   const uchar2 e = __ldg(reinterpret_cast<const uchar2*>(a.in.e + s0));
-  const uchar2 sp = __ldg(reinterpret_cast<const uchar2*>(a.span + s0));
-  long long r0 = check_word(gf::unweighted(v.re, e.x), sp.x, fl);
-  const long long r1 = check_word(gf::unweighted(v.im, e.y), sp.y, fl);
+  long long r0 = check_word(gf::unweighted(v.re, e.x), fl);
+  const long long r1 = check_word(gf::unweighted(v.im, e.y), fl);
+  if (a.in.check_span) {
+    const uchar2 sp = __ldg(reinterpret_cast<const uchar2*>(a.span + s0));
+    check_span(r0, sp.x, fl);
+    check_span(r1, sp.y, fl);
+  }
   if (s0 == 0) r0 -= 2;
   *reinterpret_cast<longlong2*>(a.ll + s0) = make_longlong2(r0, r1);
 }

@@ -163,8 +163,12 @@ __global__ void __launch_bounds__(kIntResidentThreads, 1) ki_resident(const __gr
         const int lc = idx / H, m2 = idx - lc * H;
         const int s0 = 2 * idx;
         const g2 v = res[lc * lsc + ipad(m2)];
-        long long r0 = check_word(gf::unweighted(v.re, ex[s0]), sp[s0], &flg);
-        const long long r1 = check_word(gf::unweighted(v.im, ex[s0 + 1]), sp[s0 + 1], &flg);
+        long long r0 = check_word(gf::unweighted(v.re, ex[s0]), &flg);
+        const long long r1 = check_word(gf::unweighted(v.im, ex[s0 + 1]), &flg);
+        if (a.in.check_span) {
+          check_span(r0, sp[s0], &flg);
+          check_span(r1, sp[s0 + 1], &flg);
+        }
         if (rank == 0 && idx == 0) r0 -= 2;  // word 0
         ll[s0] = r0;
         ll[s0 + 1] = r1;

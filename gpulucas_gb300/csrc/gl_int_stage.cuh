@@ -78,15 +78,19 @@ __device__ __forceinline__ g2* int_line_fft(g2* a, g2* b, int nlines, int ls, co
   return a;
 }
 
-// the product's range checks, as round_word of the FP64 form
-__device__ __forceinline__ long long check_word(long long r, int span, unsigned* fl) {
+// The product's range checks, as round_word of the FP64 form.  Where n + 1 words always
+// hold 51 bits (all but words of a few bits), the first check implies the second.
+__device__ __forceinline__ long long check_word(long long r, unsigned* fl) {
   const unsigned long long mag = (unsigned long long)(r < 0 ? -r : r);
   if (mag >> 51) {
     *fl |= kStatusBig;
     return 0;
   }
-  if (span < 63 && (mag >> span) != 0ull) *fl |= kStatusSlice;
   return r;
+}
+__device__ __forceinline__ void check_span(long long r, int span, unsigned* fl) {
+  const unsigned long long mag = (unsigned long long)(r < 0 ? -r : r);
+  if (span < 63 && (mag >> span) != 0ull) *fl |= kStatusSlice;
 }
 
 }  // namespace gl

@@ -108,6 +108,7 @@ struct IntArgs {
   int t, V;                   // W = t V; the transform has length L = V H (gf_excess)
   int qV;                     // 2^61 - 1 mod V
   int vmax;                   // bound on a loaded word's magnitude
+  int check_span;             // n + 1 words may hold less than 51 bits
   int touch;                  // few CTAs: bring a pass's tables into L1 at its start
   int ls_col, ls_row;
   LinePlan pw, ph;

@@ -44,13 +44,16 @@ def test_field_operations_at_their_bounds(hc):
         assert abs(re) <= R and abs(im) <= R
         y = int(rng.integers(-(1 << 63) + (1 << 60) + 1, (1 << 63) - (1 << 60) - 1))
         r = hc.hc_gf_red(y)
-        assert (r - y) % Q == 0 and -(1 << 60) <= r <= (1 << 60) + 3
+        assert (r - y) % Q == 0 and -(1 << 60) - 4 <= r <= (1 << 60) + 3
         e = int(rng.integers(61))
         v = int(rng.integers(-(1 << 28), 1 << 28))
         g = hc.hc_gf_weighted(v, e)
         assert (g - v * pow(2, e, Q)) % Q == 0 and abs(g) <= R
         u = hc.hc_gf_unweighted(x[0] - x[0] // 4, e)  # within 3 R
-        assert (u * pow(2, e, Q) - (x[0] - x[0] // 4)) % Q == 0 and -(1 << 60) < u <= 1 << 60
+        assert (u * pow(2, e, Q) - (x[0] - x[0] // 4)) % Q == 0 and -(1 << 60) - 4 <= u <= (1 << 60) + 3
+        n = int(rng.integers(-(1 << 59), 1 << 59))  # a product: any representative of it gives it back
+        z = n * pow(2, e, Q) % Q + (int(rng.integers(3)) - 1) * Q
+        assert hc.hc_gf_unweighted(z - Q if z > 3 * (1 << 60) else z, e) == n
 
 
 # layouts with every radix first and later, columns or rows with an odd part (rows that pair
