@@ -38,6 +38,17 @@ __device__ __forceinline__ void touch(const int4* p, int n) {
     asm volatile("{\n .reg .s32 d;\n ld.global.nc.s32 d, [%0];\n}" ::"l"(p + i));
   }
 }
+// With a.in.dependent every pass is launched as a programmatic dependent of the one before
+// it: it becomes resident while that one runs, touches its tables, and waits here for that
+// one's end.  Only then may the next pass become resident, so at most one waits at a time.
+// For iterations launched one by one (N = 65536 without allocation: 27.3 -> 20.6 us per
+// iteration); in a replayed graph it gains nothing (163840: 23.1 -> 24-26, 65536: 18.3 ->
+// 17.2, 5120: 14.6 -> 15.5), so plans do not use it.
+__device__ __forceinline__ void after_previous_pass() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Starts bringing n table entries into L2 (one thread): with many CTAs the tables of the end
 // of a pass come from DRAM, and every CTA of a wave asks for them at the same time.
 __device__ __forceinline__ void prefetch_l2(const int4* p, int n) {
@@ -119,6 +130,7 @@ __device__ __forceinline__ void int_col_fwd_body(const IterArgs& a, const int m1
     touch(a.in.hf, plan_slots(a.in.ph));
     touch(a.in.k1 + m1 * H, H);
   }
+  if (P == 0 && a.in.dependent) after_previous_pass();
   if (P && threadIdx.x == 0) prefetch_l2(a.in.k1 + m1 * H, H);
   bool wide = false;
 #pragma unroll (P == 0 ? 2 : 1)
@@ -168,6 +180,7 @@ __device__ __forceinline__ void int_row_body(const IterArgs& a, const int pair) 
       touch(a.in.wi, plan_slots(a.in.pw));
       touch(a.in.k2 + r.x * W, W);
       touch(a.in.k2 + r.y * W, W);
+      if (a.in.dependent) after_previous_pass();
     } else if (threadIdx.x < 3) {
       prefetch_l2(threadIdx.x == 0 ? a.in.pair + r.x * W : a.in.k2 + (threadIdx.x == 1 ? r.x : r.y) * W, W);
     }
@@ -230,6 +243,7 @@ __device__ __forceinline__ void int_row_poly_body(const IterArgs& a, const int p
     touch(a.in.wi, plan_slots(a.in.pw));
     touch(a.in.k2 + r.x * W, W);
     touch(a.in.k2 + r.y * W, W);
+    if (a.in.dependent) after_previous_pass();
   }
   g2* other = ism + 2 * t * ls;
   int4* dif = reinterpret_cast<int4*>(ism + 4 * t * ls);  // line b: D in limbs
@@ -316,7 +330,10 @@ template <bool B57, int P>
 __device__ __forceinline__ void int_col_inv_body(const IterArgs& a, const int m1) {
   extern __shared__ g2 ism[];
   const int H = a.H, ls = a.in.ls_col;
-  if (P == 0 && a.in.touch) touch(a.in.hi, plan_slots(a.in.ph));
+  if (P == 0 && a.in.touch) {
+    touch(a.in.hi, plan_slots(a.in.ph));
+    if (a.in.dependent) after_previous_pass();
+  }
   for (int k2 = threadIdx.x; k2 < H; k2 += blockDim.x) ism[ipad(k2)] = ldz(a.Z2 + (size_t)m1 * H + k2);
   __syncthreads();
   const g2* res = ism;
@@ -333,25 +350,32 @@ __global__ void __launch_bounds__(kMaxThreads, B57 ? 2 : P ? 4 : 3) ki_col_inv(I
   int_col_inv_body<B57, P>(a, blockIdx.x);
 }
 
+// One pass; as a programmatic dependent of the launch before it where the kernel waits for
+// that itself (after_previous_pass).
+void run(void (*kernel)(IterArgs), int grid, int block, size_t smem, cudaStream_t s, const IterArgs& a, bool dependent) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
 template <bool FS, bool B57, int P>
 void launch_col_fwd_p(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
-  switch (a.n) {
-    case 2: ki_col_fwd<FS, 2, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-    case 3: ki_col_fwd<FS, 3, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-    case 4: ki_col_fwd<FS, 4, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-    case 5: ki_col_fwd<FS, 5, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-    default: ki_col_fwd<FS, 6, B57, P><<<a.W, g.t_col, g.sm_col, s>>>(a); break;
-  }
+  void (*const kernels[5])(IterArgs) = {ki_col_fwd<FS, 2, B57, P>, ki_col_fwd<FS, 3, B57, P>, ki_col_fwd<FS, 4, B57, P>,
+                                        ki_col_fwd<FS, 5, B57, P>, ki_col_fwd<FS, 6, B57, P>};
+  run(kernels[a.n - 2], a.W, g.t_col, g.sm_col, s, a, P == 0 && a.in.dependent);
 }
 template <bool FS, bool B57>
 void launch_col_fwd(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
   if (!B57 && g.col_p) launch_col_fwd_p<FS, false, kIntHeld>(a, g, s);
   else launch_col_fwd_p<FS, B57, 0>(a, g, s);
-}
-template <bool B57>
-void launch_col_inv(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
-  if (!B57 && g.col_p) ki_col_inv<false, kIntHeld><<<a.W, g.t_col, g.sm_col, s>>>(a);
-  else ki_col_inv<B57, 0><<<a.W, g.t_col, g.sm_col, s>>>(a);
 }
 void launch_pass(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which, bool from_state) {
   const bool c57 = has57(g.ph), r57 = has57(g.pw);
@@ -359,13 +383,15 @@ void launch_pass(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which,
     if (from_state) c57 ? launch_col_fwd<true, true>(a, g, s) : launch_col_fwd<true, false>(a, g, s);
     else c57 ? launch_col_fwd<false, true>(a, g, s) : launch_col_fwd<false, false>(a, g, s);
   } else if (which == 1) {
-    if (g.t > 1) ki_row_poly<<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
-    else if (r57) ki_row_sq<true, 256, 2><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
-    else if (g.t_row <= 192 && a.in.nrows > kRowsFor5) ki_row_sq<false, 192, 5><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
-    else ki_row_sq<false, 256, 3><<<a.in.nrows, g.t_row, g.sm_row, s>>>(a);
+    void (*kernel)(IterArgs) = ki_row_sq<false, 256, 3>;
+    if (g.t > 1) kernel = ki_row_poly;
+    else if (r57) kernel = ki_row_sq<true, 256, 2>;
+    else if (g.t_row <= 192 && a.in.nrows > kRowsFor5) kernel = ki_row_sq<false, 192, 5>;
+    run(kernel, a.in.nrows, g.t_row, g.sm_row, s, a, a.in.dependent);
   } else {
-    if (c57) launch_col_inv<true>(a, g, s);
-    else launch_col_inv<false>(a, g, s);
+    const bool ip = !c57 && g.col_p;
+    run(ip ? ki_col_inv<false, kIntHeld> : c57 ? ki_col_inv<true, 0> : ki_col_inv<false, 0>, a.W, g.t_col, g.sm_col, s, a,
+        !ip && a.in.dependent);
   }
 }
 

@@ -110,6 +110,7 @@ struct IntArgs {
   int vmax;                   // bound on a loaded word's magnitude
   int check_span;             // n + 1 words may hold less than 51 bits
   int touch;                  // few CTAs: bring a pass's tables into L1 at its start
+  int dependent;              // with touch: passes are launched as programmatic dependents
   int ls_col, ls_row;
   LinePlan pw, ph;
 };
