@@ -1188,9 +1188,7 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
 #undef GL_TRYC
 }
 
-extern "C" {
-
-int gl_plan_describe(int p, int N, const gl_plan_opts* opts, gl_plan_info* info) {
+int gl_plan_describe_ex(int p, int N, const gl_plan_opts* opts, gl_plan_info* info, bool fp64_only) {
   if (!info) return GL_ERR_ARG;
   gl_plan_opts o;
   if (opts) o = *opts;
@@ -1210,7 +1208,7 @@ int gl_plan_describe(int p, int N, const gl_plan_opts* opts, gl_plan_info* info)
   int cap_c = kMaxRadix, cap_r = kMaxRadix;
   model_caps(tmp.M, o, o.batch_layout ? 1 : 0, &cap_c, &cap_r);
   int vmax = 0;
-  const bool int_form = o.mode == GL_MODE_FUSED && !o.batch_layout && !names_fp64_variant(o) && int_range_ok(p, N, &vmax) &&
+  const bool int_form = o.mode == GL_MODE_FUSED && !fp64_only && !o.batch_layout && !names_fp64_variant(o) && int_range_ok(p, N, &vmax) &&
                         int_roundoff_ok(p, N, o.error_limit);
   const int int_h = int_form ? first_int_layout(tmp.M, sms) : 0;
   int rc = o.mode == GL_MODE_FUSED ? choose_fused_geom(tmp.M, int_h ? int_h : o.fft_h, sms, &tmp.fg, cap_c, cap_r)
@@ -1229,6 +1227,12 @@ int gl_plan_describe(int p, int N, const gl_plan_opts* opts, gl_plan_info* info)
       info->device_bytes += int_table_bytes(tmp.fg.H, tmp.fg.W, ig);
   }
   return r;
+}
+
+extern "C" {
+
+int gl_plan_describe(int p, int N, const gl_plan_opts* opts, gl_plan_info* info) {
+  return gl_plan_describe_ex(p, N, opts, info, false);
 }
 
 int gl_plan_destroy(gl_plan* plan) {

@@ -56,6 +56,7 @@ struct gl_plan {
 // fp64_only: no integer form (round-off trials).
 int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, gl_plan** out,
                       bool fp64_only = false);
+int gl_plan_describe_ex(int p, int N, const gl_plan_opts* opts, gl_plan_info* info, bool fp64_only);
 // iterations done outside the plan's own launches (by a batch): bookkeeping only
 void gl_plan_note_external_iterations(gl_plan* pl, int64_t iters);
 // non-blocking stream; level 0: normal priority, 1: the device's highest, 2: between

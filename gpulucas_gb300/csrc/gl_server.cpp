@@ -66,14 +66,14 @@ int ge_signal_size(void*, int p, double bits, int above, int* N) {
 int ge_footprint(void* ctx, int p, int N, size_t* bytes) {
   gl_plan_opts o = engine_opts(static_cast<GpuEngine*>(ctx));
   gl_plan_info info;
-  const int rc = gl_plan_describe(p, N, &o, &info);
+  const int rc = gl_plan_describe_ex(p, N, &o, &info, true);
   if (rc == GL_OK) *bytes = info.device_bytes;
   return rc;
 }
 int ge_create(void* ctx, int p, int N, void** test) {
   gl_plan_opts o = engine_opts(static_cast<GpuEngine*>(ctx));
   gl_plan* pl = nullptr;
-  const int rc = gl_plan_create(p, N, &o, &pl);  // starts from S0 = 4
+  const int rc = gl_plan_create_ex(p, N, &o, 0, &pl, true);  // FP64 alone, as the batches run; starts from S0 = 4
   *test = pl;
   return rc;
 }

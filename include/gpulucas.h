@@ -99,7 +99,7 @@ typedef struct {
 typedef struct {
     int64_t iterations;    /* iterations done by this call */
     int64_t total_iterations; /* iterations since S0 = 4 */
-    double max_roundoff;   /* max |x - rint(x)| seen by this call (checked iterations) */
+    double max_roundoff;   /* max |x - rint(x)| over this call's floating-point iterations */
     double ms;             /* device time of the call, CUDA events */
     int status;            /* GL_OK, GL_ERR_ROUNDOFF or GL_ERR_OVERFLOW */
 } gl_iter_report;
@@ -139,7 +139,13 @@ int gl_reset(gl_plan* plan);
 
 /* Runs `iters` LL iterations: the loop body mersenneIter<check,0> (gpuLucas.cu:845-942)
  * with the round-off check of mersenneTest (gpuLucas.cu:1399-1410), aborting with
- * GL_ERR_ROUNDOFF at the plan's error limit. */
+ * GL_ERR_ROUNDOFF at the plan's error limit.
+ * Fused-form plans whose round-off stays well below the default limit (p/N up to 0.3 bits
+ * over gl_safe_signal_size's line, 0.75 to 0.9 up to N = 4096; error_limit >= 0.4; no option
+ * that names an FP64 kernel variant) run most iterations in exact integer arithmetic, which
+ * gives the same products and has no round-off; one iteration in 64 runs in FP64, and the
+ * reported round-off is over those (0 if a call held none).  Other plans, the round-off
+ * trials (gl_error_test, gl_find_signal_size) and batches run FP64 in every iteration. */
 int gl_iterate(gl_plan* plan, int64_t iters, gl_iter_report* report);
 
 /* Asynchronous forms for callers that time or overlap work themselves: enqueue

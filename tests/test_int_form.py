@@ -220,3 +220,15 @@ def test_resident_integer_form_follows_the_oracle(gl, orc, p, N):
         pl.set_carry_state(d, h, 0)
         pl.iterate(5)
         assert (pl.products() == o.iterate(5).ll()).all()
+
+
+# the smallest lengths and words of a few bits (where the slice check is not implied by the
+# size check), up to the largest carry depth
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,N", [(127, 16), (127, 64), (607, 40), (1279, 70), (3217, 180), (4423, 1000), (9941, 2250)])
+def test_smallest_lengths_and_words_equal_fp64_form(gl, orc, p, N):
+    for k in (1, 3, 66):
+        want, ra, _ = _products(gl, p, N, k, error_limit=0.39)
+        got, rb, _ = _products(gl, p, N, k)
+        assert ra.status == rb.status == 0 and (got == want).all(), k
+    assert (got == orc.IBDWT(p, N).iterate(66).ll()).all()
