@@ -43,13 +43,26 @@ def flop_alg(N: int) -> float:
     return 5.0 * N * math.log2(N) + 4.0 * N
 
 
-def kernel_flops(N: int, W: int, H: int) -> dict:
-    """flop_alg split over the three fused kernels (sums to flop_alg(N))."""
+# 32 x 32 -> 64-bit multiply-adds per clock and SM, measured from registers on a GB300 (a
+# warp instruction holds its sub-partition's pipe for 4.2 cycles), and the SM count
+MAD64_PER_CLOCK_SM = 30.3
+SMS = 152
+
+
+def kernel_mads(N: int, W: int, H: int, radix_w, radix_h) -> dict:
+    """32 x 32 -> 64-bit multiply-adds that the integer form's three passes cannot do without:
+    16 per twiddle product, 4 per product with a scalar of GF(q)."""
     M = N // 2
+
+    def line(radices):
+        per = sum((r - 1) / r for r in radices[1:]) * 16.0
+        return per + sum({3: 8 / 3, 5: 32 / 5, 7: 72 / 7}.get(r, 0.0) for r in radices)
+
+    pair = (6 * 4 + 16) / 2.0  # three squares of two products, one twiddle product, per two points
     return {
-        "k_col_fwd": 5.0 * M * math.log2(H) + N,
-        "k_row_sq": 10.0 * M * math.log2(W) + 10.0 * M + 2.0 * N,
-        "k_col_inv": 5.0 * M * math.log2(H) + N,
+        "k_col_fwd": M * (line(radix_h) + 16.0),
+        "k_row_sq": M * (2 * line(radix_w) + pair + 16.0),
+        "k_col_inv": M * line(radix_h),
     }
 
 
@@ -287,9 +300,19 @@ def run_ours(args, world: int, rank: int, local: int):
 
     # per-kernel device time and the roofline of the dominant kernel
     prof = plan.profile_kernels(30)
-    kf = kernel_flops(N3, info.fft_w, info.fft_h)
     dom = max(prof, key=prof.get)
-    achieved = kf[dom] / (prof[dom] * 1e-3) / 1e12
+    # the integer form's line plans: powers of two first, then 3
+    def plan_of(n):
+        out = []
+        for r in (8, 4, 2, 3, 5, 7):
+            while n % r == 0:
+                out.append(r)
+                n //= r
+        return out
+    km = kernel_mads(N3, info.fft_w, info.fft_h, plan_of(info.fft_w), plan_of(info.fft_h))
+    sm_hz = 1e6 * (clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 2070.0)
+    mad_peak = MAD64_PER_CLOCK_SM * SMS * sm_hz / 1e12
+    achieved = km[dom] / (prof[dom] * 1e-3) / 1e12
     iter_ms = sum(prof.values())
 
     # end to end through the C ABI with pinned host buffers, every step: H2D of the state,
@@ -337,7 +360,8 @@ def run_ours(args, world: int, rank: int, local: int):
         "impl": "gpulucas_gb300", "metric": METRIC, "value": value, "unit": "iter/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": total_ms_max / args.steps,
         "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": value / REF_PUBLISHED_ITER_S / world, "dtype": "f64",
+        "vs_baseline": value / REF_PUBLISHED_ITER_S / world,
+        "dtype": "exact 61-bit integers (GF((2^61-1)^2)), one iteration in 64 in f64",
         "data": "synthetic: the LL sequence from S0=4 (no dataset)",
         "config": {"workload": WORKLOAD,
                    "p": P3, "N": N3, "fft": f"{info.fft_h} x {info.fft_w}", "parallelism": "replicas",
@@ -345,18 +369,20 @@ def run_ours(args, world: int, rank: int, local: int):
                               "column_variant": info.col_variant, "row_variant": info.row_variant,
                               "threads_col": info.threads_col,
                               "threads_row": info.threads_row},
-                   "l2": "flushed before every timed step (512 MiB write); the test's ~170 MB of state and "
+                   "l2": "flushed before every timed step (512 MiB write); the test's ~227 MB of state and "
                          "tables exceed the 129 MB L2 anyway",
                    "vs_baseline_note": "reference's published 204.72 iter/s at N=2359296 (GTX 480/C2050)"},
-        "roofline": {"bound": "fp64", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                     "frac": achieved / peak, "traffic": read_traffic(dom),
-                     "peak_source": "measured live: DFMA probe (gl_probe_fp64_peak); MEASURED_PEAKS.json has "
-                                    "no FP64 figure",
-                     "algorithmic_flops_per_launch": kf[dom], "kernel_ms": prof,
-                     "butterfly_issue": {"fp64_instr_per_s": bfly, "of_dfma_probe": bfly / (peak * 0.5e12),
-                                         "note": "FP64 issue rate of the line DFTs' twiddled radix-8 butterfly "
-                                                 "from registers (gl_probe_fp64_butterfly), beside the DFMA "
-                                                 "probe's rate (peak/2 instructions per second)"},
+        "roofline": {"bound": "int32 multiply-add pipe", "kernel": dom, "achieved": achieved, "peak": mad_peak,
+                     "unit": "T 32x32->64-bit multiply-adds/s", "frac": achieved / mad_peak,
+                     "traffic": read_traffic(dom),
+                     "peak_source": f"{MAD64_PER_CLOCK_SM} per clock and SM (measured from registers) x {SMS} SMs "
+                                    "x the SM clock of the timed region",
+                     "algorithmic_mads_per_launch": km[dom], "kernel_ms": prof,
+                     "fp64": {"dfma_peak_tflops": peak, "butterfly_instr_per_s": bfly,
+                              "note": "the FP64 form's denominators; most iterations run in exact integer "
+                                      "arithmetic and exceed that form's FLOP_alg roofline"},
+                     "note": "the multiply-adds of twiddle products and squares alone; their limb extraction "
+                             "and reductions take as long again on the same pipes",
                      "iteration_flop_alg": flop_alg(N3),
                      "iteration_tflops": flop_alg(N3) / (iter_ms * 1e-3) / 1e12,
                      "hbm_gbs_alg": 16.0 * N3 / (iter_ms * 1e-3) / 1e9},
