@@ -114,7 +114,8 @@ def test_int_form_products_equal_fp64_form(gl, p, N):
 def test_int_form_long_lines_equal_fp64_form(gl, p, N):
     a, ra, _ = _products(gl, p, N, 67)
     b, rb, _ = _products(gl, p, N, 67, error_limit=0.39)
-    assert ra.status == rb.status == 0 and (a == b).all()
+    c, rc, _ = _products(gl, p, N, 67, autotune=0)
+    assert ra.status == rb.status == rc.status == 0 and (a == b).all() and (c == b).all()
 
 
 @pytest.mark.gpu
