@@ -5,7 +5,7 @@
 // shared memory, many iterations per launch, the passes separated by cluster barriers.
 // Lines are short (tens of points), so an iteration is a chain of latencies: a radix-8
 // butterfly of one warp takes some 4000 cycles in FP64, where every instruction holds the
-// pipe for 64, and about 700 here.  N = 2048: 14.3 -> 10.4 us per iteration; what is left
+// pipe for 64, and about 700 here.  N = 2048: 14.3 -> 10.2 us per iteration; what is left
 // is one warp's latencies and instruction fetch between barriers (radix-4 or -2 stages,
 // 128 threads, and line DFTs out of line measured the same or slower).
 //
@@ -52,6 +52,11 @@ __global__ void __launch_bounds__(kIntResidentThreads, 1) ki_resident(const __gr
   int4* wf = reinterpret_cast<int4*>(rsm + g.o_wf);
   int4* wi = reinterpret_cast<int4*>(rsm + g.o_wi);
   const int T = blockDim.x, tid = threadIdx.x;
+  // H (int_resident_geom) and C (8 or 16) are powers of two, so divisions by them are
+  // shifts: an iteration is a chain of latencies, and a division by a run-time value is
+  // tens of instructions of it.  us per iteration: 12.67 -> 12.38 at N = 4096, 14.05 -> 13.46
+  // at 3840, 10.44 -> 10.18 at 1536, 10.20 -> 10.18 at 2048.
+  const int lh = 31 - __clz(H), lC = 31 - __clz(C);
 
   const int nw = cw * 2 * H;  // my words: one contiguous block of the column-major arrays
   const int wbase = c0 * 2 * H;
@@ -86,7 +91,7 @@ __global__ void __launch_bounds__(kIntResidentThreads, 1) ki_resident(const __gr
   for (int it = 0; it < ra.iters; ++it) {
     // (A) dice, weight, column DFTs, twiddle, scatter to the row owners
     for (int idx = tid; idx < cw * H; idx += T) {
-      const int lc = idx / H, m2 = idx - lc * H;
+      const int lc = idx >> lh, m2 = idx - (lc << lh);
       const int m1 = c0 + lc, s0 = 2 * idx;
       long long P[NC + 3];
       P[0] = ll[s0 + 1];
@@ -114,11 +119,11 @@ __global__ void __launch_bounds__(kIntResidentThreads, 1) ki_resident(const __gr
     {
       const g2* res = int_line_fft<-1, true, true>(zc, zc2, cw, lsc, a.in.ph, hf);
       for (int idx = tid; idx < cw * H; idx += T) {
-        const int lc = idx / H, k2 = idx - lc * H;
+        const int lc = idx >> lh, k2 = idx - (lc << lh);
         const g2 v = gf::cmul(res[lc * lsc + ipad(k2)], K1[idx]);
         const int c = k2 <= H / 2 ? k2 : H - k2;
-        const int slot = 2 * (c / C) + (k2 == c ? 0 : 1);
-        *cl.map_shared_rank(zr + slot * lsr + ipad(c0 + lc), c % C) = v;
+        const int slot = 2 * (c >> lC) + (k2 == c ? 0 : 1);
+        *cl.map_shared_rank(zr + slot * lsr + ipad(c0 + lc), c & (C - 1)) = v;
       }
     }
     cl.sync();
@@ -134,8 +139,8 @@ __global__ void __launch_bounds__(kIntResidentThreads, 1) ki_resident(const __gr
         const bool self = c == 0 || 2 * c == H;
         g2* la = s1 + 2 * lp * lsr;
         g2* lb = self ? la : la + lsr;
-        const unsigned shift = (unsigned)__ldg(&a.in.rows[c].z);
-        const int u = (int)(((unsigned)a.in.qV * (unsigned)t + shift) % (unsigned)W);
+        const unsigned uq = (unsigned)a.in.qV * (unsigned)t + (unsigned)__ldg(&a.in.rows[c].z);
+        const int u = (int)((W & (W - 1)) == 0 ? uq & (unsigned)(W - 1) : uq % (unsigned)W);
         if (self && u < t) continue;
         g2 vk, vkp;
         gf::pair_square(la[ipad(t)], lb[ipad(u)], pr[idx], &vk, &vkp);
@@ -160,7 +165,7 @@ __global__ void __launch_bounds__(kIntResidentThreads, 1) ki_resident(const __gr
     {
       const g2* res = int_line_fft<+1, true, true>(zc, zc2, cw, lsc, a.in.ph, hi);
       for (int idx = tid; idx < cw * H; idx += T) {
-        const int lc = idx / H, m2 = idx - lc * H;
+        const int lc = idx >> lh, m2 = idx - (lc << lh);
         const int s0 = 2 * idx;
         const g2 v = res[lc * lsc + ipad(m2)];
         long long r0 = check_word(gf::unweighted(v.re, ex[s0]), &flg);
