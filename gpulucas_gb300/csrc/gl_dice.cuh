@@ -69,7 +69,15 @@ __device__ __forceinline__ void dice_pair(const long long* P, int LO, uint32_t f
 // k = 0 .. NC+2.  Words j0+1-2d and j0-2d are the two words of point m-d, column m1-d of
 // the same row (the previous row, from the last columns, when m1 < d), adjacent in the
 // column-major layout: one 16-byte load per point, and no division to find it.
-template <bool FROM_STATE, int NC>
+// EARLY: the kernel may become resident while the pass that writes the products still runs
+// (a programmatic dependent), so they are read with ordinary loads; the non-coherent path
+// is for memory that nothing writes during the kernel's whole life.
+template <bool EARLY, typename T>
+__device__ __forceinline__ T load_product(const T* p) {
+  if constexpr (EARLY) return *p;
+  else return __ldg(p);
+}
+template <bool FROM_STATE, int NC, bool EARLY = false>
 __device__ __forceinline__ void load_point(const IterArgs& a, const int m1, const int m2, int* v0, int* v1) {
   const int H = a.H, W = a.W, N = a.N, LO = a.LO;
   constexpr int D = (NC + 2) / 2;  // points m-1 .. m-D hold the words j0-1 .. j0+1-(NC+2)
@@ -80,7 +88,7 @@ __device__ __forceinline__ void load_point(const IterArgs& a, const int m1, cons
     *v1 = a.digit[j0 + 1] + (int)a.hi[j0];
   } else {
     long long P[NC + 3];
-    const longlong2 own = __ldg(reinterpret_cast<const longlong2*>(a.ll + s0));
+    const longlong2 own = load_product<EARLY>(reinterpret_cast<const longlong2*>(a.ll + s0));
     P[0] = own.y;
     P[1] = own.x;
     uint32_t fm = 0;  // flags of word j0-1 (the upper word of point m-1)
@@ -94,11 +102,11 @@ __device__ __forceinline__ void load_point(const IterArgs& a, const int m1, cons
       const int sd = 2 * (c * H + r);
       if (d == 1) fm = __ldg(a.flags + sd + 1);
       if (2 * d + 1 < NC + 3) {
-        const longlong2 v = __ldg(reinterpret_cast<const longlong2*>(a.ll + sd));
+        const longlong2 v = load_product<EARLY>(reinterpret_cast<const longlong2*>(a.ll + sd));
         P[2 * d] = v.y;
         P[2 * d + 1] = v.x;
       } else {  // only the upper word of the farthest point
-        P[2 * d] = __ldg(a.ll + sd + 1);
+        P[2 * d] = load_product<EARLY, long long>(a.ll + sd + 1);
       }
     }
     const uchar2 ff = __ldg(reinterpret_cast<const uchar2*>(a.flags + s0));

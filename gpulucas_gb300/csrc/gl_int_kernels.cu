@@ -41,6 +41,8 @@ __device__ __forceinline__ void touch(const int4* p, int n) {
 // With a.in.dependent every pass is launched as a programmatic dependent of the one before
 // it: it becomes resident while that one runs, touches its tables, and waits here for that
 // one's end.  Only then may the next pass become resident, so at most one waits at a time.
+// What the pass before writes (products, work arrays) is read with ordinary loads: the wait
+// makes it visible to them, not to the non-coherent path, which is for the tables alone.
 // For iterations launched one by one (N = 65536 without allocation: 27.3 -> 20.6 us per
 // iteration); in a replayed graph it gains nothing (163840: 23.1 -> 24-26, 65536: 18.3 ->
 // 17.2, 5120: 14.6 -> 15.5), so plans do not use it.
@@ -136,7 +138,7 @@ __device__ __forceinline__ void int_col_fwd_body(const IterArgs& a, const int m1
 #pragma unroll (P == 0 ? 2 : 1)
   for (int m2 = threadIdx.x; m2 < H; m2 += blockDim.x) {
     int v0, v1;
-    load_point<FROM_STATE, NC>(a, m1, m2, &v0, &v1);
+    load_point<FROM_STATE, NC, P == 0>(a, m1, m2, &v0, &v1);
     if (FROM_STATE) wide |= v0 > a.in.vmax || v0 < -a.in.vmax || v1 > a.in.vmax || v1 < -a.in.vmax;
     const uchar2 e = __ldg(reinterpret_cast<const uchar2*>(a.in.e + 2 * (m1 * H + m2)));
     ism[ipad(m2)] = g2{gf::weighted(v0, e.x), gf::weighted(v1, e.y)};
