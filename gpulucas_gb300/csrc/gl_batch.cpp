@@ -154,7 +154,6 @@ int assemble(gl_batch* b) {
     t_row = std::max(t_row, b->plans[i]->fg.t_row);
     // the batched column kernels always use the two-buffer line DFT
     sm_col = std::max(sm_col, (size_t)2 * b->plans[i]->fg.ls_col * 16);
-    sm_row = std::max(sm_row, b->plans[i]->fg.sm_row);
   }
   IterArgs* d_desc = nullptr;
   GB_TRY(upload(b, &d_desc, desc));
@@ -182,12 +181,14 @@ int assemble(gl_batch* b) {
                                                                  total_pairs / ((long)kRowUnitsPerSM * sms)))
                                      : 1;
   std::vector<int> pairs((size_t)ntests, 1);
-  sm_row = 0;
   for (int i = 0; i < ntests; ++i) {
     const FusedGeom& g = b->plans[i]->fg;
     int widest = 1;
     for (int s = 0; s < g.pw.nst; ++s) widest = std::max(widest, 2 * g.W / g.pw.radix[s]);
-    const size_t lines = (size_t)4 * g.ls_row * 16, stage = g.sm_row - lines;
+    // the batched row kernel always copies the stage values into shared memory, also those
+    // of a plan whose own row pass reads them through L1 (its sm_row has no room for them)
+    const size_t lines = (size_t)4 * g.ls_row * 16, stage = (size_t)desc[i].twW_n * sizeof(DevCplx);
+    if (lines + stage > (size_t)kMaxDynSmem) return GL_ERR_SIZE;
     int k = std::max(1, std::min(kcap, t_row / widest));
     while (k > 1 && (size_t)k * lines + stage > kRowUnitSmem) --k;
     pairs[(size_t)i] = k;

@@ -25,3 +25,19 @@ def test_early_resident_passes_read_written_memory_with_ordinary_loads():
     # every pass that may be launched as a dependent (P == 0) asks for the ordinary loads
     assert re.findall(r"load_point<([^>]*)>", k) == ["FROM_STATE, NC, P == 0"]
     assert "dependent) after_previous_pass()" in k
+
+
+@pytest.mark.gpu
+def test_batch_gives_row_units_room_for_the_stage_values(gl):
+    """A plan with row_pass = 2 reads its stage values through L1; the batch's row kernel
+    copies them behind the line buffers all the same."""
+    p, N = 1257787, 65536
+    o = {"fft_h": 128, "max_radix_row": 4}
+    with gl.Plan(p, N, row_pass=2, **o) as a, gl.Plan(p, N, row_pass=1, **o) as b, gl.Plan(p, N) as want:
+        assert a.info.row_variant == 2 and b.info.row_variant == 1
+        assert a.info.smem_row < b.info.smem_row
+        with gl.Batch(plans=[a]) as batch:
+            assert batch.info.smem_row >= b.info.smem_row
+            batch.iterate(70)
+        want.iterate(70)
+        assert (a.products() == want.products()).all()
