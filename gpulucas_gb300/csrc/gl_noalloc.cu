@@ -62,7 +62,8 @@ constexpr size_t kScratchBytes = kOffRows + align256(sizeof(RowPair) * kNoAllocM
 // never a device address: the address comes from cudaGetSymbolAddress below.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
-// Host staging for the per-test tables, reused by every call (no host allocation).
+// Host staging for the per-test tables, reused by every call.  The FP64 tables' is static;
+// the integer form's is allocated on the host, with the first test that needs it.
 static DevCplx h_twM[kNoAllocMaxM];
 static DevCplx h_pair[kNoAllocMaxM];
 static double h_A[kNoAllocMaxN];
@@ -81,7 +82,8 @@ static struct {
 
 struct DeviceSlot {
   unsigned char* base = nullptr;  // device address of g_noalloc_scratch on this device
-  int p = 0, N = 0;               // test whose tables the scratch holds
+  int p = 0, N = 0;               // test whose tables the scratch holds (0: none whole)
+  bool int_known = false;         // whether the integer form's tables were asked for
   int H = 0;                      // integer form: column length, geometry (H = 0: none)
   IntGeom g{};
   int nrows = 0;
@@ -148,8 +150,8 @@ constexpr int kNoAllocFp64Every = 64;
 
 using namespace gl;
 
-extern "C" int gl_iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* ll_out, int64_t iters,
-                                  double* max_roundoff, void* stream) {
+static int iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* ll_out, int64_t iters, double* max_roundoff,
+                           void* stream) {
   if (!ll_in || !ll_out || iters < 0) return GL_ERR_ARG;
   if (p < 3 || N < 16 || (N & 1) || N > p) return GL_ERR_ARG;
   if (N > kNoAllocMaxN) return GL_ERR_TOO_LARGE;
@@ -194,16 +196,22 @@ extern "C" int gl_iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* l
     }
   }
   unsigned char* base = slot.base;
-  if (slot.p != p || slot.N != N) {
+  // The slot names no test while its tables are being replaced, so that a call that ends
+  // half way (an error, an exception) leaves none that a later call would take for whole.
+  const int held_p = slot.p, held_N = slot.N;
+  slot.p = slot.N = 0;
+  if (held_p != p || held_N != N) {
     build_tables(p, N);
     if (cudaMemcpyAsync(base + kOffTwM, h_twM, sizeof(DevCplx) * M, cudaMemcpyHostToDevice, s) ||
         cudaMemcpyAsync(base + kOffPair, h_pair, sizeof(DevCplx) * M, cudaMemcpyHostToDevice, s) ||
         cudaMemcpyAsync(base + kOffA, h_A, sizeof(double) * N, cudaMemcpyHostToDevice, s) ||
         cudaMemcpyAsync(base + kOffAinv, h_Ainv, sizeof(double) * N, cudaMemcpyHostToDevice, s) ||
-        cudaMemcpyAsync(base + kOffFlags, h_flags, N, cudaMemcpyHostToDevice, s)) {
-      slot.p = slot.N = 0;
+        cudaMemcpyAsync(base + kOffFlags, h_flags, N, cudaMemcpyHostToDevice, s))
       return GL_ERR_CUDA;
-    }
+    slot.int_known = false;
+    slot.H = 0;
+  }
+  if (iters >= 2 && !slot.int_known) {  // shorter calls run the plain form alone
     build_int_tables(p, N, n);
     if (h_int.H) {
       auto up = [&](size_t off, const auto& v) {
@@ -212,17 +220,15 @@ extern "C" int gl_iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* l
       bool bad = up(kOffFlagsC, h_int.flags) || up(kOffSpan, h_int.span) || up(kOffExp, h_int.e) ||
                  up(kOffK1, h_int.k1) || up(kOffK2, h_int.k2) || up(kOffIntPair, h_int.pair) || up(kOffRows, h_int.rows);
       for (int i = 0; i < 4; ++i) bad = bad || up(stage_offset(i), h_int.stages[i]);
-      if (bad || set_int_smem_limits() != cudaSuccess) {
-        slot.p = slot.N = 0;
-        return GL_ERR_CUDA;
-      }
+      if (bad || set_int_smem_limits() != cudaSuccess) return GL_ERR_CUDA;
     }
     slot.H = h_int.H;
     slot.g = h_int.g;
     slot.nrows = (int)h_int.rows.size();
-    slot.p = p;
-    slot.N = N;
+    slot.int_known = true;
   }
+  slot.p = p;
+  slot.N = N;
 
   IterArgs a{};
   a.N = N; a.M = M; a.LO = p / N; a.n = n;
@@ -283,4 +289,13 @@ extern "C" int gl_iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* l
   if (h_status.flags) return GL_ERR_OVERFLOW;
   if (e >= 0.4) return GL_ERR_ROUNDOFF;
   return GL_OK;
+}
+
+extern "C" int gl_iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* ll_out, int64_t iters,
+                                  double* max_roundoff, void* stream) {
+  try {
+    return iterate_noalloc(p, N, ll_in, ll_out, iters, max_roundoff, stream);
+  } catch (...) {  // host memory for the integer form's tables
+    return GL_ERR_NOMEM;
+  }
 }

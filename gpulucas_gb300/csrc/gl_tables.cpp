@@ -115,10 +115,15 @@ void parallel_for(int64_t n, const std::function<void(int64_t, int64_t)>& chunk)
   if (nt > n / 1024) nt = n / 1024;
   std::vector<std::thread> th;
   th.reserve((size_t)nt);
-  for (int64_t t = 0; t < nt; ++t) {
-    const int64_t b = n * t / nt, e = n * (t + 1) / nt;
-    th.emplace_back([&chunk, b, e] { chunk(b, e); });
+  int64_t t = 0;
+  try {
+    for (; t < nt; ++t) {
+      const int64_t b = n * t / nt, e = n * (t + 1) / nt;
+      th.emplace_back([&chunk, b, e] { chunk(b, e); });
+    }
+  } catch (...) {  // no more threads: the rest runs here
   }
+  if (t < nt) chunk(n * t / nt, n);
   for (auto& x : th) x.join();
 }
 

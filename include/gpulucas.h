@@ -392,14 +392,15 @@ int gl_server_destroy(gl_server* server);
  * by the caller, natural word order; they may be the same buffer, but buffers that
  * overlap only in part return GL_ERR_ARG), and stores the maximum round-off of its
  * floating-point iterations (all, or one in 64 and the call's last; see gl_iterate) in
- * *max_roundoff.  It allocates nothing: its work arrays, tables and status word live in
+ * *max_roundoff.  It allocates no device memory: its work arrays, tables and status word live in
  * a static device array sized for N <= 65536 (about 5.9 MiB, held on every GPU that
  * loads the library until exit); larger N returns GL_ERR_TOO_LARGE.  A call with new
- * (p, N) uploads that test's tables into the array first.  The call is synchronous: it
- * returns after `stream` has finished the iterations, so it cannot be captured into a
- * CUDA graph (on a stream that is capturing it returns GL_ERR_ARG and enqueues
- * nothing).  All calls share the array; a lock held until the stream has finished keeps
- * the calls of one process from overlapping on the GPU.
+ * (p, N) uploads that test's tables into the array first; the integer form's are built in
+ * host memory, with the test's first call of two iterations or more (GL_ERR_NOMEM if there
+ * is none).  The call is synchronous: it returns after `stream` has finished the
+ * iterations, so it cannot be captured into a CUDA graph (on a stream that is capturing it
+ * returns GL_ERR_ARG and enqueues nothing).  All calls share the array; a lock held until
+ * the stream has finished keeps the calls of one process from overlapping on the GPU.
  * Returns GL_ERR_ROUNDOFF at round-off >= 0.4 and GL_ERR_OVERFLOW as gl_iterate. */
 int gl_iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* ll_out, int64_t iters,
                        double* max_roundoff, void* stream);

@@ -2,6 +2,8 @@
 leaves behind, which form a plan runs, and the calls of an integer plan that run in FP64."""
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 
@@ -41,3 +43,72 @@ def test_batch_gives_row_units_room_for_the_stage_values(gl):
             batch.iterate(70)
         want.iterate(70)
         assert (a.products() == want.products()).all()
+
+
+# operator new that fails on request for blocks of a size or more
+_NEW_SHIM = r"""
+#include <cstdlib>
+#include <new>
+static std::size_t g_limit = 0;
+extern "C" void fail_new_from(std::size_t n) { g_limit = n; }
+void* operator new(std::size_t n) {
+  if (g_limit && n >= g_limit) throw std::bad_alloc();
+  void* p = std::malloc(n ? n : 1);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
+"""
+
+_NOALLOC_CHILD = r"""
+import ctypes, sys
+import numpy as np
+import torch
+sys.path.insert(0, sys.argv[1])
+import gpulucas_gb300 as gl
+arm = ctypes.CDLL(None).fail_new_from
+arm.argtypes = [ctypes.c_size_t]
+
+def call(p, N, k, limit=0):
+    d = torch.zeros(N, dtype=torch.int64, device="cuda")
+    d[0] = 4
+    err = ctypes.c_double()
+    torch.cuda.synchronize()
+    arm(limit)
+    rc = gl.lib.gl_iterate_noalloc(p, N, ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(d.data_ptr()), k,
+                                   ctypes.byref(err), None)
+    arm(0)
+    return rc, d.cpu().numpy()
+
+def want(p, N, k):
+    with gl.Plan(p, N, mode=gl.MODE_PLAIN) as pl:
+        pl.iterate(k)
+        return pl.products()
+
+A, B, C = (21701, 1024), (44497, 2048), (86243, 4096)  # growing: staging is kept between calls
+rc, a = call(*A, 5)
+assert rc == 0 and (a == want(*A, 5)).all()
+rc, _ = call(*B, 5, 4096)           # no memory for B's integer tables
+assert rc == gl.GL_ERR_NOMEM, rc
+rc, a = call(*A, 5)                 # B's FP64 tables had replaced A's
+assert rc == 0 and (a == want(*A, 5)).all()
+rc, b = call(*B, 5)
+assert rc == 0 and (b == want(*B, 5)).all()
+for k in (0, 1):                    # too short for the integer form: no tables of it
+    rc, c = call(*C, k, 4096)
+    assert rc == 0 and (k == 0 or (c == want(*C, k)).all()), (k, rc)
+rc, c = call(*C, 5)
+assert rc == 0 and (c == want(*C, 5)).all()
+print("done")
+"""
+
+
+@pytest.mark.gpu
+def test_noalloc_call_that_runs_out_of_host_memory_leaves_no_stale_tables(tmp_path):
+    src, shim = tmp_path / "new.cpp", tmp_path / "new.so"
+    src.write_text(_NEW_SHIM)
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", str(src), "-o", str(shim)], check=True)
+    r = subprocess.run([sys.executable, "-c", _NOALLOC_CHILD, ROOT], env=dict(os.environ, LD_PRELOAD=str(shim)),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, r.stderr[-2000:]
