@@ -577,7 +577,7 @@ double time_int_layout(int M, int H, const IntVariant& var, int n, int iters, cu
     ok = cudaMalloc(&buf[i], bytes[i]) == cudaSuccess && cudaMemsetAsync(buf[i], 0, bytes[i], s) == cudaSuccess;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ok) ok = cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess;
-  if (ok) ok = set_int_smem_limits() == cudaSuccess;
+  if (ok) ok = set_int_smem_limits(g, n, (int)rows.size(), false) == cudaSuccess;
   if (ok)
     ok = cudaMemcpyAsync(buf[13], rows.data(), rows.size() * sizeof(RowPair), cudaMemcpyHostToDevice, s) == cudaSuccess &&
          cudaStreamSynchronize(s) == cudaSuccess;
@@ -926,7 +926,7 @@ static int build_int_tables(gl_plan* pl, int vmax) {
   gl_int_args(H, W, pl->ig, (int)rows.size(), &in);
   in.vmax = vmax;
   in.check_span = (pl->n + 1) * pl->LO < 51;
-  GL_CUDA(set_int_smem_limits());
+  GL_CUDA(set_int_smem_limits(pl->ig, pl->n, (int)rows.size(), true));
   pl->int_form = true;
   return GL_OK;
 }

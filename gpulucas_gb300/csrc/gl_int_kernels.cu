@@ -368,71 +368,55 @@ void run(void (*kernel)(IterArgs), int grid, int block, size_t smem, cudaStream_
   cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
+using IntKernel = void (*)(IterArgs);
+
 template <bool FS, bool B57, int P>
-void launch_col_fwd_p(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
-  void (*const kernels[5])(IterArgs) = {ki_col_fwd<FS, 2, B57, P>, ki_col_fwd<FS, 3, B57, P>, ki_col_fwd<FS, 4, B57, P>,
-                                        ki_col_fwd<FS, 5, B57, P>, ki_col_fwd<FS, 6, B57, P>};
-  run(kernels[a.n - 2], a.W, g.t_col, g.sm_col, s, a, P == 0 && a.in.dependent);
+IntKernel col_fwd_nc(int n) {
+  const IntKernel kernels[5] = {ki_col_fwd<FS, 2, B57, P>, ki_col_fwd<FS, 3, B57, P>, ki_col_fwd<FS, 4, B57, P>,
+                                ki_col_fwd<FS, 5, B57, P>, ki_col_fwd<FS, 6, B57, P>};
+  return kernels[n - 2];
 }
-template <bool FS, bool B57>
-void launch_col_fwd(const IterArgs& a, const IntGeom& g, cudaStream_t s) {
-  if (!B57 && g.col_p) launch_col_fwd_p<FS, false, kIntHeld>(a, g, s);
-  else launch_col_fwd_p<FS, B57, 0>(a, g, s);
+bool cols_in_place(const IntGeom& g) { return g.col_p && !has57(g.ph); }
+
+// The kernels of the three passes for a geometry.
+IntKernel col_fwd_kernel(const IntGeom& g, int n, bool from_state) {
+  if (cols_in_place(g)) return from_state ? col_fwd_nc<true, false, kIntHeld>(n) : col_fwd_nc<false, false, kIntHeld>(n);
+  if (has57(g.ph)) return from_state ? col_fwd_nc<true, true, 0>(n) : col_fwd_nc<false, true, 0>(n);
+  return from_state ? col_fwd_nc<true, false, 0>(n) : col_fwd_nc<false, false, 0>(n);
 }
+IntKernel row_kernel(const IntGeom& g, int nrows) {
+  if (g.t > 1) return ki_row_poly;
+  if (has57(g.pw)) return ki_row_sq<true, 256, 2>;
+  if (g.t_row <= 192 && nrows > kRowsFor5) return ki_row_sq<false, 192, 5>;
+  return ki_row_sq<false, 256, 3>;
+}
+IntKernel col_inv_kernel(const IntGeom& g) {
+  if (cols_in_place(g)) return ki_col_inv<false, kIntHeld>;
+  return has57(g.ph) ? ki_col_inv<true, 0> : ki_col_inv<false, 0>;
+}
+
 void launch_pass(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which, bool from_state) {
-  const bool c57 = has57(g.ph), r57 = has57(g.pw);
-  if (which == 0) {
-    if (from_state) c57 ? launch_col_fwd<true, true>(a, g, s) : launch_col_fwd<true, false>(a, g, s);
-    else c57 ? launch_col_fwd<false, true>(a, g, s) : launch_col_fwd<false, false>(a, g, s);
-  } else if (which == 1) {
-    void (*kernel)(IterArgs) = ki_row_sq<false, 256, 3>;
-    if (g.t > 1) kernel = ki_row_poly;
-    else if (r57) kernel = ki_row_sq<true, 256, 2>;
-    else if (g.t_row <= 192 && a.in.nrows > kRowsFor5) kernel = ki_row_sq<false, 192, 5>;
-    run(kernel, a.in.nrows, g.t_row, g.sm_row, s, a, a.in.dependent);
-  } else {
-    const bool ip = !c57 && g.col_p;
-    run(ip ? ki_col_inv<false, kIntHeld> : c57 ? ki_col_inv<true, 0> : ki_col_inv<false, 0>, a.W, g.t_col, g.sm_col, s, a,
-        !ip && a.in.dependent);
-  }
+  if (which == 1) run(row_kernel(g, a.in.nrows), a.in.nrows, g.t_row, g.sm_row, s, a, a.in.dependent);
+  else
+    run(which == 0 ? col_fwd_kernel(g, a.n, from_state) : col_inv_kernel(g), a.W, g.t_col, g.sm_col, s, a,
+        !cols_in_place(g) && a.in.dependent);
 }
 
-template <typename K>
-cudaError_t raise(K* kernel) {
+// A kernel's limit is process-wide: it is raised to the layout chooser's bound, whoever asks
+// first, and only where a launch needs more than every kernel may have.
+cudaError_t raise(IntKernel kernel, size_t smem) {
+  if (smem <= 48 * 1024) return cudaSuccess;
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxIntSmem);
-}
-
-template <bool FS, bool B57, int P>
-cudaError_t raise_col_fwd() {
-  cudaError_t e;
-  if ((e = raise(ki_col_fwd<FS, 2, B57, P>))) return e;
-  if ((e = raise(ki_col_fwd<FS, 3, B57, P>))) return e;
-  if ((e = raise(ki_col_fwd<FS, 4, B57, P>))) return e;
-  if ((e = raise(ki_col_fwd<FS, 5, B57, P>))) return e;
-  return raise(ki_col_fwd<FS, 6, B57, P>);
-}
-
-template <bool B57, int P>
-cudaError_t raise_col() {
-  cudaError_t e;
-  if ((e = raise_col_fwd<false, B57, P>())) return e;
-  if ((e = raise_col_fwd<true, B57, P>())) return e;
-  return raise(ki_col_inv<B57, P>);
 }
 
 }  // namespace
 
-// per kernel and process-wide, raised to the layout chooser's bound
-cudaError_t set_int_smem_limits() {
+cudaError_t set_int_smem_limits(const IntGeom& g, int n, int nrows, bool from_state) {
   cudaError_t e;
-  if ((e = raise_col<false, 0>())) return e;
-  if ((e = raise_col<true, 0>())) return e;
-  if ((e = raise_col<false, kIntHeld>())) return e;
-  if ((e = raise(ki_row_poly))) return e;
-  if ((e = raise(ki_row_sq<false, 192, 5>))) return e;
-  if ((e = raise(ki_row_sq<false, 256, 3>))) return e;
-  if ((e = raise(ki_row_sq<true, 256, 2>))) return e;
-  return cudaSuccess;
+  if ((e = raise(col_fwd_kernel(g, n, false), g.sm_col))) return e;
+  if (from_state && (e = raise(col_fwd_kernel(g, n, true), g.sm_col))) return e;
+  if ((e = raise(row_kernel(g, nrows), g.sm_row))) return e;
+  return raise(col_inv_kernel(g), g.sm_col);
 }
 
 cudaError_t launch_int_kernel(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which) {

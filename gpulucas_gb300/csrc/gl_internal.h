@@ -199,7 +199,9 @@ cudaError_t launch_fused_kernel(const IterArgs& a, const FusedGeom& g, cudaStrea
 // (from_state) with a word beyond a.in.vmax sets kStatusWide and its products are invalid.
 cudaError_t launch_int_iteration(const IterArgs& a, const IntGeom& g, cudaStream_t s, bool from_state);
 cudaError_t launch_int_kernel(const IterArgs& a, const IntGeom& g, cudaStream_t s, int which);
-cudaError_t set_int_smem_limits();
+// Shared-memory limits of the kernels that the geometry's iterations launch, and of no others
+// (naming a kernel loads its code onto the device); from_state: also from a loaded state.
+cudaError_t set_int_smem_limits(const IntGeom& g, int n, int nrows, bool from_state);
 cudaError_t launch_plain_iteration(const IterArgs& a, const PlainGeom& g, cudaStream_t s);
 cudaError_t launch_set_initial(const IterArgs& a, int mode, cudaStream_t s);
 // carry-save state (digit, hi) = dice(ll) for the fused form; plain keeps it already

@@ -220,7 +220,7 @@ static int iterate_noalloc(int p, int N, const int64_t* ll_in, int64_t* ll_out, 
       bool bad = up(kOffFlagsC, h_int.flags) || up(kOffSpan, h_int.span) || up(kOffExp, h_int.e) ||
                  up(kOffK1, h_int.k1) || up(kOffK2, h_int.k2) || up(kOffIntPair, h_int.pair) || up(kOffRows, h_int.rows);
       for (int i = 0; i < 4; ++i) bad = bad || up(stage_offset(i), h_int.stages[i]);
-      if (bad || set_int_smem_limits() != cudaSuccess) return GL_ERR_CUDA;
+      if (bad || set_int_smem_limits(h_int.g, n, (int)h_int.rows.size(), false) != cudaSuccess) return GL_ERR_CUDA;
     }
     slot.H = h_int.H;
     slot.g = h_int.g;

@@ -394,7 +394,8 @@ int gl_server_destroy(gl_server* server);
  * floating-point iterations (all, or one in 64 and the call's last; see gl_iterate) in
  * *max_roundoff.  It allocates no device memory: its work arrays, tables and status word live in
  * a static device array sized for N <= 65536 (about 5.9 MiB, held on every GPU that
- * loads the library until exit); larger N returns GL_ERR_TOO_LARGE.  A call with new
+ * loads the library until exit; the driver loads a kernel's code when it is first launched,
+ * 4 to 6 MiB with a process's first call); larger N returns GL_ERR_TOO_LARGE.  A call with new
  * (p, N) uploads that test's tables into the array first; the integer form's are built in
  * host memory, with the test's first call of two iterations or more (GL_ERR_NOMEM if there
  * is none).  The call is synchronous: it returns after `stream` has finished the

@@ -112,3 +112,31 @@ def test_noalloc_call_that_runs_out_of_host_memory_leaves_no_stale_tables(tmp_pa
     r = subprocess.run([sys.executable, "-c", _NOALLOC_CHILD, ROOT], env=dict(os.environ, LD_PRELOAD=str(shim)),
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "done" in r.stdout, r.stderr[-2000:]
+
+
+_FIRST_CALL_CHILD = r"""
+import sys
+import torch
+sys.path.insert(0, sys.argv[1])
+import gpulucas_gb300 as gl
+p, N = 859433, 49152
+d = torch.zeros(N, dtype=torch.int64, device="cuda")
+d[0] = 4
+torch.cuda.synchronize()
+free = [torch.cuda.mem_get_info()[0]]
+for _ in range(2):
+    gl.iterate_noalloc(p, N, d.data_ptr(), d.data_ptr(), 70, 0)
+    free.append(torch.cuda.mem_get_info()[0])
+print(free[0] - free[1], free[1] - free[2])
+"""
+
+
+@pytest.mark.gpu
+def test_noalloc_first_call_loads_only_the_kernels_it_launches():
+    """The call allocates nothing, but the driver loads each kernel's code when it is first
+    named, in granules of 2 MiB: two for the plain form's kernels, one for the integer form's
+    three of this geometry.  All of the integer form's kernels would take two."""
+    r = subprocess.run([sys.executable, "-c", _FIRST_CALL_CHILD, ROOT], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    first, second = map(int, r.stdout.split())
+    assert first <= 6 << 20 and second == 0
