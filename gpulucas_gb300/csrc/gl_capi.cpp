@@ -1,6 +1,7 @@
 // gl_capi.cpp -- the C ABI (include/gpulucas.h): plans, iteration, residues and the
 // reference-named entry points errorTest / mersenneTest / setSliceAndDice.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <map>
@@ -478,25 +479,29 @@ double time_layout(int M, int H, int rc, int rr, bool ip, bool pf, bool ws, int 
 // weights, two columns per CTA) are timed on the best lengths, and the winner once more
 // with radix-4 rows: a radix-8 row stage of W/8 butterflies per line leaves part of a warp
 // idle when 2W/8 is not a multiple of 32 (W = 576: 144 butterflies on 192 threads), while
-// radix-4 stages fill whole warps.
+// radix-4 stages fill whole warps.  only_h: that column length alone (an integer-form plan's,
+// whose FP64 iterations run on the layout the integer search picked).
 struct TunedLayout {
   int H = 0, rc = kMaxRadix, rr = kMaxRadix, row = 0;
   bool ip = false, pf = false, ws = false;
   double ms = 0.0;
 };
 std::mutex g_tune_mutex;
-std::map<std::pair<int, int>, TunedLayout> g_tune_cache;
+std::map<std::array<int, 3>, TunedLayout> g_tune_cache;
 
-TunedLayout autotune_layout(int M, int n, int sms, cudaStream_t s, double* ms_out) {
+TunedLayout autotune_layout(int M, int n, int sms, cudaStream_t s, double* ms_out, int only_h = 0) {
   {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
-    auto it = g_tune_cache.find({M, sms});
+    auto it = g_tune_cache.find({M, sms, only_h});
     if (it != g_tune_cache.end()) {
       if (ms_out) *ms_out = it->second.ms;
       return it->second;
     }
   }
-  const auto ranked = ranked_layouts(M, sms);
+  auto ranked = ranked_layouts(M, sms);
+  if (only_h)
+    ranked.erase(std::remove_if(ranked.begin(), ranked.end(), [&](const auto& c) { return c.second != only_h; }),
+                 ranked.end());
   TunedLayout best;
   double best_ms = 1e300;
   const int iters = M >= (1 << 18) ? 10 : 40;
@@ -552,7 +557,7 @@ TunedLayout autotune_layout(int M, int n, int sms, cudaStream_t s, double* ms_ou
   if (!best.H) return best;
   best.ms = best_ms;
   std::lock_guard<std::mutex> lock(g_tune_mutex);
-  g_tune_cache[{M, sms}] = best;
+  g_tune_cache[{M, sms, only_h}] = best;
   if (ms_out) *ms_out = best_ms;
   return best;
 }
@@ -1025,8 +1030,8 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   }
   bool col_ip = false, col_pf = false, col_ws = false;
   int row_var = 0;
-  if (o.mode == GL_MODE_FUSED && !force_h && o.autotune && !sms_override) {
-    const TunedLayout t = autotune_layout(M, n, sms, 0, nullptr);
+  if (o.mode == GL_MODE_FUSED && (!force_h || (int_form && !resident)) && o.autotune && !sms_override) {
+    const TunedLayout t = autotune_layout(M, n, sms, 0, nullptr, force_h);
     if (t.H) {
       force_h = t.H;
       if (!o.max_radix_col) cap_c = t.rc;

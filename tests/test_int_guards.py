@@ -140,3 +140,16 @@ def test_noalloc_first_call_loads_only_the_kernels_it_launches():
     assert r.returncode == 0, r.stderr[-2000:]
     first, second = map(int, r.stdout.split())
     assert first <= 6 << 20 and second == 0
+
+
+@pytest.mark.gpu
+def test_fp64_iterations_of_an_integer_plan_run_a_timed_variant(gl):
+    """The integer search fixes the column length; the FP64 form's variants are timed for it.
+    At 2048 x 2048 every timed variant beats the untimed default (two line buffers, radix-8
+    rows in the kernel for any radix) by several per cent."""
+    p, N = 74207281, 4194304
+    with gl.Plan(p, N) as pl:
+        assert pl.info.col_variant != -1 or pl.info.row_variant != -1
+        assert pl.iterate(1).max_roundoff == 0.0  # an integer iteration
+    with gl.Plan(p, N, autotune=0) as pl:
+        assert pl.info.col_variant == -1 and pl.info.row_variant == -1
