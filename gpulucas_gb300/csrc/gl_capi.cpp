@@ -425,10 +425,35 @@ bool int_roundoff_ok(int p, int N, double error_limit) {
   return error_limit >= 0.4 && (double)p / N <= 19.2 + over - 0.26 * std::log2(N / 163840.0);
 }
 
+// Device buffers of a layout search, kept from one variant to the next: allocated
+// zero-filled, grown where a variant needs more.
+struct SearchBuffers {
+  static constexpr int kMax = 16;
+  void* ptr[kMax] = {};
+  size_t cap[kMax] = {};
+  ~SearchBuffers() {
+    for (void* p : ptr)
+      if (p) cudaFree(p);
+  }
+  bool get(int i, size_t bytes, cudaStream_t s) {
+    if (cap[i] >= bytes) return true;
+    if (ptr[i]) cudaFree(ptr[i]);
+    ptr[i] = nullptr;
+    cap[i] = 0;
+    if (cudaMalloc(&ptr[i], bytes) != cudaSuccess) {
+      cudaGetLastError();  // the next launch would return it as its own
+      ptr[i] = nullptr;
+      return false;
+    }
+    cap[i] = bytes;
+    return cudaMemsetAsync(ptr[i], 0, bytes, s) == cudaSuccess;
+  }
+};
+
 // Device time of one fused iteration with column length H, measured on zero-filled
 // buffers (the kernels' time does not depend on the values).  Returns ms, or -1.
 double time_layout(int M, int H, int rc, int rr, bool ip, bool pf, bool ws, int row, int n, int sms, int iters,
-                   cudaStream_t s) {
+                   SearchBuffers& sb, cudaStream_t s) {
   FusedGeom g{};
   if (choose_fused_geom(M, H, sms, &g, rc, rr, ip, pf, ws, row) != GL_OK) return -1.0;
   const int N = 2 * M;
@@ -438,11 +463,11 @@ double time_layout(int M, int H, int rc, int rr, bool ip, bool pf, bool ws, int 
                           16 * (size_t)szw, 16 * (size_t)szh, sizeof(int) * N, (size_t)N, sizeof(Status),
                           16 * (size_t)M};
   constexpr int nb = sizeof(bytes) / sizeof(bytes[0]);
-  void* buf[nb] = {};
+  static_assert(nb <= SearchBuffers::kMax, "buffers of a search");
+  void* const* buf = sb.ptr;
   double ms = -1.0;
   bool ok = true;
-  for (int i = 0; i < nb && ok; ++i) ok = cudaMalloc(&buf[i], bytes[i]) == cudaSuccess &&
-                                         cudaMemsetAsync(buf[i], 0, bytes[i], s) == cudaSuccess;
+  for (int i = 0; i < nb && ok; ++i) ok = sb.get(i, bytes[i], s);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ok) ok = cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess;
   if (ok) ok = set_fused_smem_limits(g) == cudaSuccess;
@@ -466,8 +491,6 @@ double time_layout(int M, int H, int rc, int rr, bool ip, bool pf, bool ws, int 
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   cudaStreamSynchronize(s);
-  for (void* b : buf)
-    if (b) cudaFree(b);
   return ms;
 }
 
@@ -505,8 +528,9 @@ TunedLayout autotune_layout(int M, int n, int sms, cudaStream_t s, double* ms_ou
   TunedLayout best;
   double best_ms = 1e300;
   const int iters = M >= (1 << 18) ? 10 : 40;
+  SearchBuffers sb;
   auto consider = [&](int H, int rc, int rr, bool ip, bool pf = false, bool ws = false, int row = 0) {
-    const double ms = time_layout(M, H, rc, rr, ip, pf, ws, row, n, sms, iters, s);
+    const double ms = time_layout(M, H, rc, rr, ip, pf, ws, row, n, sms, iters, sb, s);
     if (ms > 0.0 && ms < best_ms) {
       best_ms = ms;
       best.H = H;
@@ -562,8 +586,11 @@ TunedLayout autotune_layout(int M, int n, int sms, cudaStream_t s, double* ms_ou
   return best;
 }
 
-// Device time of one integer-form iteration on the H x (M / H) layout, or -1.
-double time_int_layout(int M, int H, const IntVariant& var, int n, int iters, cudaStream_t s) {
+// Device time of one integer-form iteration on the H x (M / H) layout, or -1.  The best of
+// three runs, since variants of short lengths lie within a few per cent; of fewer, once it is
+// a third above best_ms, the fastest variant so far (a hiccup of the host makes up a tenth).
+double time_int_layout(int M, int H, const IntVariant& var, int n, int iters, double best_ms, SearchBuffers& sb,
+                       cudaStream_t s) {
   IntGeom g{};
   const int W = M / H, N = 2 * M;
   if (!choose_int_geom(H, W, &g, var)) return -1.0;
@@ -575,11 +602,11 @@ double time_int_layout(int M, int H, const IntVariant& var, int n, int iters, cu
   const size_t bytes[] = {8 * (size_t)N, (size_t)N, (size_t)N, (size_t)N, m16, m16, m16, m16, m16,
                           szw, szw, szh, szh, rows.size() * sizeof(RowPair), sizeof(Status)};
   constexpr int nb = sizeof(bytes) / sizeof(bytes[0]);
-  void* buf[nb] = {};
+  static_assert(nb <= SearchBuffers::kMax, "buffers of a search");
+  void* const* buf = sb.ptr;
   double ms = -1.0;
   bool ok = true;
-  for (int i = 0; i < nb && ok; ++i)
-    ok = cudaMalloc(&buf[i], bytes[i]) == cudaSuccess && cudaMemsetAsync(buf[i], 0, bytes[i], s) == cudaSuccess;
+  for (int i = 0; i < nb && ok; ++i) ok = sb.get(i, bytes[i], s);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ok) ok = cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess;
   if (ok) ok = set_int_smem_limits(g, n, (int)rows.size(), false) == cudaSuccess;
@@ -597,8 +624,7 @@ double time_int_layout(int M, int H, const IntVariant& var, int n, int iters, cu
     a.in.rows = (const int4*)buf[13]; a.status = (Status*)buf[14];
     gl_int_args(H, W, g, (int)rows.size(), &a.in);
     for (int i = 0; i < 2 && ok; ++i) ok = launch_int_iteration(a, g, s, false) == cudaSuccess;
-    // the best of three runs: variants of short lengths lie within a few per cent
-    for (int round = 0; round < 3 && ok; ++round) {
+    for (int round = 0; round < 3 && ok && !(ms > 1.33 * best_ms); ++round) {
       ok = cudaEventRecord(e0, s) == cudaSuccess;
       for (int i = 0; i < iters && ok; ++i) ok = launch_int_iteration(a, g, s, false) == cudaSuccess;
       ok = ok && cudaEventRecord(e1, s) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess;
@@ -609,8 +635,6 @@ double time_int_layout(int M, int H, const IntVariant& var, int n, int iters, cu
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   cudaStreamSynchronize(s);
-  for (void* b : buf)
-    if (b) cudaFree(b);
   return ms;
 }
 
@@ -635,9 +659,10 @@ IntTuned autotune_int_layout(int M, int n, int sms, cudaStream_t s) {
     if (it != g_int_tune_cache.end()) return it->second;
   }
   IntTuned best;
+  SearchBuffers sb;
   std::vector<std::pair<double, int>> timed;  // column lengths by their best time
   auto consider = [&](int H, const IntVariant& var) {
-    const double ms = time_int_layout(M, H, var, n, M >= (1 << 18) ? 10 : 40, s);
+    const double ms = time_int_layout(M, H, var, n, M >= (1 << 18) ? 10 : 40, best.ms, sb, s);
     if (ms > 0.0 && ms < best.ms) best = IntTuned{H, var, ms};
     return ms;
   };
