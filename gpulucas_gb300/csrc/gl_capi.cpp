@@ -38,7 +38,10 @@ template <typename T>
 int dev_alloc(gl_plan* pl, T** ptr, size_t count) {
   void* p = nullptr;
   size_t bytes = sizeof(T) * count;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) return GL_ERR_NOMEM;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();  // the next launch would return it as its own
+    return GL_ERR_NOMEM;
+  }
   pl->allocs.push_back(p);
   pl->device_bytes += bytes;
   *ptr = static_cast<T*>(p);
@@ -1213,7 +1216,17 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   a.ll = ll; a.flags = fl; a.span = span; a.A = dA; a.Ainv = dAi; a.Z = Z; a.Z2 = Z2;
   a.twM = dtwM; a.twW = dtwW; a.twH = dtwH; a.twK1 = dK1; a.twPair = dPair; a.twK2 = dK2;
   a.digit = digit; a.hi = hi; a.status = status;
-  if (int_form) GL_TRY(build_int_tables(pl, vmax));
+  if (int_form) {
+    const size_t held = pl->allocs.size(), bytes = pl->device_bytes;
+    const int ri = build_int_tables(pl, vmax);
+    if (ri == GL_ERR_NOMEM) {  // its tables do not fit beside the FP64 form's: FP64 alone
+      for (; pl->allocs.size() > held; pl->allocs.pop_back()) cudaFree(pl->allocs.back());
+      pl->device_bytes = bytes;
+      a.in = IntArgs{};
+    } else {
+      GL_TRY(ri);
+    }
+  }
   *out = pl;
   int r = gl_reset(pl);
   if (r != GL_OK) {

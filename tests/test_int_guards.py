@@ -1,11 +1,15 @@
 """Guards around the integer form: memory that an early-resident pass reads, what a failed call
 leaves behind, which form a plan runs, and the calls of an integer plan that run in FP64."""
+import ctypes
 import os
 import re
 import subprocess
 import sys
 
+import numpy as np
 import pytest
+
+from gpulucas_gb300 import _build
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "gpulucas_gb300", "csrc")
@@ -150,6 +154,84 @@ def test_fp64_iterations_of_an_integer_plan_run_a_timed_variant(gl):
     p, N = 74207281, 4194304
     with gl.Plan(p, N) as pl:
         assert pl.info.col_variant != -1 or pl.info.row_variant != -1
-        assert pl.iterate(1).max_roundoff == 0.0  # an integer iteration
+        assert pl.iterate(60).max_roundoff == 0.0  # integer iterations
     with gl.Plan(p, N, autotune=0) as pl:
         assert pl.info.col_variant == -1 and pl.info.row_variant == -1
+
+
+# a device of a given size: cudaMalloc fails beyond it, as it would on a full one
+_MALLOC_SHIM = r"""
+#include <cuda_runtime.h>
+#include <map>
+#include <mutex>
+static std::mutex g_lock;
+static std::map<void*, size_t> g_held;
+static size_t g_used = 0, g_limit = 0;
+extern "C" {
+cudaError_t __real_cudaMalloc(void**, size_t);
+cudaError_t __real_cudaFree(void*);
+void shim_limit(size_t n) { g_limit = n; }
+size_t shim_used() { return g_used; }
+cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
+  std::lock_guard<std::mutex> l(g_lock);
+  if (g_limit && g_used + n > g_limit) return cudaErrorMemoryAllocation;
+  const cudaError_t e = __real_cudaMalloc(p, n);
+  if (e == cudaSuccess) g_used += g_held[*p] = n;
+  return e;
+}
+cudaError_t __wrap_cudaFree(void* p) {
+  std::lock_guard<std::mutex> l(g_lock);
+  g_used -= g_held[p];
+  g_held.erase(p);
+  return __real_cudaFree(p);
+}
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def limited(tmp_path_factory):
+    """The library linked with a cudaMalloc that a test can limit."""
+    d = tmp_path_factory.mktemp("limited")
+    (d / "shim.cu").write_text(_MALLOC_SHIM)
+    objs = [os.path.join(_build.BUILD, os.path.splitext(s)[0] + ".o") for s in _build.SOURCES]
+    if not all(map(os.path.exists, objs)):
+        pytest.skip("the library's object files are not here")
+    subprocess.run([_build.nvcc(), "-c", "-std=c++17", "-Xcompiler", "-fPIC", str(d / "shim.cu"), "-o", str(d / "shim.o")],
+                   check=True)
+    subprocess.run([_build.nvcc(), "-shared"] + _build.ARCH + ["-o", str(d / "limited.so")] + objs +
+                   [str(d / "shim.o"), "-Xlinker", "--wrap=cudaMalloc", "-Xlinker", "--wrap=cudaFree"], check=True)
+    lib = ctypes.CDLL(str(d / "limited.so"))
+    lib.shim_limit.argtypes = [ctypes.c_size_t]
+    lib.shim_used.restype = ctypes.c_size_t
+    lib.gl_iterate.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]
+    return lib
+
+
+@pytest.mark.gpu
+def test_plan_without_room_for_the_integer_tables_runs_fp64(gl, limited):
+    """Device memory for the FP64 form's arrays but not for the integer form's 25 bytes per
+    word beside them: the plan is made, and runs FP64 in every iteration."""
+    p, N, k = 1257787, 65536, 66
+    with gl.Plan(p, N, error_limit=0.39) as ref:
+        need = ref.info.device_bytes
+        ref.iterate(k)
+        want = ref.products()
+    h, info, rep = ctypes.c_void_p(), gl.PlanInfo(), gl.IterReport()
+    out = np.empty(N, np.int64)
+    for limit, fits in ((need + 65536, False), (need + 30 * N, True), (need // 2, None)):
+        limited.shim_limit(limit)
+        rc = limited.gl_plan_create(p, N, None, ctypes.byref(h))
+        if fits is None:
+            assert rc == gl.GL_ERR_NOMEM and limited.shim_used() == 0
+            continue
+        assert rc == 0, (limit, rc)
+        assert limited.gl_plan_get_info(h, ctypes.byref(info)) == 0
+        assert (info.device_bytes > need + 24 * N) == fits and limited.shim_used() == info.device_bytes
+        assert limited.gl_iterate(h, 60, ctypes.byref(rep)) == 0
+        assert (rep.max_roundoff == 0.0) == fits  # an FP64 iteration measures its round-off
+        assert limited.gl_iterate(h, k - 60, ctypes.byref(rep)) == 0
+        assert limited.gl_get_products(h, ctypes.c_void_p(out.ctypes.data)) == 0
+        assert (out == want).all()
+        assert limited.gl_plan_destroy(h) == 0 and limited.shim_used() == 0
+    limited.shim_limit(0)
