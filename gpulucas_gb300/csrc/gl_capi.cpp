@@ -910,6 +910,13 @@ static bool names_fp64_variant(const gl_plan_opts& o) {
          o.row_pass;
 }
 
+// Whether a plan of (p, N) with these options is to run the integer form (where a layout
+// for it is found).
+static bool wants_int_form(int p, int N, const gl_plan_opts& o, int* vmax) {
+  return o.mode == GL_MODE_FUSED && !o.batch_layout && !names_fp64_variant(o) && int_range_ok(p, N, vmax) &&
+         int_roundoff_ok(p, N, o.error_limit);
+}
+
 // Device bytes of the integer form's tables for an H x W layout.
 static size_t int_table_bytes(int H, int W, const IntGeom& g) {
   LinePlan pw = g.pw, ph = g.ph;
@@ -999,8 +1006,7 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   ResidentGeom rg{};
   int vmax = 0;
   // The integer form, unless an option names a variant of the FP64 kernels.
-  bool int_form = o.mode == GL_MODE_FUSED && !fp64_only && !sms_override && !names_fp64_variant(o) &&
-                  int_range_ok(p, N, &vmax) && int_roundoff_ok(p, N, o.error_limit);
+  bool int_form = !fp64_only && !sms_override && wants_int_form(p, N, o, &vmax);
   IntGeom ig{};
   IntVariant int_var;
   IntResidentGeom irg{};
@@ -1259,8 +1265,7 @@ int gl_plan_describe_ex(int p, int N, const gl_plan_opts* opts, gl_plan_info* in
   int cap_c = kMaxRadix, cap_r = kMaxRadix;
   model_caps(tmp.M, o, o.batch_layout ? 1 : 0, &cap_c, &cap_r);
   int vmax = 0;
-  const bool int_form = o.mode == GL_MODE_FUSED && !fp64_only && !o.batch_layout && !names_fp64_variant(o) && int_range_ok(p, N, &vmax) &&
-                        int_roundoff_ok(p, N, o.error_limit);
+  const bool int_form = !fp64_only && wants_int_form(p, N, o, &vmax);
   const int int_h = int_form ? first_int_layout(tmp.M, sms) : 0;
   int rc = o.mode == GL_MODE_FUSED ? choose_fused_geom(tmp.M, int_h ? int_h : o.fft_h, sms, &tmp.fg, cap_c, cap_r)
                                    : choose_plain_geom(tmp.M, &tmp.pg);
@@ -1789,6 +1794,7 @@ int gl_find_signal_size(int p, const gl_plan_opts* opts, int* N_out, double* ms_
   if (opts) o = *opts;
   else gl_default_opts(&o);
   o.mode = GL_MODE_FUSED;
+  const gl_plan_opts want = o;  // the plan that the caller will make
   o.fft_h = 0;
   o.error_limit = 0.5;
   o.check_every = 100;
@@ -1809,16 +1815,29 @@ int gl_find_signal_size(int p, const gl_plan_opts* opts, int* N_out, double* ms_
   double best_ms = 1e300, best_err = 0.0;
   for (int N : cand) {
     if (first && N > first + first / 7) break;  // within ~15 % of the smallest accepted
+    // The trial measures the round-off, in FP64; its own layout search is left out where the
+    // plan will run the integer form.
+    int vmax = 0;
+    const bool integer = wants_int_form(p, N, want, &vmax);
+    gl_plan_opts trial = o;
+    if (integer) trial.autotune = 0;
     gl_plan* pl = nullptr;
-    int rc = gl_plan_create_ex(p, N, &o, o.batch_layout ? 1 : 0, &pl, true);  // measures the round-off
+    int rc = gl_plan_create_ex(p, N, &trial, o.batch_layout ? 1 : 0, &pl, true);
     if (rc == GL_ERR_NOMEM || rc == GL_ERR_NODEVICE || rc == GL_ERR_CUDA) return rc;
     if (rc != GL_OK) continue;
     gl_iter_report rep{};
     rc = gl_iterate(pl, 100, &rep);
+    // ranked by the time of the form the plan will run
     double ms = -1.0;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device);
-    autotune_layout(N / 2, pl->n, sms, 0, &ms);
+    if (integer) {
+      const IntTuned it = autotune_int_layout(N / 2, pl->n, sms, 0);
+      double fp64 = -1.0;
+      if (it.H) autotune_layout(N / 2, pl->n, sms, 0, &fp64, it.H);
+      if (fp64 > 0.0) ms = ((kFp64Every - 1) * it.ms + fp64) / kFp64Every;
+    }
+    if (ms <= 0.0) autotune_layout(N / 2, pl->n, sms, 0, &ms);
     gl_plan_destroy(pl);
     if (rc == GL_ERR_CUDA) return rc;
     if (rc != GL_OK || rep.max_roundoff >= 0.30 || ms <= 0.0) continue;
@@ -1830,8 +1849,18 @@ int gl_find_signal_size(int p, const gl_plan_opts* opts, int* N_out, double* ms_
     }
   }
   if (!best) return GL_ERR_SIZE;
+  if (ms_per_iter) {  // measured on the plan itself: its graphs, its resident form
+    gl_plan* pl = nullptr;
+    gl_iter_report rep{};
+    const int rc = gl_plan_create_ex(p, best, &want, want.batch_layout ? 1 : 0, &pl);
+    if (rc == GL_OK) {
+      gl_iterate(pl, kGraphBatch, &rep);
+      if (gl_iterate(pl, 4 * kGraphBatch, &rep) == GL_OK && rep.ms > 0.0) best_ms = rep.ms / (4 * kGraphBatch);
+      gl_plan_destroy(pl);
+    }
+    *ms_per_iter = best_ms;
+  }
   *N_out = best;
-  if (ms_per_iter) *ms_per_iter = best_ms;
   if (max_roundoff) *max_roundoff = best_err;
   return GL_OK;
 }

@@ -124,9 +124,10 @@ int gl_plan_create(int p, int N, const gl_plan_opts* opts, gl_plan** plan);
 /* findSignalSize (gpuLucas.cu:1064-1187): FFT length for exponent p.  Candidates are the
  * even N with N/2 = 2^a 3^b 5^c 7^d (b <= 5, c <= 3, d <= 2) from the smallest the carry
  * table accepts (p/N < 22) upward; each gets a 100-iteration round-off trial of the real
- * test and is accepted below 0.30 (ERROR_LIMIT, gpuLucas.cu:176); among the accepted ones
- * within 15 % of the smallest, the fastest autotuned iteration wins.  *ms_per_iter and
- * *max_roundoff (either may be NULL) describe the choice. */
+ * test, in FP64, and is accepted below 0.30 (ERROR_LIMIT, gpuLucas.cu:176); among the
+ * accepted ones within 15 % of the smallest, the fastest autotuned iteration of the form that
+ * a plan with these options runs (see gl_iterate) wins.  *ms_per_iter (measured on such a
+ * plan) and *max_roundoff (of the trial) describe the choice; either may be NULL. */
 int gl_find_signal_size(int p, const gl_plan_opts* opts, int* N_out, double* ms_per_iter, double* max_roundoff);
 /* Replaces freeArrays (gpuLucas.cu:1031-1057). */
 int gl_plan_destroy(gl_plan* plan);

@@ -235,3 +235,20 @@ def test_plan_without_room_for_the_integer_tables_runs_fp64(gl, limited):
         assert (out == want).all()
         assert limited.gl_plan_destroy(h) == 0 and limited.shim_used() == 0
     limited.shim_limit(0)
+
+
+@pytest.mark.gpu
+def test_find_signal_size_reports_the_time_of_the_plan_it_describes(gl):
+    """The length is ranked and its time reported for the form that a plan of it runs.  Where
+    that is the integer form, FP64 takes about twice as long at these lengths."""
+    p = 9300017
+    N, ms, err = gl.find_signal_size(p)
+    with gl.Plan(p, N) as pl:
+        integer = pl.iterate(60).max_roundoff == 0.0
+        pl.iterate(64)
+        plan_ms = min(pl.iterate(256).ms for _ in range(3)) / 256
+    assert 0.8 < ms / plan_ms < 1.25 and 0.0 < err < 0.30
+    with gl.Plan(p, N, error_limit=0.39) as pl:
+        pl.iterate(64)
+        fp64_ms = min(pl.iterate(256).ms for _ in range(3)) / 256
+    assert integer and plan_ms < 0.75 * fp64_ms
