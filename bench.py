@@ -60,9 +60,9 @@ def kernel_mads(N: int, W: int, H: int, radix_w, radix_h) -> dict:
 
     pair = (6 * 4 + 16) / 2.0  # three squares of two products, one twiddle product, per two points
     return {
-        "k_col_fwd": M * (line(radix_h) + 16.0),
-        "k_row_sq": M * (2 * line(radix_w) + pair + 16.0),
-        "k_col_inv": M * line(radix_h),
+        "ki_col_fwd": M * (line(radix_h) + 16.0),
+        "ki_row_sq": M * (2 * line(radix_w) + pair + 16.0),
+        "ki_col_inv": M * line(radix_h),
     }
 
 
@@ -301,15 +301,11 @@ def run_ours(args, world: int, rank: int, local: int):
     # per-kernel device time and the roofline of the dominant kernel
     prof = plan.profile_kernels(30)
     dom = max(prof, key=prof.get)
-    # the integer form's line plans: powers of two first, then 3
-    def plan_of(n):
-        out = []
-        for r in (8, 4, 2, 3, 5, 7):
-            while n % r == 0:
-                out.append(r)
-                n //= r
-        return out
-    km = kernel_mads(N3, info.fft_w, info.fft_h, plan_of(info.fft_w), plan_of(info.fft_h))
+    form = plan.int_info  # without it the operation counts below would be of kernels that did not run
+    if not form.integer:
+        raise RuntimeError("the plan runs FP64 in every iteration (no device memory for the integer form's tables?)")
+    radix_w, radix_h = [r for r in form.radix_w if r], [r for r in form.radix_h if r]
+    km = kernel_mads(N3, info.fft_w, info.fft_h, radix_w, radix_h)
     sm_hz = 1e6 * (clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 2070.0)
     mad_peak = MAD64_PER_CLOCK_SM * SMS * sm_hz / 1e12
     achieved = km[dom] / (prof[dom] * 1e-3) / 1e12
@@ -361,14 +357,15 @@ def run_ours(args, world: int, rank: int, local: int):
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": total_ms_max / args.steps,
         "higher_is_better": True, "scaling": "weak",
         "vs_baseline": value / REF_PUBLISHED_ITER_S / world,
-        "dtype": "exact 61-bit integers (GF((2^61-1)^2)), one iteration in 64 in f64",
+        "dtype": f"exact 61-bit integers (GF((2^61-1)^2)), one iteration in {form.fp64_every} in f64",
         "data": "synthetic: the LL sequence from S0=4 (no dataset)",
         "config": {"workload": WORKLOAD,
                    "p": P3, "N": N3, "fft": f"{info.fft_h} x {info.fft_w}", "parallelism": "replicas",
-                   "layout": {"radix_h": [r for r in info.radix_h if r], "radix_w": [r for r in info.radix_w if r],
-                              "column_variant": info.col_variant, "row_variant": info.row_variant,
-                              "threads_col": info.threads_col,
-                              "threads_row": info.threads_row},
+                   "layout": {"radix_h": radix_h, "radix_w": radix_w, "columns_in_place": bool(form.col_inplace),
+                              "threads_col": form.threads_col, "threads_row": form.threads_row,
+                              "fp64": {"every": form.fp64_every, "radix_h": [r for r in info.radix_h if r],
+                                       "radix_w": [r for r in info.radix_w if r],
+                                       "column_variant": info.col_variant, "row_variant": info.row_variant}},
                    "l2": "flushed before every timed step (512 MiB write); the test's ~227 MB of state and "
                          "tables exceed the 129 MB L2 anyway",
                    "vs_baseline_note": "reference's published 204.72 iter/s at N=2359296 (GTX 480/C2050)"},
@@ -565,7 +562,7 @@ def served_leg(gl, dev: int, window: int) -> dict:
 
 
 def plan_launches(gl) -> int:
-    return 3  # fused form: k_col_fwd, k_row_sq, k_col_inv per iteration
+    return 3  # fused form: ki_col_fwd, ki_row_sq, ki_col_inv per iteration (k_* where in FP64)
 
 
 def main():

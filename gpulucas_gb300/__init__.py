@@ -59,6 +59,14 @@ class PlanInfo(ctypes.Structure):
                 ("row_variant", ctypes.c_int)]
 
 
+class IntInfo(ctypes.Structure):
+    """The integer form of a plan (all zero: FP64 in every iteration)."""
+    _fields_ = [("integer", ctypes.c_int), ("fp64_every", ctypes.c_int), ("poly", ctypes.c_int),
+                ("col_inplace", ctypes.c_int), ("radix_w", ctypes.c_int * 8), ("radix_h", ctypes.c_int * 8),
+                ("threads_col", ctypes.c_int), ("threads_row", ctypes.c_int), ("smem_col", ctypes.c_int),
+                ("smem_row", ctypes.c_int), ("resident_ctas", ctypes.c_int), ("resident_smem", ctypes.c_int)]
+
+
 class BatchInfo(ctypes.Structure):
     _fields_ = [("ntests", ctypes.c_int), ("col_units", ctypes.c_int), ("row_units", ctypes.c_int),
                 ("threads_col", ctypes.c_int), ("threads_row", ctypes.c_int), ("smem_col", ctypes.c_int),
@@ -140,6 +148,7 @@ def _load():
         "gl_plan_create": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.POINTER(PlanOpts), PP]),
         "gl_plan_destroy": (ctypes.c_int, [P]),
         "gl_plan_get_info": (ctypes.c_int, [P, ctypes.POINTER(PlanInfo)]),
+        "gl_plan_int_info": (ctypes.c_int, [P, ctypes.POINTER(IntInfo)]),
         "gl_plan_describe": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.POINTER(PlanOpts),
                                             ctypes.POINTER(PlanInfo)]),
         "gl_reset": (ctypes.c_int, [P]),
@@ -215,7 +224,7 @@ lib = _load()
 
 # exported C symbols that include/gpulucas.h declares (checked by the tests)
 ABI_SYMBOLS = tuple(sorted([
-    "gl_default_opts", "gl_plan_create", "gl_plan_destroy", "gl_plan_get_info", "gl_plan_describe",
+    "gl_default_opts", "gl_plan_create", "gl_plan_destroy", "gl_plan_get_info", "gl_plan_int_info", "gl_plan_describe",
     "gl_reset", "gl_iterate",
     "gl_plan_stream", "gl_enqueue", "gl_sync_status", "gl_launches_per_iteration", "gl_profile_kernels",
     "gl_get_products",
@@ -312,6 +321,12 @@ class Plan:
         return rep
 
     @property
+    def int_info(self) -> IntInfo:
+        info = IntInfo()
+        _check(lib.gl_plan_int_info(self._h, ctypes.byref(info)), "plan integer form")
+        return info
+
+    @property
     def stream(self) -> int:
         s = ctypes.c_void_p()
         _check(lib.gl_plan_stream(self._h, ctypes.byref(s)), "stream")
@@ -322,7 +337,7 @@ class Plan:
         return _check(lib.gl_launches_per_iteration(self._h), "launches")
 
     def profile_kernels(self, iters: int = 10) -> dict:
-        """Average ms per launch of each fused kernel (events between launches)."""
+        """Average ms per launch of each of the plan's kernels, by name (events between launches)."""
         ms = (ctypes.c_double * 3)()
         names = (ctypes.c_char_p * 3)()
         nk = ctypes.c_int()

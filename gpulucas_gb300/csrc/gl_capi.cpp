@@ -1321,6 +1321,24 @@ int gl_plan_get_info(const gl_plan* pl, gl_plan_info* info) {
   return GL_OK;
 }
 
+int gl_plan_int_info(const gl_plan* pl, gl_int_info* info) {
+  if (!pl || !info) return GL_ERR_ARG;
+  std::memset(info, 0, sizeof(*info));
+  if (!pl->int_form) return GL_OK;
+  const IntGeom& g = pl->ig;
+  info->integer = 1;
+  info->fp64_every = kFp64Every;
+  info->poly = g.t;
+  info->col_inplace = g.col_p;
+  for (int i = 0; i < g.pw.nst; ++i) info->radix_w[i] = g.pw.radix[i];
+  for (int i = 0; i < g.ph.nst; ++i) info->radix_h[i] = g.ph.radix[i];
+  info->threads_col = g.t_col; info->threads_row = g.t_row;
+  info->smem_col = (int)g.sm_col; info->smem_row = (int)g.sm_row;
+  info->resident_ctas = pl->resident ? pl->irg.C : 0;
+  info->resident_smem = pl->resident ? pl->irg.smem : 0;
+  return GL_OK;
+}
+
 int gl_reset(gl_plan* pl) {
   if (!pl) return GL_ERR_ARG;
   GL_CUDA(cudaSetDevice(pl->device));
@@ -1417,7 +1435,8 @@ int gl_profile_kernels(gl_plan* pl, int iters, double* ms_out, const char** name
   if (!pl || !ms_out || iters < 1) return GL_ERR_ARG;
   if (pl->mode != GL_MODE_FUSED) return GL_ERR_STATE;
   GL_CUDA(cudaSetDevice(pl->device));
-  static const char* kNames[3] = {"k_col_fwd", "k_row_sq", "k_col_inv"};
+  static const char* const kFp64Names[3] = {"k_col_fwd", "k_row_sq", "k_col_inv"};
+  static const char* const kIntNames[3] = {"ki_col_fwd", "ki_row_sq", "ki_col_inv"};
   if (pl->from_state) {  // consume a pending state load first
     int rc = launch_iterations(pl, 1);
     if (rc != GL_OK) return rc;
@@ -1450,7 +1469,7 @@ int gl_profile_kernels(gl_plan* pl, int iters, double* ms_out, const char** name
   pl->carry_valid = false;
   for (int k = 0; k < 3; ++k) {
     ms_out[k] = acc[k] / iters;
-    if (names) names[k] = kNames[k];
+    if (names) names[k] = !pl->int_form ? kFp64Names[k] : k == 1 && pl->ig.t > 1 ? "ki_row_poly" : kIntNames[k];
   }
   if (nk) *nk = 3;
   return GL_OK;

@@ -88,13 +88,27 @@ typedef struct {
     int threads_col, threads_row;  /* CTA sizes of the column and row passes */
     int smem_col, smem_row;        /* dynamic shared memory bytes of those passes */
     size_t device_bytes;   /* device memory held by the plan */
-    int resident_ctas;     /* CTAs of the resident form's cluster, 0 if not used */
+    int resident_ctas;     /* CTAs of the FP64 resident form's cluster, 0 if not used */
     int resident_smem;     /* its shared memory per CTA */
     int col_variant;       /* fused form: the column passes as a col_inplace value (-1 two
                               buffers, 1 in place, 2 + prefetched weights, 3 two columns per
                               CTA, 4 two columns forward + prefetched weights inverse) */
     int row_variant;       /* fused form: the row pass as a row_pass value (-1, 1, 2) */
-} gl_plan_info;
+} gl_plan_info;            /* (layout and CTAs of the FP64 form; gl_int_info has the other's) */
+
+typedef struct {
+    int integer;           /* 1: the plan has the integer form (see gl_iterate); 0: FP64 in every
+                              iteration, and the fields below are 0 */
+    int fp64_every;        /* one iteration in this many runs in FP64 */
+    int poly;              /* length of the polynomials transformed: 1, or the part of N/2 that
+                              the field has no roots for */
+    int col_inplace;       /* 1: column passes with in-place line DFTs */
+    int radix_w[8], radix_h[8];    /* line plans of fft_w / poly and of fft_h points */
+    int threads_col, threads_row;  /* CTA sizes of the column and row passes */
+    int smem_col, smem_row;        /* dynamic shared memory bytes of those passes */
+    int resident_ctas;     /* CTAs of the resident form's cluster, 0 if not used */
+    int resident_smem;     /* its shared memory per CTA */
+} gl_int_info;
 
 typedef struct {
     int64_t iterations;    /* iterations done by this call */
@@ -132,6 +146,8 @@ int gl_find_signal_size(int p, const gl_plan_opts* opts, int* N_out, double* ms_
 /* Replaces freeArrays (gpuLucas.cu:1031-1057). */
 int gl_plan_destroy(gl_plan* plan);
 int gl_plan_get_info(const gl_plan* plan, gl_plan_info* info);
+/* Which form the plan's iterations run in, and the integer form's geometry. */
+int gl_plan_int_info(const gl_plan* plan, gl_int_info* info);
 /* The layout gl_plan_create would choose for (p, N, opts), without touching a GPU. */
 int gl_plan_describe(int p, int N, const gl_plan_opts* opts, gl_plan_info* info);
 
@@ -157,8 +173,9 @@ int gl_sync_status(gl_plan* plan, gl_iter_report* report);
 /* kernel launches one iteration issues (3 for the fused form) */
 int gl_launches_per_iteration(const gl_plan* plan);
 /* Fused form only: run `iters` iterations launching each kernel between CUDA events
- * on the plan's stream; ms_out[i] = average ms of kernel i (k_col_fwd, k_row_sq,
- * k_col_inv); names (may be NULL) receives their names, *nk the count. */
+ * on the plan's stream; ms_out[i] = average ms of kernel i: k_col_fwd, k_row_sq, k_col_inv,
+ * or of a plan with the integer form ki_col_fwd, ki_row_sq (ki_row_poly), ki_col_inv;
+ * names (may be NULL) receives their names, *nk the count. */
 int gl_profile_kernels(gl_plan* plan, int iters, double* ms_out, const char** names, int* nk);
 
 /* The state after the last iteration. */

@@ -252,3 +252,67 @@ def test_find_signal_size_reports_the_time_of_the_plan_it_describes(gl):
         pl.iterate(64)
         fp64_ms = min(pl.iterate(256).ms for _ in range(3)) / 256
     assert integer and plan_ms < 0.75 * fp64_ms
+
+
+def test_int_info_layout_matches_header(tmp_path, gl):
+    lines = ["#include <stdio.h>", "#include <stddef.h>", '#include "gpulucas.h"', "int main(void) {",
+             'printf("%zu\\n", sizeof(gl_int_info));']
+    names = [n for n, _ in gl.IntInfo._fields_]
+    lines += [f'printf("%zu\\n", offsetof(gl_int_info, {n}));' for n in names] + ["return 0; }"]
+    (tmp_path / "l.c").write_text("\n".join(lines))
+    subprocess.run(["gcc", "-std=c11", "-I", os.path.join(ROOT, "include"), str(tmp_path / "l.c"), "-o",
+                    str(tmp_path / "l")], check=True)
+    got = [int(x) for x in subprocess.run([str(tmp_path / "l")], check=True, capture_output=True, text=True).stdout.split()]
+    assert got == [ctypes.sizeof(gl.IntInfo)] + [getattr(gl.IntInfo, n).offset for n in names]
+
+
+# every length that tests/test_int_form.py and the test below compare, with the polynomial length of its integer
+# form and whether the resident form runs it
+_INTEGER = [(100003, 5120, 1, 0), (100003, 6272, 7, 0), (90007, 5600, 1, 0), (1000003, 53760, 1, 0),
+            (859433, 49152, 1, 0), (859433, 50400, 1, 0), (2976221, 163840, 1, 0), (2976221, 201600, 1, 0),
+            (1398269, 86016, 1, 0), (9300017, 524288, 1, 0), (20996011, 1179648, 1, 0), (24000001, 1310720, 1, 0),
+            (74207281, 4194304, 1, 0), (100003, 5184, 9, 0), (500009, 27648, 3, 0), (300007, 16000, 5, 0),
+            (748003, 44100, 7, 0), (300007, 16200, 9, 0), (1000003, 52500, 25, 0), (1000003, 54432, 27, 0),
+            (1500007, 78400, 7, 0), (800011, 43904, 49, 0),
+            (1257787, 65536, 1, 0), (9689, 512, 1, 1), (21701, 1024, 1, 1),
+            (33013, 1536, 1, 1), (44497, 2048, 1, 1), (60013, 3072, 1, 1), (86243, 4096, 1, 1), (76003, 3840, 1, 1)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,N,t,resident", _INTEGER)
+def test_the_lengths_compared_run_the_integer_form(gl, p, N, t, resident):
+    """A silent fall back to FP64 would pass every comparison of products.  Both by what the
+    plan says and by what it does: 60 iterations without a round-off, against some in FP64."""
+    for opts in ({}, {"autotune": 0}) if N < 100000 else ({"autotune": 0},):
+        with gl.Plan(p, N, **opts) as pl:
+            f = pl.int_info
+            assert f.integer == 1 and f.fp64_every == 64 and f.poly == t and bool(f.resident_ctas) == bool(resident)
+            V, H = pl.info.fft_w // t, pl.info.fft_h
+            assert np.prod([r for r in f.radix_w if r]) == V and np.prod([r for r in f.radix_h if r]) == H
+            assert f.threads_col and f.threads_row and f.smem_col and f.smem_row
+            assert pl.iterate(60).max_roundoff == 0.0 and pl.iterate(4).max_roundoff > 0.0
+            row = "ki_row_poly" if t > 1 else "ki_row_sq"
+            assert list(pl.profile_kernels(1)) == ["ki_col_fwd", row, "ki_col_inv"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("opts", [{"error_limit": 0.39}, {"fft_h": 64}, {"batch_layout": 1}, {"col_inplace": -1}])
+def test_options_that_keep_a_plan_in_fp64_say_so(gl, opts):
+    with gl.Plan(100003, 5120, **opts) as pl:
+        f = pl.int_info
+        assert not f.integer and not f.fp64_every and not f.threads_col
+        assert pl.iterate(60).max_roundoff > 0.0
+        assert list(pl.profile_kernels(1)) == ["k_col_fwd", "k_row_sq", "k_col_inv"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p,N", [(800011, 43904), (45878401, 2592000)])
+def test_longest_polynomials_equal_fp64_form(gl, orc, p, N):
+    """t = 49 and 45 (odd parts 7^3 and 3^4 5^3), the longest that the integer form takes."""
+    for k in (1, 66):
+        with gl.Plan(p, N) as a, gl.Plan(p, N, error_limit=0.39) as b:
+            assert a.int_info.poly in (45, 49) and not b.int_info.integer
+            a.iterate(k)
+            b.iterate(k)
+            assert (a.products() == b.products()).all(), k
+            assert k == 1 or p > 1000000 or a.res64() == orc.Exact(p).iterate(k).res64()
