@@ -340,9 +340,16 @@ int int_stage_offsets(LinePlan* lp) {
 
 // Largest polynomial length (gf_excess) the integer form is used at.  Squaring takes about
 // t/2 products per coefficient, but a test alone waits on latencies more than it computes
-// (us per iteration, integer/FP64: N = 44100, t = 7, 25.2/35.5; 52500, 25, 29.4/35.8;
-// 54432, 27, 30.5/31.6; 78400, 49, 27.8/39.5).
+// (us per iteration, integer/FP64: t = 7, N = 44100, 24.9/35.2, 78400, 26.1/39.2; t = 25,
+// 52500, 27.0/35.7; t = 27, 54432, 28.8/31.6, 62208, 28.0/27.0, 124416, 29.7/32.9, 995328,
+// 96.8/140; t = 35, 98000, 34.3/43.1; t = 49, 43904, 28.7/34.6, 351232, 68.2/75.6).
 constexpr int kMaxIntPoly = 49;
+// Longer polynomials than this pay at some lengths only (t = 45: 40500, 28.3/30.5; 81000,
+// 36.0/33.5; 324000, 74.3/65.9; 648000, 123/117; 1296000, 211/223; 2592000, 386/434; t = 49:
+// 82320, 37.6/40.1; 98784, 43.8/39.7; 137200, 49.2/47.5), so there both forms are timed; from
+// 2^14 points, since below launches take most of either's time and the integer form is faster.
+constexpr int kMaxSurePoly = 27;
+constexpr int kMinTimedFormM = 1 << 14;
 
 // Geometry of the integer form on an H x W layout; false where its polynomials do not fit
 // the rows or a CTA's lines its shared memory.
@@ -390,6 +397,13 @@ IntVariant untimed_variant(int H, int W) {
     if (!choose_int_geom(H, W, &g, v)) v.in_place = false;
   }
   return v;
+}
+
+// Whether the integer form is worth its while at M points, where nothing is timed: not at
+// t = 45 (see kMaxSurePoly; the FP64 form's radices 3 and 5 lose little there) below 2^19.
+bool int_pays_untimed(int M) {
+  const int t = gf_excess(M);
+  return t <= kMaxSurePoly || t % 7 == 0 || M < kMinTimedFormM || M >= (1 << 19);
 }
 
 // Column length of the first layout of the cost model that the integer form can run, or 0.
@@ -696,6 +710,19 @@ IntTuned autotune_int_layout(int M, int n, int sms, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   g_int_tune_cache[{M, sms}] = best;
   return best;
+}
+
+// The integer form's layout for a plan whose layouts are timed; H = 0 where the FP64 form is
+// faster.  The forms are compared as launched one by one; 3 % is what the FP64 form gains more
+// from a captured graph at most.
+IntTuned timed_int_layout(int M, int n, int sms, cudaStream_t s) {
+  IntTuned it = autotune_int_layout(M, n, sms, s);
+  if (it.H && M >= kMinTimedFormM && gf_excess(M) > kMaxSurePoly) {
+    double fp64 = -1.0;
+    autotune_layout(M, n, sms, s, &fp64);
+    if (fp64 > 0.0 && fp64 < 0.97 * it.ms) it.H = 0;
+  }
+  return it;
 }
 
 void free_plan(gl_plan* pl) {
@@ -1053,8 +1080,8 @@ int gl_plan_create_ex(int p, int N, const gl_plan_opts* opts, int sms_override, 
   if (o.resident > 0 && !resident) return GL_ERR_SIZE;
   if (int_form && !resident) {
     IntTuned it;
-    if (o.autotune && !sms_override) it = autotune_int_layout(M, n, sms, 0);
-    else {
+    if (o.autotune && !sms_override) it = timed_int_layout(M, n, sms, 0);
+    else if (int_pays_untimed(M)) {
       it.H = first_int_layout(M, sms);
       if (it.H) it.var = untimed_variant(it.H, M / it.H);
     }
@@ -1266,7 +1293,7 @@ int gl_plan_describe_ex(int p, int N, const gl_plan_opts* opts, gl_plan_info* in
   model_caps(tmp.M, o, o.batch_layout ? 1 : 0, &cap_c, &cap_r);
   int vmax = 0;
   const bool int_form = !fp64_only && wants_int_form(p, N, o, &vmax);
-  const int int_h = int_form ? first_int_layout(tmp.M, sms) : 0;
+  const int int_h = int_form && int_pays_untimed(tmp.M) ? first_int_layout(tmp.M, sms) : 0;
   int rc = o.mode == GL_MODE_FUSED ? choose_fused_geom(tmp.M, int_h ? int_h : o.fft_h, sms, &tmp.fg, cap_c, cap_r)
                                    : choose_plain_geom(tmp.M, &tmp.pg);
   if (rc != GL_OK) return rc;
@@ -1851,7 +1878,7 @@ int gl_find_signal_size(int p, const gl_plan_opts* opts, int* N_out, double* ms_
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device);
     if (integer) {
-      const IntTuned it = autotune_int_layout(N / 2, pl->n, sms, 0);
+      const IntTuned it = timed_int_layout(N / 2, pl->n, sms, 0);
       double fp64 = -1.0;
       if (it.H) autotune_layout(N / 2, pl->n, sms, 0, &fp64, it.H);
       if (fp64 > 0.0) ms = ((kFp64Every - 1) * it.ms + fp64) / kFp64Every;

@@ -316,3 +316,17 @@ def test_longest_polynomials_equal_fp64_form(gl, orc, p, N):
             b.iterate(k)
             assert (a.products() == b.products()).all(), k
             assert k == 1 or p > 1000000 or a.res64() == orc.Exact(p).iterate(k).res64()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [81000, 98784, 162000, 324000])
+def test_plans_run_fp64_where_it_is_faster(gl, N):
+    """Long polynomials (t = 45, 49) at lengths where the FP64 form takes 5 to 12 % less: the
+    plan runs it, as a plan that may not run the other does."""
+    p = int(18.3 * N) | 1
+    ms = []
+    for limit in (0.4, 0.39):
+        with gl.Plan(p, N, error_limit=limit) as pl:
+            pl.iterate(64, check=False)
+            ms.append(min(pl.iterate(256, check=False).ms for _ in range(3)) / 256)
+    assert ms[0] < 1.03 * ms[1]
