@@ -157,6 +157,7 @@ struct ResidentGeom {
   int twH_n, twW_n;
 };
 constexpr int kResidentThreads = 256;
+constexpr int kResidentSmem = 200 * 1024;  // shared memory per CTA, at most
 constexpr int kResidentMaxN = 32768;   // largest N the resident form is tried at (opts.resident = 1)
 constexpr int kResidentAutoN = 4096;   // used by default up to here: measured faster than the
                                        // three-launch form (13.8 vs 18.3 us at N = 2048, 16.1 vs

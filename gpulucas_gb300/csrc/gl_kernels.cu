@@ -1294,8 +1294,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 template <int NC>
-static cudaError_t resident_attrs(int smem, int C, cudaLaunchConfig_t* cfg, int* clusters) {
-  cudaError_t e = cudaFuncSetAttribute(k_resident<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+static cudaError_t resident_attrs(int C, cudaLaunchConfig_t* cfg, int* clusters) {
+  // process-wide: the layouts' common bound, not this one's size, which would take room from
+  // the plans made before it
+  cudaError_t e = cudaFuncSetAttribute(k_resident<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem);
   if (e != cudaSuccess) return e;
   if (C > 8 && (e = cudaFuncSetAttribute(k_resident<NC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) !=
                    cudaSuccess)
@@ -1316,11 +1318,11 @@ static cudaError_t resident_fits(int n, int smem, int C, int* clusters) {
   cfg.attrs = at;
   cfg.numAttrs = 1;
   switch (n) {
-    case 2: return resident_attrs<2>(smem, C, &cfg, clusters);
-    case 3: return resident_attrs<3>(smem, C, &cfg, clusters);
-    case 4: return resident_attrs<4>(smem, C, &cfg, clusters);
-    case 5: return resident_attrs<5>(smem, C, &cfg, clusters);
-    default: return resident_attrs<6>(smem, C, &cfg, clusters);
+    case 2: return resident_attrs<2>(C, &cfg, clusters);
+    case 3: return resident_attrs<3>(C, &cfg, clusters);
+    case 4: return resident_attrs<4>(C, &cfg, clusters);
+    case 5: return resident_attrs<5>(C, &cfg, clusters);
+    default: return resident_attrs<6>(C, &cfg, clusters);
   }
 }
 
@@ -1357,7 +1359,7 @@ cudaError_t resident_geom(const FusedGeom& fg, int twH_n, int twW_n, int n, Resi
     g.o_K2 = take((size_t)2 * g.npl * W * 16);
     g.o_twH = take((size_t)twH_n * 16);
     g.o_twW = take((size_t)twW_n * 16);
-    if (o > (size_t)200 * 1024) continue;
+    if (o > (size_t)kResidentSmem) continue;
     g.smem = (int)o;
     int clusters = 0;
     if (resident_fits(n, g.smem, C, &clusters) != cudaSuccess) {

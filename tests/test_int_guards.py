@@ -330,3 +330,15 @@ def test_plans_run_fp64_where_it_is_faster(gl, N):
             pl.iterate(64, check=False)
             ms.append(min(pl.iterate(256, check=False).ms for _ in range(3)) / 256)
     assert ms[0] < 1.03 * ms[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("first,second", [((86243, 4096, 0.4), (9689, 512, 0.4)), ((76003, 3840, 0.4), (76003, 3840, 0.39)),
+                                          ((44497, 2048, 0.39), (21701, 1024, 0.39))])
+def test_a_resident_plan_runs_on_after_a_smaller_one_is_made(gl, orc, first, second):
+    """The resident kernels' shared-memory limit is the process's, not a plan's."""
+    p, N, limit = first
+    with gl.Plan(p, N, error_limit=limit) as a, gl.Plan(second[0], second[1], error_limit=second[2]) as b:
+        assert a.info.resident_ctas and b.info.resident_ctas
+        a.iterate(70)
+        assert (a.products() == orc.IBDWT(p, N).iterate(70).ll()).all()
