@@ -713,15 +713,37 @@ IntTuned autotune_int_layout(int M, int n, int sms, cudaStream_t s) {
 }
 
 // The integer form's layout for a plan whose layouts are timed; H = 0 where the FP64 form is
-// faster.  The forms are compared as launched one by one; 3 % is what the FP64 form gains more
-// from a captured graph at most.
+// faster.  The forms are compared as launched one by one, each search's winner timed three
+// times more (a search times a variant once or a few times, and a hiccup of the host is 3 %);
+// 2 % is what the FP64 form gains more from a captured graph at most.  Once per (M, SM count)
+// per process.
+std::map<std::pair<int, int>, bool> g_fp64_faster;
 IntTuned timed_int_layout(int M, int n, int sms, cudaStream_t s) {
   IntTuned it = autotune_int_layout(M, n, sms, s);
-  if (it.H && M >= kMinTimedFormM && gf_excess(M) > kMaxSurePoly) {
-    double fp64 = -1.0;
-    autotune_layout(M, n, sms, s, &fp64);
-    if (fp64 > 0.0 && fp64 < 0.97 * it.ms) it.H = 0;
+  if (!it.H || M < kMinTimedFormM || gf_excess(M) <= kMaxSurePoly) return it;
+  {
+    std::lock_guard<std::mutex> lock(g_tune_mutex);
+    auto known = g_fp64_faster.find({M, sms});
+    if (known != g_fp64_faster.end()) {
+      if (known->second) it.H = 0;
+      return it;
+    }
   }
+  const TunedLayout t = autotune_layout(M, n, sms, s, nullptr);
+  if (!t.H) return it;
+  const int iters = M >= (1 << 18) ? 10 : 40;
+  SearchBuffers sb;
+  double fp64 = t.ms, integer = it.ms;
+  for (int i = 0; i < 3; ++i) {
+    const double f = time_layout(M, t.H, t.rc, t.rr, t.ip, t.pf, t.ws, t.row, n, sms, iters, sb, s);
+    if (f > 0.0 && f < fp64) fp64 = f;
+    const double k = time_int_layout(M, it.H, it.var, n, iters, 1e300, sb, s);
+    if (k > 0.0 && k < integer) integer = k;
+  }
+  const bool faster = fp64 < 0.98 * integer;
+  if (faster) it.H = 0;
+  std::lock_guard<std::mutex> lock(g_tune_mutex);
+  g_fp64_faster[{M, sms}] = faster;
   return it;
 }
 
