@@ -415,8 +415,8 @@ int gl_server_destroy(gl_server* server);
  * loads the library until exit; the driver loads a kernel's code when it is first launched,
  * 4 to 6 MiB with a process's first call); larger N returns GL_ERR_TOO_LARGE.  A call with new
  * (p, N) uploads that test's tables into the array first; the integer form's are built in
- * host memory, with the test's first call of two iterations or more (GL_ERR_NOMEM if there
- * is none).  The call is synchronous: it returns after `stream` has finished the
+ * host memory (GL_ERR_NOMEM if there is none) once the test has asked for max(2, N/1024)
+ * iterations, and all iterations before run in FP64.  The call is synchronous: it returns after `stream` has finished the
  * iterations, so it cannot be captured into a CUDA graph (on a stream that is capturing it
  * returns GL_ERR_ARG and enqueues nothing).  All calls share the array; a lock held until
  * the stream has finished keeps the calls of one process from overlapping on the GPU.

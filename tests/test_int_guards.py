@@ -99,9 +99,11 @@ rc, a = call(*A, 5)                 # B's FP64 tables had replaced A's
 assert rc == 0 and (a == want(*A, 5)).all()
 rc, b = call(*B, 5)
 assert rc == 0 and (b == want(*B, 5)).all()
-for k in (0, 1):                    # too short for the integer form: no tables of it
+for k in (0, 1, 2):                 # N/1024 iterations pay for the integer form's tables
     rc, c = call(*C, k, 4096)
     assert rc == 0 and (k == 0 or (c == want(*C, k)).all()), (k, rc)
+rc, c = call(*C, 2, 4096)
+assert rc == gl.GL_ERR_NOMEM, rc
 rc, c = call(*C, 5)
 assert rc == 0 and (c == want(*C, 5)).all()
 print("done")
