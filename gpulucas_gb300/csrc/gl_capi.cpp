@@ -985,10 +985,10 @@ static int build_int_tables(gl_plan* pl, int vmax) {
   gf_pass_tables(W, H, t, k1, pair, k2);
   gf_row_pairs(V, H, rows);
   gf_weights(pl->p, N, e);
-  gf_stage_twiddles(V, pl->ig.pw.radix, pl->ig.pw.nst, false, wf, off);
-  gf_stage_twiddles(V, pl->ig.pw.radix, pl->ig.pw.nst, true, wi, off);
-  gf_stage_twiddles(H, pl->ig.ph.radix, pl->ig.ph.nst, false, hf, off);
-  gf_stage_twiddles(H, pl->ig.ph.radix, pl->ig.ph.nst, true, hi, off);
+  gf_stage_twiddles(pl->ig.pw.radix, pl->ig.pw.nst, false, wf, off);
+  gf_stage_twiddles(pl->ig.pw.radix, pl->ig.pw.nst, true, wi, off);
+  gf_stage_twiddles(pl->ig.ph.radix, pl->ig.ph.nst, false, hf, off);
+  gf_stage_twiddles(pl->ig.ph.radix, pl->ig.ph.nst, true, hi, off);
   for (int m1 = 0, c = 0; m1 < W; ++m1)  // column-major, as the other per-word tables
     for (int m2 = 0; m2 < H; ++m2, c += 2) {
       e_c[c] = e[2 * (m1 + (size_t)W * m2)];

@@ -235,7 +235,7 @@ template <int S>
 void gf_line(g2* x, int st, int L, const std::vector<int>& radices, int64_t* peak) {
   std::vector<gl::HostTw> tw;
   std::vector<int> off(radices.size() + 1);
-  gl::gf_stage_twiddles(L, radices.data(), (int)radices.size(), S > 0, tw, off.data());
+  gl::gf_stage_twiddles(radices.data(), (int)radices.size(), S > 0, tw, off.data());
   std::vector<g2> a((size_t)L), b((size_t)L);
   for (int i = 0; i < L; ++i) a[i] = x[(size_t)i * st];
   int Ns = 1;

@@ -118,10 +118,10 @@ void build_int_tables(int p, int N, int n) {
   gf_weights(p, N, e);
   int off[8];
   const LinePlan &pw = h_int.g.pw, &ph = h_int.g.ph;
-  gf_stage_twiddles(V, pw.radix, pw.nst, false, h_int.stages[0], off);
-  gf_stage_twiddles(V, pw.radix, pw.nst, true, h_int.stages[1], off);
-  gf_stage_twiddles(H, ph.radix, ph.nst, false, h_int.stages[2], off);
-  gf_stage_twiddles(H, ph.radix, ph.nst, true, h_int.stages[3], off);
+  gf_stage_twiddles(pw.radix, pw.nst, false, h_int.stages[0], off);
+  gf_stage_twiddles(pw.radix, pw.nst, true, h_int.stages[1], off);
+  gf_stage_twiddles(ph.radix, ph.nst, false, h_int.stages[2], off);
+  gf_stage_twiddles(ph.radix, ph.nst, true, h_int.stages[3], off);
   for (const auto& s : h_int.stages)
     if (s.size() > (size_t)kNoAllocMaxLine) return;
   if (h_int.rows.size() > (size_t)kNoAllocMaxLine) return;

@@ -401,6 +401,8 @@ int64_t inv_mod(int64_t a, int64_t m) {
   return 0;  // m == 1
 }
 
+// exp(-2 pi i t / L)'s counterpart: a multiplicative family of roots of unity (root(t, L)
+// root(u, L) = root(t + u, L), root(t k, L k) = root(t, L)), as c + i d with 0 <= c, d < q
 Gf groot(int64_t t, int64_t L) {
   static const Pow2Roots pr;
   t %= L;
@@ -442,18 +444,12 @@ int gf_excess(int M) {
   return t;
 }
 
-void gf_root(int64_t t, int64_t L, uint64_t* c, uint64_t* d) {
-  const Gf w = groot(t, L);
-  *c = w.re;
-  *d = w.im;
-}
-
 HostTw gf_pack(uint64_t c, uint64_t d) {
   const gf::Limbs a = gf::limbs(c), b = gf::limbs(d);
   return {a.c0, a.c1, b.c0, b.c1};
 }
 
-void gf_stage_twiddles(int L, const int* radices, int nst, bool inverse, std::vector<HostTw>& tw, int* off) {
+void gf_stage_twiddles(const int* radices, int nst, bool inverse, std::vector<HostTw>& tw, int* off) {
   tw.assign(1, HostTw{1, 0, 0, 0});
   int Ns = 1;
   for (int s = 0; s < nst; ++s) {
@@ -471,7 +467,6 @@ void gf_stage_twiddles(int L, const int* radices, int nst, bool inverse, std::ve
     }
     Ns *= R;
   }
-  (void)L;
 }
 
 void gf_pass_tables(int W, int H, int t, std::vector<HostTw>& k1, std::vector<HostTw>& pair,

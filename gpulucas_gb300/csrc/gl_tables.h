@@ -72,13 +72,13 @@ struct HostTw {
 // y^t - root(k, M/t).  Returns t (1: a plain transform).  N = 2 M is prime to 61, so the
 // weights are powers of two.
 int gf_excess(int M);
-// exp(-2 pi i t / L)'s counterpart: a multiplicative family of roots of unity (root(t, L)
-// root(u, L) = root(t + u, L), root(t k, L k) = root(t, L)), as c + i d with 0 <= c, d < q
-void gf_root(int64_t t, int64_t L, uint64_t* c, uint64_t* d);
+// the entry of c + i d, 0 <= c, d < q
 HostTw gf_pack(uint64_t c, uint64_t d);
-// Values of one Stockham line DFT of length L: for every stage after the first, span Ns
-// and radix R, w^q (q = 1..R-1) of w = root(+-k, Ns R) at off[s] + (q-1) Ns + k.
-void gf_stage_twiddles(int L, const int* radices, int nst, bool inverse, std::vector<HostTw>& tw, int* off);
+// Values of one Stockham line DFT: for every stage after the first, span Ns and radix R, w^q
+// (q = 1..R-1) of w = root(+-k, Ns R) at off[s] + (q-1) Ns + k, where root(t, L) is a fixed
+// family of roots of unity with root(t, L) root(u, L) = root(t + u, L) and root(t k, L k) =
+// root(t, L).
+void gf_stage_twiddles(const int* radices, int nst, bool inverse, std::vector<HostTw>& tw, int* off);
 // For t = gf_excess(W H), W = t V, L = V H (t = 1: V = W, L = M):
 // k1[m1 H + k2] = root((m1/t) k2, L); k2t[k2 W + m1] = root(-(m1/t) k2, L) / L;
 // pair[k2 V + k1] = -(1 + root(k2 + H k1, L)) / 4 for t = 1, root(k2 + H k1, L) for t > 1
