@@ -12,6 +12,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "gl_gf61.cuh"
 #include "gl_internal.h"
 #include "gl_plan.h"
 #include "gl_tables.h"
@@ -415,28 +416,33 @@ int first_int_layout(int M, int sms) {
 }
 
 // Whether the passes touch the tables they will read at their start (IntArgs::touch): where
-// at most one CTA runs per SM, its L1 is empty and has room for all of them.
-int int_touch(int H, int W) { return W <= 152 * 2 && H / 2 < 152 * 2; }
+// at most two CTAs run per SM, its L1 is empty and has room for all of them.
+int int_touch(int H, int W) { return W <= 2 * kSms && H / 2 < 2 * kSms; }
 
 // Whether the products of (p, N) are determined by their residues mod q = 2^61 - 1 for
 // every state the iteration can reach: words are at most 2^LO plus a carry in magnitude,
-// an unweighted product sums N of their products times at most 2, and must stay below 2^60.
-// *vmax: the bound on a word used here (a loaded state is checked against it).
+// an unweighted product sums N of their products times at most 2, and must stay within
+// gf::kMaxProduct.  *vmax: the bound on a word used here (a loaded state is checked against it).
+constexpr double kProductBound = 1152921504606846976.0 - 1024.0;  // 2^60, less the rounding of the sum
 bool int_range_ok(int p, int N, int* vmax) {
   const int LO = p / N;
   if (LO > 28) return false;
   const double v = (double)(1 << LO) + 256.0;
   *vmax = (1 << LO) + 256;
-  return 2.0 * N * v * v < 1152921504606846976.0;  // 2^60
+  static_assert((int64_t)kProductBound <= gf::kMaxProduct, "the sum below is rounded");
+  return 2.0 * N * v * v <= kProductBound;
 }
 
 // The integer form has no round-off to watch, so it is used where the FP64 form's stays
 // below the default limit and with a limit that is not tightened; elsewhere every iteration
 // measures its round-off.  The line is gl_safe_signal_size's (round-off <= 0.125) plus 0.3
-// bits per word: the round-off doubles every 0.45 bits or so, so <= 0.2 there.  At the
-// resident lengths the line is known better, from 60000 iterations each: plus 0.9 up to
-// N = 2048 (0.34 at 2048 and 21.73 bits, 0.31 at 1024 and 21.98), plus 0.75 up to 4096
-// (0.28 at 4096 and 21.29 bits, plus 0.72; 0.22 at 3072 and 21.30, plus 0.61).
+// bits per word: the round-off doubles every 0.45 bits or so, so <= 0.2 there (measured on
+// the line, 1500 to 30000 iterations at 18 lengths from 4200 to 4194304: 0.14 to 0.19).  At
+// the resident lengths, which a full test of p - 2 iterations is short at, the line is closer
+// to the limit: plus 0.9 up to N = 2048, plus 0.75 up to 4096.  Measured on it, 60000
+// iterations each: N = 2048 0.34, 2000 and 1920 0.38, 1536 and 1280 0.31, 4096 0.27, 3840 0.31,
+// 3072 0.28, 2560 0.31.  From N = 1024 down the carry table's 22 bits come before the line:
+// 0.31 at 1024 and 960, 0.38 at 1000, 0.27 at 768, 0.19 at 512, 0.06 at 128.
 bool int_roundoff_ok(int p, int N, double error_limit) {
   const double over = N <= 2048 ? 0.9 : N <= kResidentAutoN ? 0.75 : 0.3;
   return error_limit >= 0.4 && (double)p / N <= 19.2 + over - 0.26 * std::log2(N / 163840.0);
@@ -932,7 +938,7 @@ bool gl_int_layout(int p, int N, int* H, IntGeom* g) {
   int vmax = 0;
   if (!int_range_ok(p, N, &vmax) || !int_roundoff_ok(p, N, 0.4)) return false;
   const int M = N / 2;
-  if (!(*H = first_int_layout(M, 152))) return false;
+  if (!(*H = first_int_layout(M, kSms))) return false;
   return choose_int_geom(*H, M / *H, g, untimed_variant(*H, M / *H));
 }
 

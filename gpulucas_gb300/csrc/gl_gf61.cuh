@@ -439,7 +439,9 @@ GL_HD int64_t weighted(int v, int e) {
 }
 
 // The integer congruent to x 2^-e in [-2^60 - 4, 2^60 + 3], x within 3R, 0 <= e <= 60.  A
-// product below 2^59 in magnitude is that integer itself.
+// product of at most kMaxProduct in magnitude is that integer itself: its other
+// representatives, q away, lie outside.
+constexpr int64_t kMaxProduct = (1ll << 60) - 6;
 GL_HD int64_t unweighted(int64_t x, int e) {
   return red((int64_t)(((uint64_t)x << (61 - e)) & kQ) + (x >> e));
 }

@@ -229,6 +229,11 @@ struct GfSlot {
   __host__ __device__ int4 operator()(int q) const { return tw4(tw[q * step]); }
 };
 
+struct PolyGet {
+  const int4* l;
+  __host__ __device__ int4 operator()(int i) const { return l[i]; }
+};
+
 // One line of L points, stride st, transformed as the integer form's stages do; *peak: the
 // largest magnitude of a stage's output.
 template <int S>
@@ -327,5 +332,23 @@ void hc_gf_cmul(const long long* x, const unsigned long long* w, long long* out)
 long long hc_gf_red(long long x) { return gl::gf::red(x); }
 long long hc_gf_weighted(int v, int e) { return gl::gf::weighted(v, e); }
 long long hc_gf_unweighted(long long x, int e) { return gl::gf::unweighted(x, e); }
+
+// One value within R in limbs (c0, c1 of each part).
+void hc_gf_as_limbs(const long long* x, int* out) {
+  const int4 w = gl::gf::as_limbs(g2{x[0], x[1]});
+  out[0] = w.x, out[1] = w.y, out[2] = w.z, out[3] = w.w;
+}
+// u(y)^2 mod y^t - z for coefficients u within R, as the polynomial row pass computes it;
+// z as residues.
+void hc_gf_poly_square(int t, const long long* u, const unsigned long long* z, long long* out) {
+  std::vector<int4> l((size_t)t);
+  for (int i = 0; i < t; ++i) l[i] = gl::gf::as_limbs(g2{u[2 * i], u[2 * i + 1]});
+  const PolyGet get{l.data()};
+  for (int b = 0; b < t; ++b) {
+    const g2 r = gl::gf::poly_square(get, t, b, tw4(gl::gf_pack(z[0], z[1])));
+    out[2 * b] = r.re;
+    out[2 * b + 1] = r.im;
+  }
+}
 
 }  // extern "C"

@@ -79,6 +79,7 @@ struct PlainGeom {
 // 16-byte accesses are served eight lanes at a time
 constexpr int int_stride(int L) { return L + (L >> 3) + 1; }
 constexpr int kMaxIntSmem = 120 * 1024;
+constexpr int kSms = 152;  // GB300's, for the integer form's rules, which were measured there
 constexpr int kIntHeld = 8;
 
 // Geometry of the integer form (gl_int_kernels.cu) on the same H x W array.

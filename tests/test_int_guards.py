@@ -256,6 +256,83 @@ def test_find_signal_size_reports_the_time_of_the_plan_it_describes(gl):
     assert integer and plan_ms < 0.75 * fp64_ms
 
 
+Q = (1 << 61) - 1
+R = (1 << 60) + (1 << 35)
+MAX_PRODUCT = (1 << 60) - 6
+
+
+@pytest.fixture(scope="module")
+def hc():
+    lib = ctypes.CDLL(_build.HOSTCHECK)
+    i64 = np.ctypeslib.ndpointer(np.int64, flags="C_CONTIGUOUS")
+    lib.hc_gf_as_limbs.argtypes = [i64, np.ctypeslib.ndpointer(np.int32, flags="C_CONTIGUOUS")]
+    lib.hc_gf_poly_square.argtypes = [ctypes.c_int, i64, np.ctypeslib.ndpointer(np.uint64, flags="C_CONTIGUOUS"), i64]
+    lib.hc_gf_unweighted.argtypes = [ctypes.c_longlong, ctypes.c_int]
+    lib.hc_gf_unweighted.restype = ctypes.c_longlong
+    return lib
+
+
+# values whose limbs are at their bounds, and those within R at its ends
+_EDGE = [s * v for s in (1, -1) for v in ((1 << 60) + (1 << 30), (1 << 60) - (1 << 30) - 1, (1 << 60) + (1 << 35), 1 << 60,
+                                          1 << 30, (1 << 31) - 1, 0)]
+
+
+def test_values_in_limbs_at_their_bounds(hc):
+    out = np.zeros(4, np.int32)
+    for a in _EDGE:
+        for b in _EDGE:
+            hc.hc_gf_as_limbs(np.array([a, b], np.int64), out)
+            c = [int(v) for v in out]
+            assert c[0] + (c[1] << 31) == a and c[2] + (c[3] << 31) == b
+            assert abs(c[0]) <= 1 << 30 and abs(c[2]) <= 1 << 30
+            assert abs(c[1]) <= (1 << 29) + 16 and abs(c[3]) <= (1 << 29) + 16
+
+
+@pytest.mark.parametrize("t", [3, 5, 7, 9, 15, 21, 25, 27, 35, 45, 49])
+def test_polynomial_squares_at_the_limbs_bounds(hc, t):
+    """Every length of polynomial that the integer form takes, against Python integers: all
+    coefficients at one bound (the sums of products at their largest), mixed, and random."""
+    rng = np.random.default_rng(t)
+    out = np.zeros(2 * t, np.int64)
+    zs = [(0, Q - 1), (Q >> 1, (Q >> 1) + 1), ((1 << 60) - 1, 1 << 60), (1 << 30, Q - (1 << 30))]
+    cases = [[e] * (2 * t) for e in _EDGE] + [[e, -e] * t for e in _EDGE[:4]]
+    cases += [[_EDGE[i] for i in rng.integers(len(_EDGE), size=2 * t)] for _ in range(6)]
+    cases += [[int(v) for v in rng.integers(-R, R + 1, size=2 * t)] for _ in range(6)]
+    for i, u in enumerate(cases):
+        zc, zd = zs[i % len(zs)] if i % 3 else [int(v) for v in rng.integers(0, Q, 2)]
+        hc.hc_gf_poly_square(t, np.array(u, np.int64), np.array([zc, zd], np.uint64), out)
+        for b in range(t):
+            re = im = 0
+            for half in (0, 1):
+                hr = hi = 0
+                for j in range(t):
+                    k = b + half * t - j
+                    if 0 <= k < t:
+                        hr += u[2 * j] * u[2 * k] - u[2 * j + 1] * u[2 * k + 1]
+                        hi += u[2 * j] * u[2 * k + 1] + u[2 * j + 1] * u[2 * k]
+                if half:
+                    hr, hi = hr * zc - hi * zd, hr * zd + hi * zc
+                re, im = re + hr, im + hi
+            x, y = int(out[2 * b]), int(out[2 * b + 1])
+            assert (x - re) % Q == 0 and (y - im) % Q == 0, (i, b)
+            assert abs(x) <= R and abs(y) <= R
+
+
+def test_products_up_to_their_bound_come_back_themselves(hc):
+    """Any representative that the inverse transform may give of a product within the bound
+    that plans are held to."""
+    rng = np.random.default_rng(60)
+    ns = [s * (MAX_PRODUCT - d) for s in (1, -1) for d in (0, 1, 2, 3, 1 << 20)] + [
+        s * (1 << 59) + d for s in (1, -1) for d in (-1, 0, 1)] + [
+        int(v) for v in rng.integers(-MAX_PRODUCT, MAX_PRODUCT + 1, 200)]
+    for n in ns:
+        for e in range(61):
+            for k in (-1, 0, 1):
+                x = n * pow(2, e, Q) % Q + k * Q
+                if abs(x) <= 3 * R:
+                    assert hc.hc_gf_unweighted(x, e) == n
+
+
 def test_int_info_layout_matches_header(tmp_path, gl):
     lines = ["#include <stdio.h>", "#include <stddef.h>", '#include "gpulucas.h"', "int main(void) {",
              'printf("%zu\\n", sizeof(gl_int_info));']
