@@ -44,8 +44,8 @@ __device__ __forceinline__ void touch(const int4* p, int n) {
 // What the pass before writes (products, work arrays) is read with ordinary loads: the wait
 // makes it visible to them, not to the non-coherent path, which is for the tables alone.
 // For iterations launched one by one (N = 65536 without allocation: 27.3 -> 20.6 us per
-// iteration); in a replayed graph it gains nothing (163840: 23.1 -> 24-26, 65536: 18.3 ->
-// 17.2, 5120: 14.6 -> 15.5), so plans do not use it.
+// iteration).  In a replayed graph it gains at some lengths and loses at others (65536: 18.3
+// -> 17.2, 163840: 23.1 -> 24-26, 5120: 14.6 -> 15.5); plans do not use it.
 __device__ __forceinline__ void after_previous_pass() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) ki_row_poly(IterArgs a) { int_
 // Two builds for radices 8, 4, 2, 3: five CTAs of 192 threads per SM (64 registers) where the
 // row pairs are enough to fill them, else 80 registers, which shorten the dependent chains
 // of a pass with few CTAs (N = 49152, 49 pairs: 14.1 us against 15.6).
-constexpr int kRowsFor5 = 3 * 152;
+constexpr int kRowsFor5 = 3 * kSms;
 template <bool B57, int T, int MB>
 __global__ void __launch_bounds__(T, MB) ki_row_sq(IterArgs a) {
   int_row_body<B57>(a, blockIdx.x);

@@ -157,12 +157,15 @@ int gl_reset(gl_plan* plan);
 /* Runs `iters` LL iterations: the loop body mersenneIter<check,0> (gpuLucas.cu:845-942)
  * with the round-off check of mersenneTest (gpuLucas.cu:1399-1410), aborting with
  * GL_ERR_ROUNDOFF at the plan's error limit.
- * Fused-form plans whose round-off stays well below the default limit (p/N up to 0.3 bits
- * over gl_safe_signal_size's line, 0.75 to 0.9 up to N = 4096; error_limit >= 0.4; no option
- * that names an FP64 kernel variant) run most iterations in exact integer arithmetic, which
- * gives the same products and has no round-off; one iteration in 64 runs in FP64, and the
- * reported round-off is over those (0 if a call held none).  Other plans, the round-off
- * trials (gl_error_test, gl_find_signal_size) and batches run FP64 in every iteration. */
+ * Fused-form plans whose FP64 round-off was measured below the default limit (p/N up to 0.3
+ * bits over gl_safe_signal_size's line, round-off 0.2; 0.75 to 0.9 bits up to N = 4096,
+ * round-off up to 0.38 in 60000 iterations), with error_limit >= 0.4 and no option that names
+ * an FP64 kernel variant, run most iterations in exact integer arithmetic, which gives the
+ * same products and has no round-off; one iteration in 64 runs in FP64, and the reported
+ * round-off is over those (0 if a call held none).  Other plans, those the integer form's
+ * tables do not fit the device for, the few lengths (odd parts with high powers of 3, 5 and
+ * 7) that FP64 is faster at, the round-off trials (gl_error_test, gl_find_signal_size) and
+ * batches run FP64 in every iteration.  gl_plan_int_info tells which a plan does. */
 int gl_iterate(gl_plan* plan, int64_t iters, gl_iter_report* report);
 
 /* Asynchronous forms for callers that time or overlap work themselves: enqueue
